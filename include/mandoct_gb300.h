@@ -206,16 +206,16 @@ int mct_helical_rebin(const mct_helical* h, const float* sgm, const float* z_pos
 /* ---------------------------------------------------------------- forward projection */
 
 /* Bytes of the optional forward-projection workspace (gather copies of the volume:
- * cone beam, two float32 quad copies of 16 bytes per voxel; fan beam, one
- * x/y-transposed copy). */
+ * cone beam, two float32 quad copies of 16 bytes per voxel, their rows padded by 3 to 10
+ * elements from 128 columns; fan beam, one x/y-transposed copy). */
 size_t mct_fp_workspace_size(const mct_geom* g);
 
 /* Ray-driven trilinear forward projection of vol [nz][nx][nx] for all views into
  * sgm [nv][views][nu] (overwritten).  Rays with mask != 1 (mask [nv][views][nu], or
  * NULL for none) give 0.  workspace (mct_fp_workspace_size bytes, 16-byte aligned, or
- * NULL) receives gather copies of vol: for cone beam, per voxel the z-pairs of the
- * voxel and of its neighbour along the copy's slow axis (16 bytes; a trilinear cell is
- * two adjacent elements) in [z][y][x] and [z][x][y] order, for fan beam an
+ * NULL) receives gather copies of vol: for cone beam, per voxel its value and its
+ * differences along z, the copy's slow axis and both (16 bytes; a trilinear cell is two
+ * adjacent elements) in [z][y][x] and [z][x][y] order, for fan beam an
  * x/y-transposed copy; views whose detector columns run along y read the transposed
  * order, so a warp's gathers are coalesced.  Results agree with and without the
  * workspace to float32 rounding (the same samples, so the same zero pattern).
@@ -226,7 +226,8 @@ int mct_fp(const mct_geom* g, const mct_tables* t, const float* vol, const float
            void* workspace, void* stream);
 
 /* Bytes of the mct_fp_storage workspace for dtype (MCT_F32: mct_fp_workspace_size;
- * MCT_BF16 / MCT_F16: two 16-bit cell copies, 32 bytes per voxel (+16 for float16);
+ * MCT_BF16 / MCT_F16: two 16-bit cell copies, 32 bytes per voxel, rows padded alike (+16
+ * for float16);
  * 0 if unsupported). */
 size_t mct_fp_storage_workspace_size(const mct_geom* g, int32_t dtype);
 

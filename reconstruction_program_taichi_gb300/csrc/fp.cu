@@ -30,6 +30,7 @@ struct FpParams {
     // of the block's (view, row) slots; blockIdx.y runs over 2^rs row tiles within
     // each view group (the block order is column tile, row tile, view group, row group)
     int vshift, bcs, wcs, rs;
+    int pitch;  // elements per row of the volume or its copies (a plane is nx rows)
 };
 
 struct Ray {
@@ -163,34 +164,30 @@ __device__ __forceinline__ bool spread_along_y(const FpParams& p, int j, const f
     return fabsf(cb) > fabsf(sb);  // d(x, y)/du is (-sin b, cos b)
 }
 
-// Grid of every ray kernel: x = 32-column detector tiles, y = views, z = 8-row
+// Grid of the other ray kernels: x = 32-column detector tiles, y = views, z = 8-row
 // detector tiles.  Blocks are scheduled x, then y, then z, so the blocks resident at
 // one time cover many views of the same detector rows; those rays cross only a thin
-// z-slab of the volume, which then stays in L2 across views.  fp_kernel with copies
-// instead takes tiles of 16 columns x 2^vshift consecutive views x 2^(4 - vshift)
-// rows (x = column tiles, y = view groups, z = row tiles), each warp 4 columns x 8
-// (view, row) slots; each ray's arithmetic is the same either way.
+// z-slab of the volume, which then stays in L2 across views.  fp_kernel takes tiles of
+// 16 columns x 2^vshift consecutive views x 2^(4 - vshift) rows (x = column tiles, y =
+// view groups, z = row tiles).
 //
 // One thread per ray (u, v) of view j.  vol is [z][y][x]; vol_t, when
 // given, is the same volume as [z][x][y]: views whose detector columns spread along
 // y read vol_t so that neighbouring rays touch consecutive addresses.  With ZP
 // (cone beam, workspace given) the volume is read from copies zp_x ([z][y][x]) and
-// zp_y ([z][x][y]): float32 quads (two adjacent 16-byte elements per cell reload) or
+// zp_y ([z][x][y]): float32 quads (two adjacent 16-byte elements per cell) or
 // 16-bit cells (the whole 2x2x2 trilinear cell in one 16-byte element), below.
 
 // float32 quad copy, indexed in a (slow s, fast f) frame: (s, f) = (y, x) for views whose
 // detector columns spread along x (copy cx, [z][y][x]) and (x, y) for the others (copy
 // cy, [z][x][y]), so that neighbouring rays read neighbouring elements.  Element
-// (z, s, f) holds the z-pairs of the voxel and of its neighbour along s,
-//   {V(z, s, f), V(z+1, s, f), V(z, s+1, f), V(z+1, s+1, f)}    (16 bytes),
-// and the neighbour along f is the next element: a cell reload is two adjacent 16-byte
-// loads, and the f-differences are taken in registers (the same float32 subtraction a
-// direct read would do).  Against a 32-byte element holding the whole cell (differences
-// included) this halves the copies (32 instead of 64 bytes per voxel for both
-// orientations), so twice the cells fit L1 and L2; with blocks of 8 consecutive views,
-// whose rays cross nearly the same cells at the same step, the projector at
-// 512x512x256 / 1080 views went 297.6 -> 267.3 ms (the 32-byte cells: 304-312 ms with
-// 2-8 views per block, 297.6 with 8 rows of one view).
+// (z, s, f) holds the voxel and its forward differences along z, s and both,
+//   {V, Dz V, Ds V, Dz Ds V}(z, s, f)    (16 bytes),
+// and the neighbour along f is the next element: a cell is two adjacent 16-byte loads,
+// and its f-differences are taken in registers.  Whole 32-byte cells would double the
+// copies, and half as many cells fit L1 and L2.  Differences instead of the four values
+// themselves: the interpolation then needs no z-subtractions (five of about 50
+// instructions per cell; 171.9 -> 158.9 ms at 512x512x256 / 1080 views).
 struct __align__(16) Quad16 {
     float v[4];
 };
@@ -206,23 +203,51 @@ __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
     return *reinterpret_cast<uint32_t*>(&b);
 }
 
-// Resident blocks per SM that the register allocation of fp_kernel targets.  The
-// float32 cone-beam path waits on L1 and needs its warps: with quad copies and the
-// 16 x 16-view tiles, 5 blocks (48 registers) take 237.2 ms at 512x512x256 / 1080
-// views, 4 blocks 240.2 ms (8-view tiles: 5 blocks 267.3, 4 blocks 273.8, 6 blocks,
-// 40 registers with spills, 317.1); the fan-beam path keeps 40 registers (6 blocks).
-// The 16-bit paths are issue-bound and gain from registers: 1 (80 registers, 3 blocks
-// of 256) gives bf16 237.4 ms against 254.9 with 5 blocks (8-view tiles), float16
-// 274.4 against 291.7; with the 16-column tiles 1 and 2 blocks are equal (224.0).
-template <bool CONE, typename ZT>
-struct FpMinBlocks {
-    static constexpr int value = (std::is_same<ZT, uint4>::value || std::is_same<ZT, h16x8>::value) ? 1
-                                 : CONE                                                             ? 5
-                                                                                                    : 6;
-};
+// Resident blocks per SM that the register allocation of fp_kernel targets: 5 (48
+// registers) with copies.  512x512x256 / 1080 views, float32: 4 blocks 160.6 ms, 5
+// 158.9, 6 164.7; 512x512x64 / 360 views, bf16: 4 blocks 13.55 ms, 5 13.41, 6 14.27.
+// The fan-beam path needs 40 registers (6 blocks).
+template <bool CONE>
+constexpr int fp_min_blocks() {
+    return CONE ? 5 : 6;
+}
 
-template <bool CONE, bool ZP, typename ZT>
-__global__ void __launch_bounds__(256, FpMinBlocks<CONE, ZT>::value)
+// Above this many steps a ray's indices are no longer exact in float32 (and would not
+// advance one by one): such rays are sampled one sample at a time.
+constexpr int kMaxWalkSteps = 1 << 23;
+
+// Planes along the rays' main axis per window (WIN, below).
+constexpr int kWinPlanes = 64;
+
+// A ray's sum over its samples, cell by cell.  The samples are equally spaced (step df)
+// and the interpolant of one 2x2x2 cell is trilinear, so the n samples that fall into a
+// cell need not be taken one by one: with m their midpoint and s^2 = (n^2 - 1) / 12 the
+// variance of n consecutive integers,
+//     sum = n [ V(m) + s^2 (dx dy Vxy(m) + dx dz Vxz(m) + dy dz Vyz(m)) ]
+// exactly (the odd central moments vanish, the second differences along one axis too).
+// n is the number of steps to the nearest face the ray leaves the cell through.  At the
+// default step of 0.2 voxel diagonals a cell holds 2.2 samples on average (0.1: 4.4,
+// 0.5: 0.9), and every lane of a warp loads a cell in every iteration, where a walk by
+// samples has some lane entering a cell at almost every sample, with the others idle.
+// A sample within rounding of a face may be taken from the cell before it: the
+// interpolant is continuous there.
+//
+// What bounds it: L1 data-pipe wavefronts (84 % for float32 at 128^3, 93 % at 256x256x64
+// / 180 views), then issue (62 %, 49 %).  A warp's loads take a tag lookup per 4 lines
+// and a wavefront per conflicting 16-byte bank, so the copies' rows are padded to an odd
+// number of elements (copy_pitch), a warp's rays are neighbours (ray tiles, below), and
+// with WIN the lanes are kept together: they cross the volume in windows of kWinPlanes
+// planes along their main axis and wait for each other at the end of each, which keeps
+// rays whose cells are counted differently in the same rows of the copy.  The wait costs
+// what the rays' entry points differ by, so it pays for wide volumes.
+//   ms, by samples / by cells / with windows:
+//     512x512x256, 1080 views, float32     237.6 / 159.0 / 153.0
+//     128x128x64, 270 views, float32       1.036 / 0.699 / 0.738
+//     512x512x64, 360 views, bf16          18.32 / 13.41 / 14.9 (windows: 16-bit cells lose)
+//     512^2 fan beam, 720 views            1.34 / 0.80 / 0.66
+//     256x256x128, 360 views, step 0.1     18.83 / 7.19;  step 0.5: 6.20 / 5.95
+template <bool CONE, bool ZP, typename ZT, bool WIN>
+__global__ void __launch_bounds__(256, fp_min_blocks<CONE>())
 fp_kernel(FpParams p, const float* __restrict__ angles, const float* __restrict__ u_arr,
           const float* __restrict__ v_arr, const float* __restrict__ czv, const float* __restrict__ pa,
           const float* __restrict__ pxs, const float* __restrict__ vol, const float* __restrict__ vol_t,
@@ -254,8 +279,8 @@ fp_kernel(FpParams p, const float* __restrict__ angles, const float* __restrict_
     constexpr bool kQuad = ZP && std::is_same<ZT, Quad16>::value;
     const float* __restrict__ V = tr ? vol_t : vol;
     const ZT* __restrict__ V2 = tr ? zp_y : zp_x;
-    const int sx = (tr && !kQuad) ? nx : 1, sy = (tr && !kQuad) ? 1 : nx;
-    const int plane = nx * nx;  // volumes below 2^31 voxels (checked on the host)
+    const int sx = (tr && !kQuad) ? p.pitch : 1, sy = (tr && !kQuad) ? 1 : p.pitch;
+    const int plane = p.pitch * nx;  // volumes and copies below 2^31 elements (checked on the host)
     Ray r;
     float acc = 0.0f;
     if (setup_ray(p, iu, iv, j, angles, u_arr, v_arr, czv, pa, pxs, true, r)) {
@@ -268,23 +293,23 @@ fp_kernel(FpParams p, const float* __restrict__ angles, const float* __restrict_
             r.dfy = t;
         }
         const float xmax = (float)(nx - 1), zmax = (float)(p.nz - 1);
-        // Consecutive samples are 0.2 voxel diagonals apart, so most fall in the same
-        // 2x2x2 cell as the previous one: the cell stays in registers (as corner values
-        // and x-differences, lower and upper z-plane packed side by side) and is
-        // reloaded only when the ray enters a new cell.
-        int cell = -1;
-        float2 e00 = make_float2(0.f, 0.f), e10 = e00, g00 = e00, g10 = e00;  // corners, x-differences
-        auto load_cell = [&](int off) {
-            if (off == cell) return;
-            cell = off;
+        struct Cell {
+            // trilinear coefficients: corner, x, y and xy differences, each as {value, z-difference}
+            // (float32 quads) or {lower plane, upper plane} (the others)
+            float2 e, ex, ey, exy;
+        };
+        auto load_cell = [&](int off, Cell& c) {
             if constexpr (kQuad) {
                 const float4 q0 = __ldg(reinterpret_cast<const float4*>(V2 + off));
                 const float4 q1 = __ldg(reinterpret_cast<const float4*>(V2 + off + 1));
-                e00 = make_float2(q0.x, q0.y);
-                e10 = make_float2(q0.z, q0.w);
-                g00 = __fadd2_rn(make_float2(q1.x, q1.y), make_float2(-q0.x, -q0.y));
-                g10 = __fadd2_rn(make_float2(q1.z, q1.w), make_float2(-q0.z, -q0.w));
-            } else if constexpr (ZP && std::is_same<ZT, uint4>::value) {
+                c.e = make_float2(q0.x, q0.y);
+                c.ey = make_float2(q0.z, q0.w);
+                c.ex = __fadd2_rn(make_float2(q1.x, q1.y), make_float2(-q0.x, -q0.y));
+                c.exy = __fadd2_rn(make_float2(q1.z, q1.w), make_float2(-q0.z, -q0.w));
+                return;
+            }
+            float2 e00, g00, e10, g10;  // corners and x-differences of the lower and upper z-plane
+            if constexpr (ZP && std::is_same<ZT, uint4>::value) {
                 const uint4 q = __ldg(V2 + off);
                 e00 = bf16x2_to_float2(q.x);
                 g00 = bf16x2_to_float2(q.y);
@@ -296,106 +321,154 @@ fp_kernel(FpParams p, const float* __restrict__ angles, const float* __restrict_
                 g00 = h16x2_to_float2(q.y);
                 e10 = h16x2_to_float2(q.z);
                 g10 = h16x2_to_float2(q.w);
-            } else {
+            } else if constexpr (!kQuad) {
                 const float* b = V + off;
                 const float a00 = __ldg(b), a01 = __ldg(b + sx), a10 = __ldg(b + sy), a11 = __ldg(b + sx + sy);
                 float c00 = 0.f, c01 = 0.f, c10 = 0.f, c11 = 0.f;
                 if (CONE) {
-                    const float* c = b + plane;
-                    c00 = __ldg(c); c01 = __ldg(c + sx); c10 = __ldg(c + sy); c11 = __ldg(c + sx + sy);
+                    const float* u = b + plane;
+                    c00 = __ldg(u); c01 = __ldg(u + sx); c10 = __ldg(u + sy); c11 = __ldg(u + sx + sy);
                 }
                 e00 = make_float2(a00, c00);
                 e10 = make_float2(a10, c10);
                 g00 = __fadd2_rn(make_float2(a01, c01), make_float2(-a00, -c00));
                 g10 = __fadd2_rn(make_float2(a11, c11), make_float2(-a10, -c10));
             }
+            c.e = e00;
+            c.ex = g00;
+            c.ey = __fadd2_rn(e10, make_float2(-e00.x, -e00.y));
+            c.exy = __fadd2_rn(g10, make_float2(-g00.x, -g00.y));
         };
-        // lower (.x) and upper (.y) z-plane bilinear values in packed f32x2 FMAs; per
-        // lane this is exactly fmaf(xw, a01 - a00, a00) etc.
-        auto interp = [&](float xw, float yw, float zw) -> float {
-            const float2 xw2 = make_float2(xw, xw), yw2 = make_float2(yw, yw);
-            const float2 l0 = __ffma2_rn(xw2, g00, e00);
-            const float2 l1 = __ffma2_rn(xw2, g10, e10);
-            const float2 pl = __ffma2_rn(yw2, __fadd2_rn(l1, make_float2(-l0.x, -l0.y)), l0);
-            return CONE ? fmaf(zw, pl.y - pl.x, pl.x) : pl.x;
-        };
-        auto sample = [&](int k, bool check) {
+        auto dz = [](float2 a) { return kQuad ? a.y : a.y - a.x; };  // the z-difference of a pair
+        // Checked samples at the ends of the range, where the inside test decides; the range
+        // between them (at least 1e-3 voxel inside on every axis) is walked cell by cell.
+        auto sample = [&](int k) {
             const float fk = (float)k;
             const float fx = fmaf(fk, r.dfx, r.fx0);
             const float fy = fmaf(fk, r.dfy, r.fy0);
             const float xf = floorf(fx), yf = floorf(fy);
-            bool ok = true;
-            int xi = (int)xf, yi = (int)yf, zi;
-            if (check) {
-                ok = xf >= 0.0f && xf < xmax && yf >= 0.0f && yf < xmax;
-                xi = min(max(xi, 0), nx - 2);
-                yi = min(max(yi, 0), nx - 2);
-            }
-            const float xw = fx - xf, yw = fy - yf;
+            bool ok = xf >= 0.0f && xf < xmax && yf >= 0.0f && yf < xmax;
+            const int xi = min(max((int)xf, 0), nx - 2), yi = min(max((int)yf, 0), nx - 2);
+            int zi = iv;
             float zw = 0.0f;
             if (CONE) {
                 const float fz = fmaf(fk, r.dfz, r.fz0);
                 const float zf = floorf(fz);
-                zi = (int)zf;
-                if (check) {
-                    ok = ok && zf >= 0.0f && zf < zmax;
-                    zi = min(max(zi, 0), p.nz - 2);
-                }
+                ok = ok && zf >= 0.0f && zf < zmax;
+                zi = min(max((int)zf, 0), p.nz - 2);
                 zw = fz - zf;
-            } else {
-                zi = iv;
             }
-            const int off = zi * plane + yi * sy + xi * sx;
-            load_cell(off);
-            const float val = interp(xw, yw, zw);
-            if (check) acc += ok ? val : 0.0f;
-            else acc += val;
-        };
-        // Interior samples (at least 1e-3 voxel inside on every axis).  With copies
-        // the floors come from adding M = 1.5 * 2^23 rounded toward -infinity (exactly
-        // M + floor(f) for |f| < 2^22), on the FMA pipe instead of the conversion unit
-        // (which otherwise limits the 16-bit kernels), and the x and y coordinates
-        // travel as one f32x2 pair: position, floor and weight are three packed
-        // operations for both axes.  The element offset is summed in unsigned arithmetic
-        // (the bias terms wrap, the total is the offset, below 2^31).
-        constexpr bool kRoundFloor = ZP && !std::is_same<ZT, float2>::value;
-        const float M = 12582912.0f;
-        const unsigned MB = 0x4B400000u;  // bit pattern of M
-        const unsigned obias = CONE ? MB * (unsigned)(plane + sy + sx) : MB * (unsigned)(sy + sx) - (unsigned)(iv * plane);
-        const float2 dxy = make_float2(r.dfx, r.dfy), fxy0 = make_float2(r.fx0, r.fy0);
-        const float2 M2 = make_float2(M, M), nM2 = make_float2(-M, -M);
-        auto sample_fast = [&](float fk) {
-            const float2 f = __ffma2_rn(make_float2(fk, fk), dxy, fxy0);  // fractional indices x, y
-            const float2 m = __fadd2_rd(f, M2);                            // M + floor(f)
-            const float2 fl = __fadd2_rn(m, nM2);                          // floor(f), exact
-            const float2 w = __fadd2_rn(f, make_float2(-fl.x, -fl.y));     // weights, exact
-            unsigned off = (unsigned)__float_as_int(m.x) * (unsigned)sx + (unsigned)__float_as_int(m.y) * (unsigned)sy - obias;
-            float zw = 0.0f;
-            if (CONE) {
-                const float fz = fmaf(fk, r.dfz, r.fz0);
-                const float mz = __fadd_rd(fz, M);
-                zw = fz - (mz - M);
-                off += (unsigned)__float_as_int(mz) * (unsigned)plane;
-            }
-            load_cell((int)off);
-            acc += interp(w.x, w.y, zw);
+            Cell c;
+            load_cell(zi * plane + yi * sy + xi * sx, c);
+            const float xw = fx - xf, yw = fy - yf;
+            const float2 l = __ffma2_rn(make_float2(xw, xw), c.ex, c.e);
+            const float2 gy = __ffma2_rn(make_float2(xw, xw), c.exy, c.ey);
+            const float2 pl = __ffma2_rn(make_float2(yw, yw), gy, l);
+            acc += !ok ? 0.0f : CONE ? fmaf(zw, dz(pl), pl.x) : pl.x;
         };
         int kis, kie;
         interior_range(p, r, CONE, kis, kie);
-        for (int k = r.ks; k < kis; ++k) sample(k, true);
-        if constexpr (kRoundFloor) {
-            float fk = (float)kis;
-            // unrolled 4 times for float32 quads, twice for 16-bit cells (at 512x512x256 /
-            // 1080 views: float32 237.4 ms against 239.6 with 2; bf16 215.7 against 222.1
-            // with 4)
-            constexpr int kUnroll = kQuad ? 4 : 2;
-#pragma unroll kUnroll
-            for (int k = kis; k <= kie; ++k, fk += 1.0f) sample_fast(fk);
-        } else {
-#pragma unroll 4
-            for (int k = kis; k <= kie; ++k) sample(k, false);
+        if (p.K >= kMaxWalkSteps) {  // step indices would not be exact in float32
+            kis = r.ke + 1;
+            kie = r.ke;
         }
-        for (int k = max(kie + 1, kis); k <= r.ke; ++k) sample(k, true);
+        for (int k = r.ks; k < kis; ++k) sample(k);
+        if (kis <= kie) {
+            // Positions come from f = fma(k, df, f0) and floors from adding M = 1.5 * 2^23
+            // rounded toward minus infinity (exactly M + floor(f) for |f| < 2^22), on the FMA
+            // pipe; x and y travel as one f32x2 pair.  The element offset is summed in
+            // unsigned arithmetic (the bias terms wrap, the total is the offset, below 2^31).
+            const float M = 12582912.0f;
+            const unsigned MB = 0x4B400000u;  // bit pattern of M
+            const unsigned obias =
+                CONE ? MB * (unsigned)(plane + sy + sx) : MB * (unsigned)(sy + sx) - (unsigned)(iv * plane);
+            const float2 M2 = make_float2(M, M), nM2 = make_float2(-M, -M);
+            const float2 dxy = make_float2(r.dfx, r.dfy), fxy0 = make_float2(r.fx0, r.fy0);
+            // steps from fraction w to the face that the ray leaves the cell through: A + w * B
+            const float ix = fminf(1.0f / fabsf(r.dfx), 1e6f), iy = fminf(1.0f / fabsf(r.dfy), 1e6f);
+            const float iz = fminf(1.0f / fabsf(r.dfz), 1e6f);
+            const float2 B2 = make_float2(r.dfx < 0.0f ? ix : -ix, r.dfy < 0.0f ? iy : -iy);
+            const float2 A2 = make_float2(r.dfx < 0.0f ? 0.0f : ix, r.dfy < 0.0f ? 0.0f : iy);
+            const float Bz = r.dfz < 0.0f ? iz : -iz, Az = r.dfz < 0.0f ? 0.0f : iz;
+            const float cxy = r.dfx * r.dfy * (1.0f / 12.0f);
+            const float cxz = r.dfx * r.dfz * (1.0f / 12.0f), cyz = r.dfy * r.dfz * (1.0f / 12.0f);
+            const float kend = (float)kie;
+            // midpoint: n1 / 2 steps; the 16-bit kernels scale n1 instead of the step (two
+            // registers fewer: 48, without spills)
+            constexpr float kN = ZP && !kQuad ? 0.5f : 1.0f, kD = ZP && !kQuad ? 1.0f : 0.5f;
+            const float2 hd = make_float2(kD * r.dfx, kD * r.dfy);
+            const float hdz = kD * r.dfz;
+            struct Run {
+                Cell c;
+                float2 m;      // fractions of the run's midpoint
+                float mz, n;   // and its number of samples
+            };
+            // the run of samples from fk on that lie in one cell; fk moves past it
+            auto next_run = [&](float& fk, Run& q) {
+                const float2 f = __ffma2_rn(make_float2(fk, fk), dxy, fxy0);
+                const float2 m = __fadd2_rd(f, M2);
+                const float2 fl = __fadd2_rn(m, nM2);
+                const float2 w = __fadd2_rn(f, make_float2(-fl.x, -fl.y));
+                unsigned off = (unsigned)__float_as_int(m.x) * (unsigned)sx + (unsigned)__float_as_int(m.y) * (unsigned)sy - obias;
+                float zw = 0.0f;
+                if (CONE) {
+                    const float fz = fmaf(fk, r.dfz, r.fz0);
+                    const float mz = __fadd_rd(fz, M);
+                    zw = fz - (mz - M);
+                    off += (unsigned)__float_as_int(mz) * (unsigned)plane;
+                }
+                load_cell((int)off, q.c);
+                const float2 t2 = __ffma2_rn(w, B2, A2);
+                float t = fminf(fminf(t2.x, t2.y), kend - fk);
+                if (CONE) t = fminf(t, fmaf(zw, Bz, Az));
+                const float n1 = __fadd_rd(t, M) - M;  // steps to the run's last sample
+                q.n = n1 + 1.0f;
+                const float h = kN * n1;
+                q.m = __ffma2_rn(make_float2(h, h), hd, w);
+                if (CONE) q.mz = fmaf(h, hdz, zw);
+                fk += q.n;
+            };
+            auto add_run = [&](const Run& q) {
+                const float2 x2 = make_float2(q.m.x, q.m.x), y2 = make_float2(q.m.y, q.m.y);
+                const float2 l = __ffma2_rn(x2, q.c.ex, q.c.e);
+                const float2 gy = __ffma2_rn(x2, q.c.exy, q.c.ey);
+                const float2 pl = __ffma2_rn(y2, gy, l);
+                float v = pl.x, corr = cxy * q.c.exy.x;
+                if constexpr (CONE && kQuad) {
+                    v = fmaf(q.mz, pl.y, pl.x);
+                    corr = fmaf(cxy, fmaf(q.mz, q.c.exy.y, q.c.exy.x),
+                                fmaf(cxz, fmaf(q.m.y, q.c.exy.y, q.c.ex.y), cyz * gy.y));
+                } else if constexpr (CONE) {
+                    const float2 gx = __ffma2_rn(y2, q.c.exy, q.c.ex);
+                    v = fmaf(q.mz, pl.y - pl.x, pl.x);
+                    corr = fmaf(cxy, fmaf(q.mz, q.c.exy.y - q.c.exy.x, q.c.exy.x),
+                                fmaf(cxz, gx.y - gx.x, cyz * (gy.y - gy.x)));
+                }
+                acc = fmaf(q.n, fmaf(fmaf(q.n, q.n, -1.0f), corr, v), acc);
+            };
+            float fk = (float)kis;
+            if constexpr (WIN) {
+                // window i ends at plane i * kWinPlanes along the rays' main axis, counted
+                // from the side that they enter through: step w0 + i * wi
+                const float ds = tr && !kQuad ? r.dfx : r.dfy, s0 = tr && !kQuad ? r.fx0 : r.fy0;
+                const float is = tr && !kQuad ? ix : iy;
+                const float wi = (float)kWinPlanes * is, w0 = -(ds < 0.0f ? xmax - s0 : s0) * is;
+                for (int i = 1; i * kWinPlanes < nx; ++i) {
+                    const float wend = fminf(fmaf((float)i, wi, w0), kend + 0.5f);
+                    while (fk < wend) {
+                        Run q;
+                        next_run(fk, q);
+                        add_run(q);
+                    }
+                }
+            }
+            while (fk <= kend) {
+                Run q;
+                next_run(fk, q);
+                add_run(q);
+            }
+        }
+        for (int k = max(kie + 1, kis); k <= r.ke; ++k) sample(k);
     }
     if constexpr (IsF16<ZT>::value) acc *= ldexpf(1.0f, -f16_scale_exp(*f16_max));  // float16 cells hold v * 2^e
     sgm[oidx] = acc * p.stepvd;
@@ -415,7 +488,7 @@ __global__ void vol_absmax_kernel(int64_t n, const TIN* __restrict__ v, uint32_t
 // voxel (z, y, x); corners outside the volume are 0 (no in-volume sample uses them).
 // 32x32 tiles, the transposed copy through shared memory.
 template <bool F16, typename TIN = float>
-__global__ void cell16_kernel(int nx, int nz, const TIN* __restrict__ v, uint4* __restrict__ cx,
+__global__ void cell16_kernel(int nx, int nz, int pitch, const TIN* __restrict__ v, uint4* __restrict__ cx,
                               uint4* __restrict__ cy, const uint32_t* __restrict__ f16_max) {
     __shared__ uint4 tile[32][33];
     const int64_t plane = (int64_t)nx * nx;
@@ -439,24 +512,22 @@ __global__ void cell16_kernel(int nx, int nz, const TIN* __restrict__ v, uint4* 
             q.y = pk(at(z, y, x + 1) - a0, at(z + 1, y, x + 1) - a1);
             q.z = pk(c0, c1);
             q.w = pk(at(z, y + 1, x + 1) - c0, at(z + 1, y + 1, x + 1) - c1);
-            cx[z * plane + (int64_t)y * nx + x] = q;
+            cx[((int64_t)z * nx + y) * pitch + x] = q;
             tile[i][threadIdx.x] = q;
         }
     }
     __syncthreads();
     for (int i = threadIdx.y; i < 32; i += blockDim.y) {
         const int x = x0 + i, y = y0 + threadIdx.x;
-        if (y < nx && x < nx) cy[z * plane + (int64_t)x * nx + y] = tile[threadIdx.x][i];
+        if (y < nx && x < nx) cy[((int64_t)z * nx + x) * pitch + y] = tile[threadIdx.x][i];
     }
 }
 
-// float32 quad copies (layout at Quad16): cx[z][y][x] = {V[z][y][x], V[z+1][y][x],
-// V[z][y+1][x], V[z+1][y+1][x]} (fast axis x) and cy[z][x][y] = {V[z][y][x],
-// V[z+1][y][x], V[z][y][x+1], V[z+1][y][x+1]} (fast axis y); corners outside the volume
-// are 0 (no in-volume sample uses them).  32x32 tiles, the transposed copy through
-// shared memory.
+// float32 quad copies (layout at Quad16): cx[z][y][x] with fast axis x and s = y, cy[z][x][y]
+// with fast axis y and s = x; corners outside the volume count as 0 (no in-volume sample
+// uses them).  32x32 tiles, the transposed copy through shared memory.
 template <typename TIN = float>
-__global__ void quad32_kernel(int nx, int nz, const TIN* __restrict__ v, float4* __restrict__ cx,
+__global__ void quad32_kernel(int nx, int nz, int pitch, const TIN* __restrict__ v, float4* __restrict__ cx,
                               float4* __restrict__ cy) {
     __shared__ float4 tile[32][33];
     const int64_t plane = (int64_t)nx * nx;
@@ -468,15 +539,19 @@ __global__ void quad32_kernel(int nx, int nz, const TIN* __restrict__ v, float4*
     for (int i = threadIdx.y; i < 32; i += blockDim.y) {
         const int y = y0 + i, x = x0 + threadIdx.x;
         if (y < nx && x < nx) {
-            const float a0 = at(z, y, x), a1 = at(z + 1, y, x);
-            cx[z * plane + (int64_t)y * nx + x] = make_float4(a0, a1, at(z, y + 1, x), at(z + 1, y + 1, x));
-            tile[i][threadIdx.x] = make_float4(a0, a1, at(z, y, x + 1), at(z + 1, y, x + 1));
+            const float a0 = at(z, y, x), az = at(z + 1, y, x) - a0;
+            auto quad = [&](float b0, float b1) {
+                const float d = b0 - a0;
+                return make_float4(a0, az, d, (b1 - b0) - az);
+            };
+            cx[((int64_t)z * nx + y) * pitch + x] = quad(at(z, y + 1, x), at(z + 1, y + 1, x));
+            tile[i][threadIdx.x] = quad(at(z, y, x + 1), at(z + 1, y, x + 1));
         }
     }
     __syncthreads();
     for (int i = threadIdx.y; i < 32; i += blockDim.y) {
         const int x = x0 + i, y = y0 + threadIdx.x;
-        if (y < nx && x < nx) cy[z * plane + (int64_t)x * nx + y] = tile[threadIdx.x][i];
+        if (y < nx && x < nx) cy[((int64_t)z * nx + x) * pitch + y] = tile[threadIdx.x][i];
     }
 }
 
@@ -762,6 +837,17 @@ ellipsoid_kernel(FpParams p, const float* __restrict__ angles, const float* __re
     sgm[((int64_t)iv * p.views + j) * p.nu + iu] = (float)total;
 }
 
+// Elements per row of the gather copies: from 128 columns, 3 more than a multiple of 8,
+// so that the same column of neighbouring rows lies in different 16-byte L1 banks
+// (unpadded / 3 more, by cells: 512x512x256, 1080 views 181.8 / 171.9 ms; 128x128x64, 270
+// views 0.819 / 0.800 ms; 1 to 7 more are within 0.7 %).  Narrower volumes and those whose
+// padded copy would reach 2^31 elements are not padded.
+inline int copy_pitch(const mct_geom* g) {
+    const int pitch = ((g->nx + 7) & ~7) + 3;
+    return g->nx >= 128 && (int64_t)g->nz * g->nx * pitch < ((int64_t)1 << 31) ? pitch : g->nx;
+}
+inline size_t copy_elems(const mct_geom* g) { return (size_t)g->nz * g->nx * copy_pitch(g); }
+
 int make_params(const mct_geom* g, FpParams& p, const char* who) {
     MCT_TRY(check_geom(g, who));
     MCT_TRY(check_whole_scan(g, who));
@@ -793,6 +879,7 @@ int make_params(const mct_geom* g, FpParams& p, const char* who) {
     p.bcs = 5;  // 32 columns x 8 rows of one view, warps of 32 columns
     p.wcs = 5;
     p.rs = 0;
+    p.pitch = g->nx;
     return MCT_OK;
 }
 
@@ -808,7 +895,7 @@ size_t mct_fp_workspace_size(const mct_geom* g) {
     const size_t n = (size_t)g->nz * g->nx * g->nx;
     // cone beam: two float32 quad copies (16 bytes per voxel each); fan beam: one
     // transposed copy
-    return (g->flags & MCT_CONE) ? 2 * n * sizeof(Quad16) : n * sizeof(float);
+    return (g->flags & MCT_CONE) ? 2 * copy_elems(g) * sizeof(Quad16) : n * sizeof(float);
 }
 
 size_t mct_fp_storage_workspace_size(const mct_geom* g, int32_t dtype) {
@@ -816,7 +903,7 @@ size_t mct_fp_storage_workspace_size(const mct_geom* g, int32_t dtype) {
     if (dtype == MCT_F32) return mct_fp_workspace_size(g);
     if (!(g->flags & MCT_CONE) || (dtype != MCT_BF16 && dtype != MCT_F16)) return 0;
     // two 16-bit cell copies (+16 bytes for the float16 scale's source maximum)
-    return 2 * (size_t)g->nz * g->nx * g->nx * sizeof(uint4) + (dtype == MCT_F16 ? 16 : 0);
+    return 2 * copy_elems(g) * sizeof(uint4) + (dtype == MCT_F16 ? 16 : 0);
 }
 
 }  // extern "C"
@@ -851,41 +938,38 @@ int fp_storage_impl(const mct_geom* g, const mct_tables* t, const TIN* vol_in, c
         return MCT_OK;
     }
     dim3 tb(32, 8), tg((g->nx + 31) / 32, (g->nx + 31) / 32, g->nz);
-    // Ray tiles with copies: 16 detector columns x 16 consecutive views of one row
-    // (float32 quads) or 16 columns x 4 views x 4 rows (16-bit cells), warps of 4
-    // columns x 8 (view, row) slots.  The rays of neighbouring views cross nearly the
-    // same cells at the same step, so a compact warp touches fewer L1 lines per
-    // reload than 32 columns of one view.  Measured at 512x512x256 / 1080 views
-    // (float32 / bf16 ms): 32 columns x 8 views with warps of 32 columns 263.6 / 230.5,
-    // of 8 x 4 248.1 / 223.3, of 4 x 8 244.7 / 223.5; 16 x 16 views with warps of
-    // 4 x 8 237.2 / 224.0 (bf16 with 4 views x 4 rows: 222.2), 2 x 16 244.8 / 222.9,
-    // 8 x 4 240.8 / 224.2; 8 x 32 views with warps of 2 x 16 245.4 / 226.9, 1 x 32
-    // 255.9 / 227.1.  Short scans keep 4 views x 4 rows: float32 at 512x512x128 / 90
-    // views 12.96 ms against 14.34 with 16 views (512x512x64 / 360 views: 21.55 against
-    // 20.92).  Without copies: 32 columns x 8 rows of one view.
-    // The 16-view tiles take 4 rows in turn per view group (row tile, then view group):
-    // neighbouring rows' rays cross nearly the same cells, and the outer rows' slab (up
-    // to ~50 planes) does not fit L2 across all views.  DRAM per launch at 512x512x256 /
-    // 1080 views: 31.3 GB with one row at a time, 19.1 GB with 2 (236.3 ms), 12.8 GB
-    // with 4 (237.8 ms against 237.6), 10.7 GB with 8 (238.7 ms); the 16-bit tiles already
-    // span 4 rows (2 more in turn: 219.7 against 215.9 ms).
-    if (p.cone && workspace) {
-        p.vshift = (dtype == MCT_F32 && g->views >= 256) ? 4 : 2;
-        p.bcs = 4;
-        p.wcs = 2;
-        p.rs = p.vshift == 4 ? 2 : 0;
-    }
+    // Ray tiles: 16 detector columns x 16 consecutive views of one row, warps of 2^wcs
+    // columns.  The rays of neighbouring views cross nearly the same cells, the more so the
+    // closer the views, so long scans take warps of 4 columns x 8 views and short ones 16
+    // columns x 2 views.  float32, ms with 4 / 16 columns per warp: 512x512x256, 1080 views
+    // 159.0 / 168.7; 128x128x64, 270 views 0.698 / 0.741; 512x512x64: 180 views 8.68 / 8.28,
+    // 90 views 5.23 / 4.86, 60 views 3.74 / 3.48.  16-bit cells of short scans keep 4
+    // views x 4 rows: bf16 512x512x128, 90 views 7.60 ms against 7.73 with 16 views.  Fan
+    // beam: warps of 8 columns x 4 views (512^2, 720 views, 4 / 8 / 16 columns: 0.604 /
+    // 0.596 / 0.595; 128^2 x 16, 360 views 0.327 / 0.324 / 0.339; one row of 32 columns x 8
+    // rows, 7 of them idle for one slice: 0.664).
+    // With copies, 4 row tiles are taken in turn per view group: neighbouring rows' rays
+    // cross nearly the same cells, and the outer rows' slab (up to ~50 planes) does not fit
+    // L2 across all views.  Otherwise row tiles are only grouped where the grid needs it.
+    const bool copies = p.cone && workspace;
+    const bool long_scan = g->views >= 256;
+    p.bcs = 4;
+    p.vshift = copies && dtype != MCT_F32 && !long_scan ? 2 : 4;
+    p.wcs = !p.cone ? 3 : long_scan ? 2 : 4;
+    p.rs = copies ? (p.vshift == 4 ? 2 : 0) : (g->nv > 65535 ? 3 : 0);
+    if (copies) p.pitch = copy_pitch(g);
+    const bool windows = g->nx >= 256;  // float32 quads; fan beam always (its warps span more cells)
     const int vb = 1 << p.vshift, rb = 1 << (8 - p.bcs - p.vshift + p.rs), cb = 1 << p.bcs;
     dim3 block(32, 8), grid((g->nu + cb - 1) / cb, ((g->views + vb - 1) / vb) << p.rs, (g->nv + rb - 1) / rb);
-    const size_t n = (size_t)g->nz * g->nx * g->nx;
-    if (p.cone && workspace && dtype == MCT_BF16) {
+    const size_t n = copy_elems(g);
+    if (copies && dtype == MCT_BF16) {
         uint4* cx = static_cast<uint4*>(workspace);
         uint4* cy = cx + n;
-        cell16_kernel<false><<<tg, tb, 0, s>>>(g->nx, g->nz, vol_in, cx, cy, nullptr);
+        cell16_kernel<false><<<tg, tb, 0, s>>>(g->nx, g->nz, p.pitch, vol_in, cx, cy, nullptr);
         MCT_TRY(launched("cell16_kernel"));
-        fp_kernel<true, true, uint4><<<grid, block, 0, s>>>(p, t->angles, t->u, t->v, t->cz, t->pmat_a, t->pmat_xs, vol,
+        fp_kernel<true, true, uint4, false><<<grid, block, 0, s>>>(p, t->angles, t->u, t->v, t->cz, t->pmat_a, t->pmat_xs, vol,
                                                             nullptr, cx, cy, mask, sgm, nullptr);
-    } else if (p.cone && workspace && dtype == MCT_F16) {
+    } else if (copies && dtype == MCT_F16) {
         uint4* cx = static_cast<uint4*>(workspace);
         uint4* cy = cx + n;
         uint32_t* vmax = reinterpret_cast<uint32_t*>(cy + n);
@@ -894,22 +978,23 @@ int fp_storage_impl(const mct_geom* g, const mct_tables* t, const TIN* vol_in, c
             set_error("mct_fp: %s", cudaGetErrorString(e));
             return MCT_E_CUDA;
         }
-        const int64_t blocks = ((int64_t)n + 255) / 256;
-        vol_absmax_kernel<<<(int)(blocks < 152 * 32 ? blocks : 152 * 32), 256, 0, s>>>((int64_t)n, vol_in, vmax);
+        const int64_t voxels = vol_elems(*g), blocks = (voxels + 255) / 256;
+        vol_absmax_kernel<<<(int)(blocks < 152 * 32 ? blocks : 152 * 32), 256, 0, s>>>(voxels, vol_in, vmax);
         MCT_TRY(launched("vol_absmax_kernel"));
-        cell16_kernel<true><<<tg, tb, 0, s>>>(g->nx, g->nz, vol_in, cx, cy, vmax);
+        cell16_kernel<true><<<tg, tb, 0, s>>>(g->nx, g->nz, p.pitch, vol_in, cx, cy, vmax);
         MCT_TRY(launched("cell16_kernel"));
-        fp_kernel<true, true, h16x8><<<grid, block, 0, s>>>(p, t->angles, t->u, t->v, t->cz, t->pmat_a, t->pmat_xs, vol,
+        fp_kernel<true, true, h16x8, false><<<grid, block, 0, s>>>(p, t->angles, t->u, t->v, t->cz, t->pmat_a, t->pmat_xs, vol,
                                                             nullptr, reinterpret_cast<const h16x8*>(cx),
                                                             reinterpret_cast<const h16x8*>(cy), mask, sgm, vmax);
-    } else if (p.cone && workspace) {
+    } else if (copies) {
         Quad16* cx = static_cast<Quad16*>(workspace);
         Quad16* cy = cx + n;
-        quad32_kernel<<<tg, tb, 0, s>>>(g->nx, g->nz, vol_in, reinterpret_cast<float4*>(cx),
+        quad32_kernel<<<tg, tb, 0, s>>>(g->nx, g->nz, p.pitch, vol_in, reinterpret_cast<float4*>(cx),
                                         reinterpret_cast<float4*>(cy));
         MCT_TRY(launched("quad32_kernel"));
-        fp_kernel<true, true, Quad16><<<grid, block, 0, s>>>(p, t->angles, t->u, t->v, t->cz, t->pmat_a, t->pmat_xs,
-                                                             vol, nullptr, cx, cy, mask, sgm, nullptr);
+        auto go = windows ? fp_kernel<true, true, Quad16, true> : fp_kernel<true, true, Quad16, false>;
+        go<<<grid, block, 0, s>>>(p, t->angles, t->u, t->v, t->cz, t->pmat_a, t->pmat_xs, vol, nullptr, cx, cy, mask, sgm,
+                                  nullptr);
     } else if constexpr (kIn32) {
         float* vt = static_cast<float*>(workspace);
         if (vt) {
@@ -917,11 +1002,11 @@ int fp_storage_impl(const mct_geom* g, const mct_tables* t, const TIN* vol_in, c
             MCT_TRY(launched("transpose_xy_kernel"));
         }
         if (p.cone)
-            fp_kernel<true, false, float2><<<grid, block, 0, s>>>(p, t->angles, t->u, t->v, t->cz, t->pmat_a,
+            fp_kernel<true, false, float2, false><<<grid, block, 0, s>>>(p, t->angles, t->u, t->v, t->cz, t->pmat_a,
                                                                   t->pmat_xs, vol, vt, nullptr, nullptr, mask, sgm,
                                                                   nullptr);
         else
-            fp_kernel<false, false, float2><<<grid, block, 0, s>>>(p, t->angles, t->u, t->v, t->cz, t->pmat_a,
+            fp_kernel<false, false, float2, true><<<grid, block, 0, s>>>(p, t->angles, t->u, t->v, t->cz, t->pmat_a,
                                                                    t->pmat_xs, vol, vt, nullptr, nullptr, mask, sgm,
                                                                    nullptr);
     }
