@@ -32,10 +32,12 @@ static_assert(BP_ZC % 2 == 0, "the 16-bit axial loop takes slices in pairs");
 // thread.  The axial kernel needs enough registers to issue all BP_ZC stencil gathers
 // of a view before their arithmetic (that hides the gather latency): measured at
 // 512x512x256 / 1080 views, float32 stencils run fastest with 128 registers (2
-// blocks), bf16 stencils with 80 (3 blocks).  The general modes use 2.
-template <int MODE, typename QT>
+// blocks), bf16 stencils with 80 (3 blocks); 16-bit stencils of a curved detector spill
+// there (512x512x128 / 360 views, FDK: 15.9 ms with 3 blocks, 8.4 with 2).  The general
+// modes use 2.
+template <int MODE, typename QT, bool CURVED>
 constexpr int bp_min_blocks() {
-    return MODE == 0 && sizeof(QT) == 8 ? 3 : 2;
+    return (MODE == 0 || MODE == 2) && sizeof(QT) == 8 && !CURVED ? 3 : 2;
 }
 
 struct BpParams {
@@ -74,11 +76,23 @@ __device__ __forceinline__ void fill_view_table(const BpParams& p, const float* 
 }
 
 // MODE 0: cone beam in any view mode; flat or curved detector, no projection matrix
-//         (u hoisted per column of the kernel's frame)
+//         (u hoisted per column of the kernel's frame); MODE 2: the same for detectors of
+//         more than 2^22 rows
 // MODE 1: fan beam in the coronal or sagittal view mode (per-voxel u)
 // MODE 3: projection matrix geometry in any view mode (per-column matrix rows)
-template <int MODE, bool CONE, typename QT, typename PT>
-__global__ void __launch_bounds__(BP_TX* BP_TY, bp_min_blocks<MODE, QT>())
+// Views between checks whether a column has left the detector (8 and 256 within 0.5 %).
+constexpr int kViewRun = 32;
+
+// 1 / x from the hardware approximation (1 ulp) and one Newton-Raphson step r + r (1 - x r),
+// without the division's branch for special values: 0 and infinities give NaN, which the
+// detector test rejects like the infinite or zero magnification of the division.
+__device__ __forceinline__ float reciprocal(float x) {
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return fmaf(r, fmaf(-x, r, 1.0f), r);
+}
+template <int MODE, bool CONE, typename QT, typename PT, bool CURVED = false>
+__global__ void __launch_bounds__(BP_TX* BP_TY, bp_min_blocks<MODE, QT, CURVED>())
 fdk_bp_kernel(BpParams p, const float* __restrict__ angles, const float* __restrict__ pmat,
               const void* __restrict__ packed, float* __restrict__ vol, const uint32_t* __restrict__ f16_max) {
     // views per chunk of the shared tables; with projection matrices the chunk's 3x4
@@ -122,68 +136,112 @@ fdk_bp_kernel(BpParams p, const float* __restrict__ angles, const float* __restr
         __syncthreads();
         if (!active || dead == 0xffffffffu) continue;
 
-        for (int q = 0; q < nvc; ++q) {
+        if constexpr (MODE == 0 || MODE == 2) {
+            // Cone beam: everything but the row is shared by the column's slices.  Views are
+            // software-pipelined: the next view's geometry (a chain of about 35 dependent
+            // instructions) is computed between the issue of this view's gathers and their
+            // use, in one basic block: the reciprocal has no branch, and a column that leaves
+            // the detector goes on with a clamped index to the end of its run of kViewRun
+            // views.  512x512x256 / 1080 views, FDK: float32 53.7 -> 49.2 ms; 256^3 / 360
+            // views coronal, bf16: 4.55 -> 4.08 ms; 333x333x101 / 500 views, curved 6.42 ->
+            // 5.30 ms (bit-identical).  L1 wavefronts bind now (82 % for float32).
+            static_assert(CONE, "cone-beam modes");
+            struct View {
+                const char* base;  // the view's cell (row 0, column floor(u))
+                float ru, w, vA, vB;  // column fraction, weight; row of slice k = vA + k vB
+            };
+            const float umax = (float)(p.nu - 1);
+            bool off = false;
+            auto geometry = [&](int q) {
+                const float4 tb = tab[q];
+                const float cb = tb.x, sb = tb.y;
+                const float L = p.sid - c0x * cb - c0y * sb;
+                const float t = -c0x * sb + c0y * cb;
+                const float rL = reciprocal(L);  // for the magnification and the flat distance weight
+                const float mag = p.sdd * rL;
+                // products rounded on their own: a detector index that fuses them differs by an
+                // ulp, and voxels at the detector's edge would change sides
+                const float u = CURVED ? __fmul_rn(p.sdd, atan2f(t, L)) : __fmul_rn(mag, t);
+                const float ui = (u - p.u0) * p.inv_ustep;
+                off |= !(ui >= 0.0f && ui + 1.0f <= umax);  // NaN counts as off-detector
+                const float uf = floorf(ui);
+                const int uc = min(max((int)uf, 0), p.nu - 2);
+                const float dw = CURVED ? 1.0f / (L * L + t * t) : rL * rL;
+                View v;
+                v.ru = ui - uf;
+                v.w = (p.sid * dw) * tb.z;
+                v.vA = (mag * c0z - p.v0) * p.kv;
+                v.vB = (mag * p.pz_z) * p.kv;
+                v.base = static_cast<const char*>(packed) + ((int64_t)(jc + q) * p.nv * nq + uc) * (int64_t)sizeof(QT);
+                return v;
+            };
+            // rows outside [0, nv-2] (negative ones wrap around) read the NaN row nv-1
+            const unsigned nan_row = (unsigned)(p.nv - 1);
+            const uint32_t stride = (uint32_t)(nq * sizeof(QT));
+            View cur = geometry(0);
+            for (int q0 = 0; q0 < nvc && !off; q0 += kViewRun) {
+                const int q1 = min(q0 + kViewRun, nvc);
+                for (int q = q0; q < q1; ++q) {
+                    const float2 ru2 = make_float2(cur.ru, cur.ru);
+                    float2 lo[BP_ZC], hi[BP_ZC];
+                    float rv[BP_ZC];
+                    auto load = [&](int k, unsigned row) {
+                        Quad<QT>::load(reinterpret_cast<const QT*>(cur.base + (uint64_t)min(row, nan_row) * stride), lo[k],
+                                       hi[k]);
+                    };
+                    // floor by adding M = 1.5 * 2^23 rounded down, on the FMA pipe: exact for
+                    // rows below 2^22 (MODE 2: taller detectors, on the conversion unit); any
+                    // other value leaves the difference to M's bits above nan_row.  float32
+                    // takes slices in pairs (f32x2), 16 bits one by one: 49.2 / 49.4 ms and
+                    // 4.14 / 4.08 ms at the sizes above.
+                    const float M = 12582912.0f;
+                    const unsigned MB = 0x4B400000u;  // M's bits
+                    if constexpr (MODE == 2) {
+#pragma unroll
+                        for (int k = 0; k < BP_ZC; ++k) {
+                            const float vi = fmaf((float)k, cur.vB, cur.vA);
+                            const float vf = floorf(vi);
+                            rv[k] = vi - vf;
+                            load(k, (unsigned)(int)vf);
+                        }
+                    } else if constexpr (sizeof(QT) == 16) {
+                        const float2 vA2 = make_float2(cur.vA, cur.vA), vB2 = make_float2(cur.vB, cur.vB);
+#pragma unroll
+                        for (int k = 0; k < BP_ZC; k += 2) {
+                            const float2 vi = __ffma2_rn(make_float2((float)k, (float)(k + 1)), vB2, vA2);
+                            const float2 m = __fadd2_rd(vi, make_float2(M, M));
+                            const float2 fl = __fadd2_rn(m, make_float2(-M, -M));
+                            const float2 f = __fadd2_rn(vi, make_float2(-fl.x, -fl.y));
+                            rv[k] = f.x;
+                            rv[k + 1] = f.y;
+                            load(k, __float_as_uint(m.x) - MB);
+                            load(k + 1, __float_as_uint(m.y) - MB);
+                        }
+                    } else {
+#pragma unroll
+                        for (int k = 0; k < BP_ZC; ++k) {
+                            const float vi = fmaf((float)k, cur.vB, cur.vA);
+                            const float m = __fadd_rd(vi, M);
+                            rv[k] = vi - (m - M);
+                            load(k, __float_as_uint(m) - MB);
+                        }
+                    }
+                    const View next = geometry(min(q + 1, nvc - 1));
+                    const float w = cur.w;
+#pragma unroll
+                    for (int k = 0; k < BP_ZC; ++k) {
+                        const float2 s2 = __ffma2_rn(ru2, hi[k], lo[k]);
+                        acc[k] = fmaf(w, fmaf(rv[k], s2.y, s2.x), acc[k]);
+                    }
+                    cur = next;
+                }
+            }
+            if (off) dead = 0xffffffffu;
+        } else for (int q = 0; q < nvc; ++q) {
             const int j = jc + q;
             const float4 tb = tab[q];
             const float cb = tb.x, sb = tb.y;
-            if (MODE == 0) {
-                // u is shared by the whole column (cone beam: axial fan beam has its own kernel)
-                static_assert(MODE != 0 || CONE, "MODE 0 is the cone-beam kernel");
-                const float L = p.sid - c0x * cb - c0y * sb;
-                const float t = -c0x * sb + c0y * cb;
-                const float rL = 1.0f / L;  // one reciprocal for the magnification and the flat distance weight
-                const float mag = p.sdd * rL;
-                const float u = p.curved ? p.sdd * atan2f(t, L) : mag * t;
-                const float ui = (u - p.u0) * p.inv_ustep;
-                if (!(ui >= 0.0f && ui + 1.0f <= (float)(p.nu - 1))) {  // NaN counts as off-detector
-                    dead = 0xffffffffu;
-                    break;
-                }
-                const float uf = floorf(ui);
-                const float ru = ui - uf;
-                const int uc = (int)uf;
-                const float dw = p.curved ? 1.0f / (L * L + t * t) : rL * rL;
-                const float w = (p.sid * dw) * tb.z;
-                const float vA = (mag * c0z - p.v0) * p.kv;
-                const float vB = (mag * p.pz_z) * p.kv;
-                const QT* base = reinterpret_cast<const QT*>(packed) + (int64_t)j * p.nv * nq + uc;
-                const float2 ru2 = make_float2(ru, ru);
-                const unsigned nan_row = (unsigned)(p.nv - 1);
-                if constexpr (sizeof(QT) == 8) {
-                    // 16-bit operands: slices in pairs, row index and weight as f32x2
-                    // (the same values; at 512x512x256 / 1080 views bf16 48.9 ms
-                    // against 49.7, float32 53.6 against 52.3, so float32 keeps the
-                    // scalar loop)
-                    const float2 vA2 = make_float2(vA, vA), vB2 = make_float2(vB, vB);
-#pragma unroll
-                    for (int k = 0; k < BP_ZC; k += 2) {
-                        const float2 vi = __ffma2_rn(make_float2((float)k, (float)(k + 1)), vB2, vA2);
-                        const float vf0 = floorf(vi.x), vf1 = floorf(vi.y);
-                        const unsigned vr0 = min((unsigned)(int)vf0, nan_row);
-                        const unsigned vr1 = min((unsigned)(int)vf1, nan_row);
-                        const float2 rv = __fadd2_rn(vi, make_float2(-vf0, -vf1));
-                        float2 lo0, hi0, lo1, hi1;
-                        Quad<QT>::load(base + vr0 * (unsigned)nq, lo0, hi0);
-                        Quad<QT>::load(base + vr1 * (unsigned)nq, lo1, hi1);
-                        const float2 s0 = __ffma2_rn(ru2, hi0, lo0), s1 = __ffma2_rn(ru2, hi1, lo1);
-                        acc[k] = fmaf(w, fmaf(rv.x, s0.y, s0.x), acc[k]);
-                        acc[k + 1] = fmaf(w, fmaf(rv.y, s1.y, s1.x), acc[k + 1]);
-                    }
-                } else {
-#pragma unroll
-                    for (int k = 0; k < BP_ZC; ++k) {
-                        const float vi = fmaf((float)k, vB, vA);
-                        const float vf = floorf(vi);
-                        // rows outside [0, nv-2] (negative ones wrap around) read the NaN row
-                        const unsigned vr = min((unsigned)(int)vf, nan_row);
-                        const float rv = vi - vf;
-                        float2 lo, hi;
-                        Quad<QT>::load(base + vr * (unsigned)nq, lo, hi);
-                        const float2 s2 = __ffma2_rn(ru2, hi, lo);
-                        acc[k] = fmaf(w, fmaf(rv, s2.y, s2.x), acc[k]);
-                    }
-                }
-            } else if (MODE == 3) {
+            if (MODE == 3) {
                 // Projection matrices: in the kernel's frame x and y are fixed per column, so
                 // the matrix rows are affine in the slice index and the distance weight does
                 // not depend on z.  An untilted trajectory has no z term in the u and depth
@@ -405,15 +463,15 @@ void launch_bp_fan(const BpParams& p, const mct_geom* g, cudaStream_t s, const f
         fdk_bp_fan_kernel<ZC, float2><<<grid, block, 0, s>>>(p, angles, packed, vol, nullptr);
 }
 
-template <int MODE, bool CONE>
+template <int MODE, bool CONE, bool CURVED = false>
 void launch_bp(const BpParams& p, dim3 grid, dim3 block, cudaStream_t s, const float* angles, const float* pmat,
                const void* packed, int dtype, float* vol, const uint32_t* f16_max) {
     if (dtype == MCT_BF16)
-        fdk_bp_kernel<MODE, CONE, uint2, uint32_t><<<grid, block, 0, s>>>(p, angles, pmat, packed, vol, nullptr);
+        fdk_bp_kernel<MODE, CONE, uint2, uint32_t, CURVED><<<grid, block, 0, s>>>(p, angles, pmat, packed, vol, nullptr);
     else if (dtype == MCT_F16)
-        fdk_bp_kernel<MODE, CONE, h16x4, h16x2><<<grid, block, 0, s>>>(p, angles, pmat, packed, vol, f16_max);
+        fdk_bp_kernel<MODE, CONE, h16x4, h16x2, CURVED><<<grid, block, 0, s>>>(p, angles, pmat, packed, vol, f16_max);
     else
-        fdk_bp_kernel<MODE, CONE, float4, float2><<<grid, block, 0, s>>>(p, angles, pmat, packed, vol, nullptr);
+        fdk_bp_kernel<MODE, CONE, float4, float2, CURVED><<<grid, block, 0, s>>>(p, angles, pmat, packed, vol, nullptr);
 }
 
 }  // namespace
@@ -491,6 +549,11 @@ extern "C" int mct_fdk_bp(const mct_geom* g, const mct_tables* t, const void* pa
     cudaStream_t s = as_stream(stream);
     const uint32_t* fm = dtype == MCT_F16 ? f16_trailer(g, packed) : nullptr;
     if (pm) launch_bp<3, true>(p, grid, block, s, t->angles, t->pmatrix, packed, dtype, vol, fm);
+    else if (cone && g->nv > (1 << 22) && p.curved)
+        launch_bp<2, true, true>(p, grid, block, s, t->angles, nullptr, packed, dtype, vol, fm);
+    else if (cone && g->nv > (1 << 22))
+        launch_bp<2, true>(p, grid, block, s, t->angles, nullptr, packed, dtype, vol, fm);
+    else if (cone && p.curved) launch_bp<0, true, true>(p, grid, block, s, t->angles, nullptr, packed, dtype, vol, fm);
     else if (cone) launch_bp<0, true>(p, grid, block, s, t->angles, nullptr, packed, dtype, vol, fm);
     else if (g->view_mode == 1) {
         MCT_REQUIRE(g->nx <= 65535, "mct_fdk_bp: fan beam images are at most 65535 pixels wide");

@@ -1,0 +1,64 @@
+"""The cone-beam backprojector's software-pipelined view loop where it could go wrong: scans of
+fewer views than a run of views, of one more and one less, columns that leave the detector in
+the first, a middle or the last view of a run, curved detectors, 16-bit operands, and
+detectors too tall for row indices from the float32 rounding constant."""
+import numpy as np
+import pytest
+
+from conftest import rel_l2
+from oracle import fbp_ops as F
+from test_gpu_parity import _cone_obj
+
+pytestmark = pytest.mark.gpu
+
+# float32 sums against float64: 1e-4 as for the other operators; 16-bit operands round the base
+# value of each cell by 2^-9 (bf16) or 2^-12 (float16) of its size, on noise with zero mean by
+# up to twice that relative to the sum.
+TOL = {"f32": 1e-4, "bf16": 2.0 ** -8, "f16": 2.0 ** -11}
+
+
+@pytest.mark.parametrize("views,storage,kw", [
+    (2, "f32", {}), (31, "f32", {}), (32, "f32", {}), (33, "f32", {"CurvedDetector": True}), (65, "f32", {}),
+    (65, "bf16", {}), (33, "bf16", {"CurvedDetector": True}), (33, "f16", {"ReconViewMode": "coronal"}),
+    (40, "f32", {"TotalScanAngle": 220, "ReconViewMode": "sagittal"})])
+def test_backprojection_matches_the_oracle_with_truncated_columns(views, storage, kw, cuda):
+    import torch
+    from reconstruction_program_taichi_gb300 import geometry, ops
+    # the detector is narrower than the image: its corners and edges leave it in some view
+    o = _cone_obj(n=37, nz=18, nu=34, nv=30, views=views, **kw)
+    dg = geometry.fbp_geometry(o)
+    g = dg.geom
+    rng = np.random.default_rng(views)
+    f = rng.normal(0, 1, (views, g.nv, g.nu)).astype(np.float32)
+    dtype = {"f32": ops.MCT_F32, "bf16": ops.MCT_BF16, "f16": ops.MCT_F16}[storage]
+    x = torch.from_numpy(f).cuda()
+    got = ops.fdk_bp(dg, ops.pack(dg, x, dtype), dtype).cpu().numpy()
+    u, v, ang = geometry.fbp_arrays(o)
+    ref = F.fdk_bp(f.transpose(1, 0, 2), ang, u, v, nx=o.img_dim, nz=o.img_dim_z, px=o.img_pix_size,
+                   pz=o.img_voxel_height, cx=o.img_center_x, cy=o.img_center_y, cz=o.img_center_z,
+                   sid=o.source_isocenter_dis, sdd=o.source_det_dis, dv=o.det_elem_height, img_rot=o.img_rot,
+                   total_scan_angle=o.total_scan_angle, short_scan=o.short_scan, cone_beam=True,
+                   curved=o.curved_dect, view_mode=o.recon_view_mode)
+    assert 0.05 < np.mean(ref == 0) < 0.95
+    # voxels within float32 rounding of the detector's edge may fall on either side
+    assert np.mean((got == 0) != (ref == 0)) < 1e-3
+    both = (got != 0) & (ref != 0)
+    assert rel_l2(got[both], ref[both]) < TOL[storage]
+
+
+def test_detector_of_more_than_2_22_rows_gives_the_same_volume(cuda):
+    """A detector whose first rows are the small one's and hold everything the volume reads:
+    the same row indices through the tall detectors' floor, so the same bits."""
+    import torch
+    from reconstruction_program_taichi_gb300 import geometry, ops
+    o = _cone_obj(n=8, nz=4, nu=8, nv=24, views=2, DetectorElementWidth=2.0)
+    dg = geometry.fbp_geometry(o)
+    rng = np.random.default_rng(3)
+    f = torch.from_numpy(rng.normal(0, 1, (2, 24, 8)).astype(np.float32)).cuda()
+    small = ops.fdk_bp(dg, ops.pack(dg, f))
+    dg.geom = dg.geom.copy(nv=(1 << 22) + 3)
+    tall = torch.zeros((2, dg.geom.nv, 8), device="cuda")
+    tall[:, :24] = f
+    got = ops.fdk_bp(dg, ops.pack(dg, tall))
+    assert float((small != 0).float().mean()) > 0.5
+    assert torch.equal(got, small)
