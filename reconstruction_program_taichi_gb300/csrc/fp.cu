@@ -203,13 +203,17 @@ __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
     return *reinterpret_cast<uint32_t*>(&b);
 }
 
+// How a ray's interior samples are summed: by cells, by cells in windows, or one by one.
+enum Walk { kCells, kWindows, kSamples };
+
 // Resident blocks per SM that the register allocation of fp_kernel targets: 5 (48
 // registers) with copies.  512x512x256 / 1080 views, float32: 4 blocks 160.6 ms, 5
 // 158.9, 6 164.7; 512x512x64 / 360 views, bf16: 4 blocks 13.55 ms, 5 13.41, 6 14.27.
-// The fan-beam path needs 40 registers (6 blocks).
-template <bool CONE>
+// The fan-beam path needs 40 registers (6 blocks), the walk by samples 62 (4; 5 blocks
+// cost it 10 %).
+template <bool CONE, int WALK>
 constexpr int fp_min_blocks() {
-    return CONE ? 5 : 6;
+    return WALK == kSamples ? 4 : CONE ? 5 : 6;
 }
 
 // Above this many steps a ray's indices are no longer exact in float32 (and would not
@@ -246,8 +250,11 @@ constexpr int kWinPlanes = 64;
 //     512x512x64, 360 views, bf16          18.32 / 13.41 / 14.9 (windows: 16-bit cells lose)
 //     512^2 fan beam, 720 views            1.34 / 0.80 / 0.66
 //     256x256x128, 360 views, step 0.1     18.83 / 7.19;  step 0.5: 6.20 / 5.95
-template <bool CONE, bool ZP, typename ZT, bool WIN>
-__global__ void __launch_bounds__(256, fp_min_blocks<CONE>())
+// 16-bit cells, which the walk by samples reloads with one load and which cells hold twice
+// the arithmetic for, are walked by samples from the step on where it is the faster
+// (walk_by_samples below): each keeps its cell in registers until it enters another.
+template <bool CONE, bool ZP, typename ZT, int WALK>
+__global__ void __launch_bounds__(256, fp_min_blocks<CONE, WALK>())
 fp_kernel(FpParams p, const float* __restrict__ angles, const float* __restrict__ u_arr,
           const float* __restrict__ v_arr, const float* __restrict__ czv, const float* __restrict__ pa,
           const float* __restrict__ pxs, const float* __restrict__ vol, const float* __restrict__ vol_t,
@@ -294,8 +301,9 @@ fp_kernel(FpParams p, const float* __restrict__ angles, const float* __restrict_
         }
         const float xmax = (float)(nx - 1), zmax = (float)(p.nz - 1);
         struct Cell {
-            // trilinear coefficients: corner, x, y and xy differences, each as {value, z-difference}
-            // (float32 quads) or {lower plane, upper plane} (the others)
+            // float32 quads: corner, x, y and xy difference, each {value, z-difference}; the
+            // others: corner and x-difference of row y (e, ex) and of row y + 1 (ey, exy), each
+            // {lower plane, upper plane}
             float2 e, ex, ey, exy;
         };
         auto load_cell = [&](int off, Cell& c) {
@@ -306,22 +314,19 @@ fp_kernel(FpParams p, const float* __restrict__ angles, const float* __restrict_
                 c.ey = make_float2(q0.z, q0.w);
                 c.ex = __fadd2_rn(make_float2(q1.x, q1.y), make_float2(-q0.x, -q0.y));
                 c.exy = __fadd2_rn(make_float2(q1.z, q1.w), make_float2(-q0.z, -q0.w));
-                return;
-            }
-            float2 e00, g00, e10, g10;  // corners and x-differences of the lower and upper z-plane
-            if constexpr (ZP && std::is_same<ZT, uint4>::value) {
+            } else if constexpr (ZP && std::is_same<ZT, uint4>::value) {
                 const uint4 q = __ldg(V2 + off);
-                e00 = bf16x2_to_float2(q.x);
-                g00 = bf16x2_to_float2(q.y);
-                e10 = bf16x2_to_float2(q.z);
-                g10 = bf16x2_to_float2(q.w);
+                c.e = bf16x2_to_float2(q.x);
+                c.ex = bf16x2_to_float2(q.y);
+                c.ey = bf16x2_to_float2(q.z);
+                c.exy = bf16x2_to_float2(q.w);
             } else if constexpr (ZP && std::is_same<ZT, h16x8>::value) {
                 const uint4 q = __ldg(reinterpret_cast<const uint4*>(V2 + off));
-                e00 = h16x2_to_float2(q.x);
-                g00 = h16x2_to_float2(q.y);
-                e10 = h16x2_to_float2(q.z);
-                g10 = h16x2_to_float2(q.w);
-            } else if constexpr (!kQuad) {
+                c.e = h16x2_to_float2(q.x);
+                c.ex = h16x2_to_float2(q.y);
+                c.ey = h16x2_to_float2(q.z);
+                c.exy = h16x2_to_float2(q.w);
+            } else {
                 const float* b = V + off;
                 const float a00 = __ldg(b), a01 = __ldg(b + sx), a10 = __ldg(b + sy), a11 = __ldg(b + sx + sy);
                 float c00 = 0.f, c01 = 0.f, c10 = 0.f, c11 = 0.f;
@@ -329,17 +334,28 @@ fp_kernel(FpParams p, const float* __restrict__ angles, const float* __restrict_
                     const float* u = b + plane;
                     c00 = __ldg(u); c01 = __ldg(u + sx); c10 = __ldg(u + sy); c11 = __ldg(u + sx + sy);
                 }
-                e00 = make_float2(a00, c00);
-                e10 = make_float2(a10, c10);
-                g00 = __fadd2_rn(make_float2(a01, c01), make_float2(-a00, -c00));
-                g10 = __fadd2_rn(make_float2(a11, c11), make_float2(-a10, -c10));
+                c.e = make_float2(a00, c00);
+                c.ey = make_float2(a10, c10);
+                c.ex = __fadd2_rn(make_float2(a01, c01), make_float2(-a00, -c00));
+                c.exy = __fadd2_rn(make_float2(a11, c11), make_float2(-a10, -c10));
             }
-            c.e = e00;
-            c.ex = g00;
-            c.ey = __fadd2_rn(e10, make_float2(-e00.x, -e00.y));
-            c.exy = __fadd2_rn(g10, make_float2(-g00.x, -g00.y));
         };
-        auto dz = [](float2 a) { return kQuad ? a.y : a.y - a.x; };  // the z-difference of a pair
+        auto sub2 = [](float2 a, float2 b) { return __fadd2_rn(a, make_float2(-b.x, -b.y)); };
+        // the cell's value at fractions (xw, yw, zw)
+        auto interp = [&](const Cell& c, float xw, float yw, float zw) -> float {
+            const float2 x2 = make_float2(xw, xw), y2 = make_float2(yw, yw);
+            const float2 l = __ffma2_rn(x2, c.ex, c.e);
+            const float2 l1 = __ffma2_rn(x2, c.exy, c.ey);
+            if constexpr (kQuad) {
+                const float2 pl = __ffma2_rn(y2, l1, l);
+                return fmaf(zw, pl.y, pl.x);
+            }
+            const float2 pl = __ffma2_rn(y2, sub2(l1, l), l);
+            return CONE ? fmaf(zw, pl.y - pl.x, pl.x) : pl.x;
+        };
+        Cell cur;       // the last sample's cell: kSamples reloads it only when a ray enters another
+        int cell = -1;
+        cur.e = cur.ex = cur.ey = cur.exy = make_float2(0.0f, 0.0f);
         // Checked samples at the ends of the range, where the inside test decides; the range
         // between them (at least 1e-3 voxel inside on every axis) is walked cell by cell.
         auto sample = [&](int k) {
@@ -358,13 +374,11 @@ fp_kernel(FpParams p, const float* __restrict__ angles, const float* __restrict_
                 zi = min(max((int)zf, 0), p.nz - 2);
                 zw = fz - zf;
             }
-            Cell c;
-            load_cell(zi * plane + yi * sy + xi * sx, c);
-            const float xw = fx - xf, yw = fy - yf;
-            const float2 l = __ffma2_rn(make_float2(xw, xw), c.ex, c.e);
-            const float2 gy = __ffma2_rn(make_float2(xw, xw), c.exy, c.ey);
-            const float2 pl = __ffma2_rn(make_float2(yw, yw), gy, l);
-            acc += !ok ? 0.0f : CONE ? fmaf(zw, dz(pl), pl.x) : pl.x;
+            const int off = zi * plane + yi * sy + xi * sx;
+            if (WALK != kSamples || off != cell) load_cell(off, cur);
+            cell = off;
+            const float v = interp(cur, fx - xf, fy - yf, zw);
+            acc += ok ? v : 0.0f;
         };
         int kis, kie;
         interior_range(p, r, CONE, kis, kie);
@@ -403,21 +417,27 @@ fp_kernel(FpParams p, const float* __restrict__ angles, const float* __restrict_
                 float2 m;      // fractions of the run's midpoint
                 float mz, n;   // and its number of samples
             };
-            // the run of samples from fk on that lie in one cell; fk moves past it
-            auto next_run = [&](float& fk, Run& q) {
+            // element of sample fk's cell and the sample's fractions in it
+            auto locate = [&](float fk, float2& w, float& zw) -> int {
                 const float2 f = __ffma2_rn(make_float2(fk, fk), dxy, fxy0);
                 const float2 m = __fadd2_rd(f, M2);
                 const float2 fl = __fadd2_rn(m, nM2);
-                const float2 w = __fadd2_rn(f, make_float2(-fl.x, -fl.y));
+                w = __fadd2_rn(f, make_float2(-fl.x, -fl.y));
                 unsigned off = (unsigned)__float_as_int(m.x) * (unsigned)sx + (unsigned)__float_as_int(m.y) * (unsigned)sy - obias;
-                float zw = 0.0f;
+                zw = 0.0f;
                 if (CONE) {
                     const float fz = fmaf(fk, r.dfz, r.fz0);
                     const float mz = __fadd_rd(fz, M);
                     zw = fz - (mz - M);
                     off += (unsigned)__float_as_int(mz) * (unsigned)plane;
                 }
-                load_cell((int)off, q.c);
+                return (int)off;
+            };
+            // the run of samples from fk on that lie in one cell; fk moves past it
+            auto next_run = [&](float& fk, Run& q) {
+                float2 w;
+                float zw;
+                load_cell(locate(fk, w, zw), q.c);
                 const float2 t2 = __ffma2_rn(w, B2, A2);
                 float t = fminf(fminf(t2.x, t2.y), kend - fk);
                 if (CONE) t = fminf(t, fmaf(zw, Bz, Az));
@@ -431,23 +451,41 @@ fp_kernel(FpParams p, const float* __restrict__ angles, const float* __restrict_
             auto add_run = [&](const Run& q) {
                 const float2 x2 = make_float2(q.m.x, q.m.x), y2 = make_float2(q.m.y, q.m.y);
                 const float2 l = __ffma2_rn(x2, q.c.ex, q.c.e);
-                const float2 gy = __ffma2_rn(x2, q.c.exy, q.c.ey);
-                const float2 pl = __ffma2_rn(y2, gy, l);
-                float v = pl.x, corr = cxy * q.c.exy.x;
-                if constexpr (CONE && kQuad) {
+                float v, corr;
+                if constexpr (kQuad) {
+                    const float2 gy = __ffma2_rn(x2, q.c.exy, q.c.ey);
+                    const float2 pl = __ffma2_rn(y2, gy, l);
                     v = fmaf(q.mz, pl.y, pl.x);
                     corr = fmaf(cxy, fmaf(q.mz, q.c.exy.y, q.c.exy.x),
                                 fmaf(cxz, fmaf(q.m.y, q.c.exy.y, q.c.ex.y), cyz * gy.y));
-                } else if constexpr (CONE) {
-                    const float2 gx = __ffma2_rn(y2, q.c.exy, q.c.ex);
-                    v = fmaf(q.mz, pl.y - pl.x, pl.x);
-                    corr = fmaf(cxy, fmaf(q.mz, q.c.exy.y - q.c.exy.x, q.c.exy.x),
-                                fmaf(cxz, gx.y - gx.x, cyz * (gy.y - gy.x)));
+                } else {
+                    const float2 gxy = sub2(q.c.exy, q.c.ex);
+                    const float2 gy = __ffma2_rn(x2, gxy, sub2(q.c.ey, q.c.e));
+                    const float2 pl = __ffma2_rn(y2, gy, l);
+                    v = pl.x;
+                    corr = cxy * gxy.x;
+                    if (CONE) {
+                        const float2 gx = __ffma2_rn(y2, gxy, q.c.ex);
+                        v = fmaf(q.mz, pl.y - pl.x, pl.x);
+                        corr = fmaf(cxy, fmaf(q.mz, gxy.y - gxy.x, gxy.x), fmaf(cxz, gx.y - gx.x, cyz * (gy.y - gy.x)));
+                    }
                 }
                 acc = fmaf(q.n, fmaf(fmaf(q.n, q.n, -1.0f), corr, v), acc);
             };
             float fk = (float)kis;
-            if constexpr (WIN) {
+            if constexpr (WALK == kSamples) {
+// 256x256x64 / 360 views, bf16, step 0.3: 3.28 / 3.22 / 3.29 ms unrolled 2 / 3 / 4
+#pragma unroll 3
+                for (int k = kis; k <= kie; ++k, fk += 1.0f) {
+                    float2 w;
+                    float zw;
+                    const int off = locate(fk, w, zw);
+                    if (off != cell) load_cell(off, cur);
+                    cell = off;
+                    acc += interp(cur, w.x, w.y, zw);
+                }
+            }
+            if constexpr (WALK == kWindows) {
                 // window i ends at plane i * kWinPlanes along the rays' main axis, counted
                 // from the side that they enter through: step w0 + i * wi
                 const float ds = tr && !kQuad ? r.dfx : r.dfy, s0 = tr && !kQuad ? r.fx0 : r.fy0;
@@ -462,7 +500,7 @@ fp_kernel(FpParams p, const float* __restrict__ angles, const float* __restrict_
                     }
                 }
             }
-            while (fk <= kend) {
+            while (WALK != kSamples && fk <= kend) {
                 Run q;
                 next_run(fk, q);
                 add_run(q);
@@ -846,6 +884,16 @@ inline int copy_pitch(const mct_geom* g) {
     const int pitch = ((g->nx + 7) & ~7) + 3;
     return g->nx >= 128 && (int64_t)g->nz * g->nx * pitch < ((int64_t)1 << 31) ? pitch : g->nx;
 }
+// Whether 16-bit cells are walked by samples: few samples per cell (the ray's cell
+// crossings per voxel length are 1.33 on average over a scan).  256x256x64, 360 views, by
+// samples / by cells, ms: bf16 step 0.2 (2.2 samples per cell) 4.84 / 3.46, 0.3 (1.4) 3.22 /
+// 3.31 (140 columns, 300 views: 0.929 / 0.966), 0.5 (0.9) 2.1 / 2.95; float16, which pays
+// more per load, 0.3 3.8 / 3.60, 0.5 2.33 / 3.19.
+inline bool walk_by_samples(const mct_geom* g, int32_t dtype) {
+    if (dtype == MCT_F32) return false;
+    const double step = g->fp_step * std::sqrt(2.0 + ((double)g->pz / g->px) * ((double)g->pz / g->px));
+    return 1.0 / (1.33 * step) < (dtype == MCT_BF16 ? 1.5 : 1.2);
+}
 inline size_t copy_elems(const mct_geom* g) { return (size_t)g->nz * g->nx * copy_pitch(g); }
 
 int make_params(const mct_geom* g, FpParams& p, const char* who) {
@@ -943,8 +991,9 @@ int fp_storage_impl(const mct_geom* g, const mct_tables* t, const TIN* vol_in, c
     // closer the views, so long scans take warps of 4 columns x 8 views and short ones 16
     // columns x 2 views.  float32, ms with 4 / 16 columns per warp: 512x512x256, 1080 views
     // 159.0 / 168.7; 128x128x64, 270 views 0.698 / 0.741; 512x512x64: 180 views 8.68 / 8.28,
-    // 90 views 5.23 / 4.86, 60 views 3.74 / 3.48.  16-bit cells of short scans keep 4
-    // views x 4 rows: bf16 512x512x128, 90 views 7.60 ms against 7.73 with 16 views.  Fan
+    // 90 views 5.23 / 4.86, 60 views 3.74 / 3.48.  16-bit cells take 4 views x 4 rows: bf16
+    // 512x512x128, 90 views 7.60 ms against 7.73 with 16 views; 256x256x64, 360 views 3.457
+    // against 3.480; by samples they keep warps of 4 columns.  Fan
     // beam: warps of 8 columns x 4 views (512^2, 720 views, 4 / 8 / 16 columns: 0.604 /
     // 0.596 / 0.595; 128^2 x 16, 360 views 0.327 / 0.324 / 0.339; one row of 32 columns x 8
     // rows, 7 of them idle for one slice: 0.664).
@@ -952,10 +1001,10 @@ int fp_storage_impl(const mct_geom* g, const mct_tables* t, const TIN* vol_in, c
     // cross nearly the same cells, and the outer rows' slab (up to ~50 planes) does not fit
     // L2 across all views.  Otherwise row tiles are only grouped where the grid needs it.
     const bool copies = p.cone && workspace;
-    const bool long_scan = g->views >= 256;
+    const bool long_scan = g->views >= 256, by_samples = copies && walk_by_samples(g, dtype);
     p.bcs = 4;
-    p.vshift = copies && dtype != MCT_F32 && !long_scan ? 2 : 4;
-    p.wcs = !p.cone ? 3 : long_scan ? 2 : 4;
+    p.vshift = copies && dtype != MCT_F32 ? 2 : 4;
+    p.wcs = !p.cone ? 3 : long_scan || by_samples ? 2 : 4;
     p.rs = copies ? (p.vshift == 4 ? 2 : 0) : (g->nv > 65535 ? 3 : 0);
     if (copies) p.pitch = copy_pitch(g);
     const bool windows = g->nx >= 256;  // float32 quads; fan beam always (its warps span more cells)
@@ -967,8 +1016,9 @@ int fp_storage_impl(const mct_geom* g, const mct_tables* t, const TIN* vol_in, c
         uint4* cy = cx + n;
         cell16_kernel<false><<<tg, tb, 0, s>>>(g->nx, g->nz, p.pitch, vol_in, cx, cy, nullptr);
         MCT_TRY(launched("cell16_kernel"));
-        fp_kernel<true, true, uint4, false><<<grid, block, 0, s>>>(p, t->angles, t->u, t->v, t->cz, t->pmat_a, t->pmat_xs, vol,
-                                                            nullptr, cx, cy, mask, sgm, nullptr);
+        auto go = by_samples ? fp_kernel<true, true, uint4, kSamples> : fp_kernel<true, true, uint4, kCells>;
+        go<<<grid, block, 0, s>>>(p, t->angles, t->u, t->v, t->cz, t->pmat_a, t->pmat_xs, vol, nullptr, cx, cy, mask, sgm,
+                                  nullptr);
     } else if (copies && dtype == MCT_F16) {
         uint4* cx = static_cast<uint4*>(workspace);
         uint4* cy = cx + n;
@@ -983,16 +1033,16 @@ int fp_storage_impl(const mct_geom* g, const mct_tables* t, const TIN* vol_in, c
         MCT_TRY(launched("vol_absmax_kernel"));
         cell16_kernel<true><<<tg, tb, 0, s>>>(g->nx, g->nz, p.pitch, vol_in, cx, cy, vmax);
         MCT_TRY(launched("cell16_kernel"));
-        fp_kernel<true, true, h16x8, false><<<grid, block, 0, s>>>(p, t->angles, t->u, t->v, t->cz, t->pmat_a, t->pmat_xs, vol,
-                                                            nullptr, reinterpret_cast<const h16x8*>(cx),
-                                                            reinterpret_cast<const h16x8*>(cy), mask, sgm, vmax);
+        auto go = by_samples ? fp_kernel<true, true, h16x8, kSamples> : fp_kernel<true, true, h16x8, kCells>;
+        go<<<grid, block, 0, s>>>(p, t->angles, t->u, t->v, t->cz, t->pmat_a, t->pmat_xs, vol, nullptr,
+                                  reinterpret_cast<const h16x8*>(cx), reinterpret_cast<const h16x8*>(cy), mask, sgm, vmax);
     } else if (copies) {
         Quad16* cx = static_cast<Quad16*>(workspace);
         Quad16* cy = cx + n;
         quad32_kernel<<<tg, tb, 0, s>>>(g->nx, g->nz, p.pitch, vol_in, reinterpret_cast<float4*>(cx),
                                         reinterpret_cast<float4*>(cy));
         MCT_TRY(launched("quad32_kernel"));
-        auto go = windows ? fp_kernel<true, true, Quad16, true> : fp_kernel<true, true, Quad16, false>;
+        auto go = windows ? fp_kernel<true, true, Quad16, kWindows> : fp_kernel<true, true, Quad16, kCells>;
         go<<<grid, block, 0, s>>>(p, t->angles, t->u, t->v, t->cz, t->pmat_a, t->pmat_xs, vol, nullptr, cx, cy, mask, sgm,
                                   nullptr);
     } else if constexpr (kIn32) {
@@ -1002,11 +1052,11 @@ int fp_storage_impl(const mct_geom* g, const mct_tables* t, const TIN* vol_in, c
             MCT_TRY(launched("transpose_xy_kernel"));
         }
         if (p.cone)
-            fp_kernel<true, false, float2, false><<<grid, block, 0, s>>>(p, t->angles, t->u, t->v, t->cz, t->pmat_a,
+            fp_kernel<true, false, float2, kCells><<<grid, block, 0, s>>>(p, t->angles, t->u, t->v, t->cz, t->pmat_a,
                                                                   t->pmat_xs, vol, vt, nullptr, nullptr, mask, sgm,
                                                                   nullptr);
         else
-            fp_kernel<false, false, float2, true><<<grid, block, 0, s>>>(p, t->angles, t->u, t->v, t->cz, t->pmat_a,
+            fp_kernel<false, false, float2, kWindows><<<grid, block, 0, s>>>(p, t->angles, t->u, t->v, t->cz, t->pmat_a,
                                                                    t->pmat_xs, vol, vt, nullptr, nullptr, mask, sgm,
                                                                    nullptr);
     }

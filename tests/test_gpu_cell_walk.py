@@ -24,7 +24,8 @@ TOL = {"f32": 5e-5, "f16": 2.0 ** -11, "bf16": 2.0 ** -8}
     (127, 6, 17, 5, 9, 0.2, "f32", True), (128, 6, 17, 5, 9, 0.2, "f32", True), (130, 6, 17, 5, 9, 0.2, "bf16", True),
     (255, 6, 17, 3, 5, 0.2, "f32", True), (256, 6, 17, 3, 5, 0.2, "f32", True), (257, 6, 33, 3, 5, 0.2, "f32", True),
     (40, 8, 35, 9, 255, 0.2, "f32", True), (40, 8, 35, 9, 257, 0.2, "f32", True), (40, 8, 35, 9, 257, 0.2, "bf16", True),
-    (40, 8, 35, 9, 30, 0.2, "f16", True), (40, 6, 35, 9, 30, 0.1, "f32", True),
+    (40, 8, 35, 9, 30, 0.2, "f16", True),
+    (40, 8, 35, 9, 30, 0.3, "bf16", True), (131, 6, 17, 5, 9, 0.5, "bf16", True), (40, 8, 35, 9, 30, 0.5, "f16", True), (40, 6, 35, 9, 30, 0.1, "f32", True),
     (34, 3, 37, 3, 30, 0.2, "f32", False), (130, 1, 41, 1, 9, 0.1, "f32", False), (260, 2, 41, 2, 5, 0.3, "f32", False)])
 def test_projection_by_cells_matches_the_sum_over_samples(n, nz, nu, nv, views, step, storage, cone, cuda):
     import torch
