@@ -18,6 +18,7 @@
 // voxel whose sum is NaN because the sinogram itself holds NaN is written as 0 too,
 // where the reference would return NaN).
 #include <cmath>
+#include <type_traits>
 
 #include "common.cuh"
 
@@ -60,19 +61,21 @@ struct BpParams {
     float o_x, o_y, o_z;     // P
 };
 
-// Per-view table of a chunk of nvc views starting at jc: {cos b', sin b', weight, 0}
-// with b' = b - img_rot and weight = delta-beta (run_mgfbp.py:1107-1111) x the
-// redundancy factor x the float16 unscale.
+// View j's entry of the tables: {cos b', sin b', weight, 0} with b' = b - img_rot and weight =
+// delta-beta (run_mgfbp.py:1107-1111) x the redundancy factor x the float16 unscale.
+__device__ __forceinline__ float4 view_entry(const BpParams& p, const float* __restrict__ angles, int j, float unscale) {
+    const int jg = p.view_begin + j;  // scan index (angles is the whole scan's table)
+    const int vt = p.views_total;
+    float s, c;
+    sincosf(angles[jg] - p.img_rot, &s, &c);
+    const float db = (jg == vt - 1) ? fabsf(angles[vt - 1] - angles[0]) / (vt - 1) : fabsf(angles[jg + 1] - angles[jg]);
+    return make_float4(c, s, db * p.div * unscale, 0.0f);
+}
+
+// Per-view table of a chunk of nvc views starting at jc.
 __device__ __forceinline__ void fill_view_table(const BpParams& p, const float* __restrict__ angles, float4* tab,
                                                 int jc, int nvc, int tid, int nthreads, float unscale) {
-    for (int q = tid; q < nvc; q += nthreads) {
-        const int jg = p.view_begin + jc + q;  // scan index (angles is the whole scan's table)
-        const int vt = p.views_total;
-        float s, c;
-        sincosf(angles[jg] - p.img_rot, &s, &c);
-        float db = (jg == vt - 1) ? fabsf(angles[vt - 1] - angles[0]) / (vt - 1) : fabsf(angles[jg + 1] - angles[jg]);
-        tab[q] = make_float4(c, s, db * p.div * unscale, 0.0f);
-    }
+    for (int q = tid; q < nvc; q += nthreads) tab[q] = view_entry(p, angles, jc + q, unscale);
 }
 
 // MODE 0: cone beam in any view mode; flat or curved detector, no projection matrix
@@ -91,6 +94,13 @@ __device__ __forceinline__ float reciprocal(float x) {
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
     return fmaf(r, fmaf(-x, r, 1.0f), r);
 }
+__device__ __forceinline__ float2 reciprocal2(float2 x) {
+    float2 r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r.x) : "f"(x.x));
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r.y) : "f"(x.y));
+    return __ffma2_rn(r, __ffma2_rn(make_float2(-x.x, -x.y), r, make_float2(1.0f, 1.0f)), r);
+}
+
 template <int MODE, bool CONE, typename QT, typename PT, bool CURVED = false>
 __global__ void __launch_bounds__(BP_TX* BP_TY, bp_min_blocks<MODE, QT, CURVED>())
 fdk_bp_kernel(BpParams p, const float* __restrict__ angles, const float* __restrict__ pmat,
@@ -360,107 +370,202 @@ __global__ void nan_to_zero_kernel(int64_t n, float* __restrict__ v) {
         if (v[i] != v[i]) v[i] = 0.0f;
 }
 
-// Axial fan beam (one detector row per slice, run_mgfbp.py:1183-1187).  A 2D image
-// has few voxels (256^2 at 720 views: 256 blocks of the kernel above, under two per
-// SM, each thread walking every view), so here the views of a column are split over
-// FB_G threads: block (32 x-voxels, FB_G view groups) for one image row and ZC slices
-// (1 for a single slice, else 8), thread g taking views g, g + FB_G, ...  The group
-// sums are added in a fixed order through shared memory (deterministic), and a column
-// is off the detector if any group saw it off.  A view that sees the column off the
-// detector does not stop the loop (its index is clamped and the column's result is
-// discarded), so independent views can overlap; 1/L is taken once per view.
-constexpr int FB_G = 8;
-template <int ZC, typename PT>
-__global__ void __launch_bounds__(32 * FB_G)
+// Axial fan beam (one detector row per slice, run_mgfbp.py:1183-1187).  With one slice
+// every voxel x view update pays for its own geometry, so instructions bound it.  A thread
+// takes one or two pairs of pixels above each other and every operation that allows it is one
+// packed f32x2 instruction for the pair: position, reciprocal step, detector index, floor,
+// weight.  The floor adds M = 1.5 * 2^23 rounded down, a column's smallest and largest index
+// are kept instead of a test per view (a view that sees it off the detector has its index
+// clamped and the column's result is discarded; a NaN index makes the sum NaN), and the
+// table holds each cosine and sine twice, as operand pairs.
+//
+// A 2D image has few pixels, so the views of a column are split over FB_G threads: block
+// (32 x-pixels, FB_G view groups) for 2 or 4 image rows and ZC slices (1 for a single slice,
+// else 8), thread g taking views g, g + FB_G, ...  The group sums are added in a fixed order
+// through shared memory (deterministic).
+//
+// 57.6 -> 19 instructions per update; now latency at half occupancy, issue 61 % and the packed
+// operations' half of the FMA pipe (63 %) share the limit.  ms, one pixel a thread with scalar
+// arithmetic / now: FBP 256^2 x 720 views 0.133 / 0.086; 1024^2 x 1440 views, bf16 2.65 / 1.21;
+// helical, 140 slices of 512^2 x 720 views 48.9 / 24.1; 512^2 x 8, 720 views 1.14 / 0.67.
+constexpr int FB_G = 8, FB_VCHUNK = 512;
+// Pairs of rows per thread and views unrolled.  One slice, 1 pair x 2 / 1 x 4 / 2 x 2 / 2 x 3 /
+// 4 x 1: helical FBP, 140 slices of 512^2 x 720 views 26.6 / 26.8 / 25.2 / 24.1 / 24.9 ms;
+// 1024^2 x 1440 views, bf16 1.33 / 1.22 / 1.24 / 1.21 / 1.17 ms.  8 slices and curved detectors
+// (two arc tangents a pair) take 1 x 2: 512^2 x 8, 720 views 0.668 ms against 0.747 with 2 x 3;
+// curved 512^2 0.419 against 0.474.  (Left to itself the compiler
+// takes 48 registers and spills: 256^2 0.092 ms against 0.086.)
+template <int ZC, bool CURVED>
+struct FanShape {
+    static constexpr int R = ZC == 1 && !CURVED ? 2 : 1, U = ZC == 1 && !CURVED ? 3 : 2;
+    static constexpr int B = ZC == 8 && !CURVED ? 3 : 2;  // blocks per SM, by the register budget
+};
+template <int ZC, bool CURVED, typename PT>
+__global__ void __launch_bounds__(32 * FB_G, FanShape<ZC, CURVED>::B)
 fdk_bp_fan_kernel(BpParams p, const float* __restrict__ angles, const void* __restrict__ packed,
                   float* __restrict__ vol, const uint32_t* __restrict__ f16_max) {
-    static_assert(ZC <= FB_G, "each of the first ZC view groups finishes one slice");
-    __shared__ float4 tab[BP_VCHUNK];
-    __shared__ float part[FB_G][ZC][32];
-    __shared__ int dead_g[FB_G][32];
+    constexpr int R = FanShape<ZC, CURVED>::R, NP = 2 * R;  // image rows of a block
+    __shared__ float4 tab[FB_VCHUNK];   // {cos b, cos b, sin b, sin b}
+    __shared__ float2 tabw[FB_VCHUNK];  // sid x weight, twice
+    __shared__ float part[FB_G][NP][ZC][32];
+    __shared__ int off_g[FB_G][NP][32];
     const int tx = threadIdx.x, g = threadIdx.y;
     const int ix = blockIdx.x * 32 + tx;
-    const int iy = blockIdx.y;
+    const int iy0 = blockIdx.y * NP;
     const int zb = blockIdx.z * ZC;
     const int tid = g * 32 + tx;
     const bool active = ix < p.nx;
     const int nq = p.nu - 1;
-    const float c0x = p.o_x + ix * p.px_x + iy * p.py_x;
-    const float c0y = p.o_y + ix * p.px_y + iy * p.py_y;
-    float acc[ZC];
+    // pixel centres (x, y) of the pairs; rows below the image are computed and not stored
+    float2 x2[R], y2[R], nx2[R], ny2[R];
 #pragma unroll
-    for (int k = 0; k < ZC; ++k) acc[k] = 0.0f;
-    bool dead = false;
+    for (int r = 0; r < R; ++r) {
+        float x[2], y[2];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int iy = iy0 + 2 * r + h;
+            x[h] = p.o_x + ix * p.px_x + iy * p.py_x;
+            y[h] = p.o_y + ix * p.px_y + iy * p.py_y;
+        }
+        x2[r] = make_float2(x[0], x[1]);
+        y2[r] = make_float2(y[0], y[1]);
+        nx2[r] = make_float2(-x[0], -x[1]);
+        ny2[r] = make_float2(-y[0], -y[1]);
+    }
+    float2 acc[R][ZC], lo[R], hi[R];  // sums; smallest and largest index of the pair's pixels
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        lo[r] = make_float2(3.0e38f, 3.0e38f);
+        hi[r] = make_float2(-3.0e38f, -3.0e38f);
+#pragma unroll
+        for (int k = 0; k < ZC; ++k) acc[r][k] = make_float2(0.0f, 0.0f);
+    }
     const float unscale = IsF16<PT>::value ? ldexpf(1.0f, -f16_scale_exp(*f16_max)) : 1.0f;
-    const float umax = (float)(p.nu - 1);
-    for (int jc = 0; jc < p.views; jc += BP_VCHUNK) {
-        const int nvc = min(BP_VCHUNK, p.views - jc);
-        __syncthreads();
-        fill_view_table(p, angles, tab, jc, nvc, tid, 32 * FB_G, unscale);
-        __syncthreads();
-        if (!active || dead) continue;
-        // views in flight per thread: a one-slice thread has one short dependent chain
-        // per view (helical FBP, 140 slices of 512^2 x 720 views, bit-identical: 51.45
-        // ms unrolled 2, 48.85 unrolled 4, 49.63 unrolled 8)
-        constexpr int kViewUnroll = ZC == 1 ? 4 : 2;
-#pragma unroll kViewUnroll
-        for (int q = g; q < nvc; q += FB_G) {
-            const int j = jc + q;
-            const float4 tb = tab[q];
-            const float cb = tb.x, sb = tb.y;
-            const float L = p.sid - c0x * cb - c0y * sb;
-            const float t = -c0x * sb + c0y * cb;
-            const float r = 1.0f / L;
-            const float mag = p.sdd * r;
-            const float u = p.curved ? p.sdd * atan2f(t, L) : mag * t;
-            const float ui = (u - p.u0) * p.inv_ustep;
-            dead |= !(ui >= 0.0f && ui + 1.0f <= umax);  // NaN counts as off-detector
-            const float uf = floorf(ui);
-            const float ru = ui - uf;
-            const int uc = min(max((int)uf, 0), p.nu - 2);
-            const float dw = p.curved ? 1.0f / (L * L + t * t) : r * r;
-            const float w = (p.sid * dw) * tb.z;
-            const PT* base = reinterpret_cast<const PT*>(packed) + ((int64_t)j * p.nv + zb) * nq + uc;
+    auto two = [](float a) { return make_float2(a, a); };
+    const float M = 12582912.0f;
+    const unsigned MB = 0x4B400000u;  // M's bits
+    const unsigned last = (unsigned)(p.nu - 2);
+    // A pixel at distance rho from the axis is seen at most asin(rho / sid) off the central
+    // ray: where that stays a column inside the detector for all the warp's pixels, no view
+    // needs the test or the clamp.
+    bool in = true;
 #pragma unroll
-            for (int k = 0; k < ZC; ++k) {
-                if (ZC == 1 || zb + k < p.nz) {
-                    const float2 pr = Pair<PT>::load(base + (int64_t)k * nq);
-                    acc[k] = fmaf(w, fmaf(ru, pr.y, pr.x), acc[k]);
+    for (int r = 0; r < R; ++r) {
+        const float rho2 = fmaxf(x2[r].x * x2[r].x + y2[r].x * y2[r].x, x2[r].y * x2[r].y + y2[r].y * y2[r].y);
+        const float c2 = p.sid * p.sid - rho2;
+        const float reach = CURVED ? p.sdd * asinf(sqrtf(rho2) / p.sid) : p.sdd * sqrtf(rho2 / c2);
+        const float i0 = (-reach - p.u0) * p.inv_ustep, i1 = (reach - p.u0) * p.inv_ustep;
+        in = in && c2 > 0.0f && fminf(i0, i1) >= 1.0f && fmaxf(i0, i1) <= (float)(p.nu - 3);
+    }
+    const bool inside = __all_sync(0xffffffffu, in);
+    if (inside) {  // no index was recorded: any valid one
+#pragma unroll
+        for (int r = 0; r < R; ++r) lo[r] = hi[r] = make_float2(0.0f, 0.0f);
+    }
+    for (int jc = 0; jc < p.views; jc += FB_VCHUNK) {
+        const int nvc = min(FB_VCHUNK, p.views - jc);
+        __syncthreads();
+        for (int q = tid; q < nvc; q += 32 * FB_G) {
+            const float4 e = view_entry(p, angles, jc + q, unscale);
+            tab[q] = make_float4(e.x, e.x, e.y, e.y);
+            tabw[q] = two(p.sid * e.z);
+        }
+        __syncthreads();
+        if (!active) continue;
+        auto views = [&](auto inside_tag) {
+            constexpr bool kInside = decltype(inside_tag)::value;
+            // with the column index taken from the bits of M + floor, M's bits are in the base
+            const char* base = static_cast<const char*>(packed) + ((int64_t)(jc + g) * p.nv + zb) * nq * (int64_t)sizeof(PT) -
+                               (kInside ? (int64_t)MB * (int64_t)sizeof(PT) : 0);
+            const int64_t step = (int64_t)FB_G * p.nv * nq * (int64_t)sizeof(PT);
+            constexpr int kViewUnroll = FanShape<ZC, CURVED>::U;
+#pragma unroll kViewUnroll
+            for (int q = g; q < nvc; q += FB_G, base += step) {
+                const float4 tb = tab[q];
+                const float2 cb = make_float2(tb.x, tb.y), sb = make_float2(tb.z, tb.w), sw = tabw[q];
+#pragma unroll
+                for (int r = 0; r < R; ++r) {
+                    const float2 L = __ffma2_rn(ny2[r], sb, __ffma2_rn(nx2[r], cb, two(p.sid)));
+                    const float2 t = __ffma2_rn(y2[r], cb, __fmul2_rn(nx2[r], sb));
+                    const float2 rL = reciprocal2(L);
+                    // u rounded on its own (an FMA with 0: a packed product would be fused with
+                    // the subtraction below, and columns at the detector's edge change sides)
+                    const float2 u = CURVED ? __ffma2_rn(two(p.sdd), make_float2(atan2f(t.x, L.x), atan2f(t.y, L.y)), two(0.0f))
+                                            : __ffma2_rn(__fmul2_rn(two(p.sdd), rL), t, two(0.0f));
+                    const float2 ui = __fmul2_rn(__fadd2_rn(u, two(-p.u0)), two(p.inv_ustep));
+                    const float2 m = __fadd2_rd(ui, two(M));
+                    const float2 uf = __fadd2_rn(m, two(-M));
+                    const float2 ru = __fadd2_rn(ui, make_float2(-uf.x, -uf.y));
+                    unsigned c0 = __float_as_uint(m.x), c1 = __float_as_uint(m.y);
+                    if (!kInside) {
+                        lo[r] = make_float2(fminf(lo[r].x, ui.x), fminf(lo[r].y, ui.y));
+                        hi[r] = make_float2(fmaxf(hi[r].x, ui.x), fmaxf(hi[r].y, ui.y));
+                        c0 = min(c0 - MB, last);
+                        c1 = min(c1 - MB, last);
+                    }
+                    const float2 dw = CURVED ? reciprocal2(__ffma2_rn(L, L, __fmul2_rn(t, t))) : __fmul2_rn(rL, rL);
+                    const float2 w = __fmul2_rn(dw, sw);
+                    const char* b0 = base + (uint64_t)c0 * (uint32_t)sizeof(PT);
+                    const char* b1 = base + (uint64_t)c1 * (uint32_t)sizeof(PT);
+#pragma unroll
+                    for (int k = 0; k < ZC; ++k) {
+                        if (ZC == 1 || zb + k < p.nz) {
+                            const float2 p0 = Pair<PT>::load(reinterpret_cast<const PT*>(b0) + (int64_t)k * nq);
+                            const float2 p1 = Pair<PT>::load(reinterpret_cast<const PT*>(b1) + (int64_t)k * nq);
+                            acc[r][k] = __ffma2_rn(w, make_float2(fmaf(ru.x, p0.y, p0.x), fmaf(ru.y, p1.y, p1.x)), acc[r][k]);
+                        }
+                    }
                 }
             }
+        };
+        if (inside) views(std::true_type{});
+        else views(std::false_type{});
+    }
+    const float umax = (float)(p.nu - 1);
+    auto off = [&](float a, float b) { return !(a >= 0.0f && b + 1.0f <= umax); };
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        off_g[g][2 * r][tx] = off(lo[r].x, hi[r].x);
+        off_g[g][2 * r + 1][tx] = off(lo[r].y, hi[r].y);
+#pragma unroll
+        for (int k = 0; k < ZC; ++k) {
+            part[g][2 * r][k][tx] = acc[r][k].x;
+            part[g][2 * r + 1][k][tx] = acc[r][k].y;
         }
     }
-#pragma unroll
-    for (int k = 0; k < ZC; ++k) part[g][k][tx] = acc[k];
-    dead_g[g][tx] = dead;
     __syncthreads();
-    const int k = g;  // the first ZC groups finish slice zb + g of their column
-    if (!active || k >= ZC || zb + k >= p.nz) return;
-    float sum = 0.0f;
-    int any_dead = 0;
-#pragma unroll
-    for (int h = 0; h < FB_G; ++h) {
-        sum += part[h][k][tx];
-        any_dead |= dead_g[h][tx];
+    if (!active) return;
+    // the groups share the block's rows and slices out among them
+    const int groups = min(FB_G, p.views);  // groups beyond the number of views saw none
+    for (int o = g; o < NP * ZC; o += FB_G) {
+        const int row = o / ZC, k = o % ZC;
+        if (iy0 + row >= p.nx || zb + k >= p.nz) continue;
+        float sum = 0.0f;
+        int any_off = 0;
+        for (int h = 0; h < groups; ++h) {
+            sum += part[h][row][k][tx];
+            any_off |= off_g[h][row][tx];
+        }
+        const bool off_detector = any_off || sum != sum;
+        float* out = vol + (int64_t)(zb + k) * p.nx * p.nx + (int64_t)(iy0 + row) * p.nx + ix;
+        if (p.accumulate)  // a voxel off the detector in any chunk stays NaN until mct_fdk_bp_finish
+            *out = off_detector ? __int_as_float(0x7fffffff) : *out + sum;
+        else
+            *out = off_detector ? 0.0f : sum;
     }
-    const bool off_detector = any_dead || sum != sum;
-    float* out = vol + (int64_t)(zb + k) * p.nx * p.nx + (int64_t)iy * p.nx + ix;
-    if (p.accumulate)  // a voxel off the detector in any chunk stays NaN until mct_fdk_bp_finish
-        *out = off_detector ? __int_as_float(0x7fffffff) : *out + sum;
-    else
-        *out = off_detector ? 0.0f : sum;
 }
 
-template <int ZC>
+template <int ZC, bool CURVED>
 void launch_bp_fan(const BpParams& p, const mct_geom* g, cudaStream_t s, const float* angles, const void* packed,
                    int dtype, float* vol, const uint32_t* f16_max) {
-    dim3 grid((g->nx + 31) / 32, g->nx, (g->nz + ZC - 1) / ZC), block(32, FB_G);
+    constexpr int rows = 2 * FanShape<ZC, CURVED>::R;
+    dim3 grid((g->nx + 31) / 32, (g->nx + rows - 1) / rows, (g->nz + ZC - 1) / ZC), block(32, FB_G);
     if (dtype == MCT_BF16)
-        fdk_bp_fan_kernel<ZC, uint32_t><<<grid, block, 0, s>>>(p, angles, packed, vol, nullptr);
+        fdk_bp_fan_kernel<ZC, CURVED, uint32_t><<<grid, block, 0, s>>>(p, angles, packed, vol, nullptr);
     else if (dtype == MCT_F16)
-        fdk_bp_fan_kernel<ZC, h16x2><<<grid, block, 0, s>>>(p, angles, packed, vol, f16_max);
+        fdk_bp_fan_kernel<ZC, CURVED, h16x2><<<grid, block, 0, s>>>(p, angles, packed, vol, f16_max);
     else
-        fdk_bp_fan_kernel<ZC, float2><<<grid, block, 0, s>>>(p, angles, packed, vol, nullptr);
+        fdk_bp_fan_kernel<ZC, CURVED, float2><<<grid, block, 0, s>>>(p, angles, packed, vol, nullptr);
 }
 
 template <int MODE, bool CONE, bool CURVED = false>
@@ -555,10 +660,12 @@ extern "C" int mct_fdk_bp(const mct_geom* g, const mct_tables* t, const void* pa
         launch_bp<2, true>(p, grid, block, s, t->angles, nullptr, packed, dtype, vol, fm);
     else if (cone && p.curved) launch_bp<0, true, true>(p, grid, block, s, t->angles, nullptr, packed, dtype, vol, fm);
     else if (cone) launch_bp<0, true>(p, grid, block, s, t->angles, nullptr, packed, dtype, vol, fm);
-    else if (g->view_mode == 1) {
+    else if (g->view_mode == 1 && g->nu <= (1 << 22)) {  // column indices exact in the float floor
         MCT_REQUIRE(g->nx <= 65535, "mct_fdk_bp: fan beam images are at most 65535 pixels wide");
-        if (g->nz == 1) launch_bp_fan<1>(p, g, s, t->angles, packed, dtype, vol, fm);
-        else launch_bp_fan<8>(p, g, s, t->angles, packed, dtype, vol, fm);
+        if (g->nz == 1 && p.curved) launch_bp_fan<1, true>(p, g, s, t->angles, packed, dtype, vol, fm);
+        else if (g->nz == 1) launch_bp_fan<1, false>(p, g, s, t->angles, packed, dtype, vol, fm);
+        else if (p.curved) launch_bp_fan<8, true>(p, g, s, t->angles, packed, dtype, vol, fm);
+        else launch_bp_fan<8, false>(p, g, s, t->angles, packed, dtype, vol, fm);
     }
     else launch_bp<1, false>(p, grid, block, s, t->angles, nullptr, packed, dtype, vol, fm);
     return launched("fdk_bp_kernel");
