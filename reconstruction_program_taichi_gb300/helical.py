@@ -10,8 +10,8 @@ slice's angular offset.  Here every slice is processed at once:
   2. weighting and the Toeplitz row filter run over the stack as one sinogram
      (slices x views rows; the fan weighting and the short-scan weights are the same
      for every slice, as the slice offsets cancel in them);
-  3. the filtered stack is packed once, slice-major, and each slice is
-     backprojected with its own angle table (base angles + the slice's offset).
+  3. the filtered stack is packed once and each slice is backprojected, from its row of
+     every view, with its own angle table (base angles + the slice's offset).
      Rotating the image by the offset, as the reference does, and adding the offset
      to the view angles are the same transform.
 """
@@ -160,26 +160,25 @@ class Mgfbp_helical(Mgfbp):  # noqa: N801 - reference name
                 filt = ops.filter_rows(pipe.dg, w, pipe.taps, out=pipe.filtered)
         if self.save_filtered_sinogram:  # the reference leaves the last slice's, as [views][1][cols]
             imwriteTiff(filt[:, nz - 1:nz, :].cpu().numpy(), self.output_dir + "/sgm_filtered_" + self.output_file)
-        # 3. slice-major pack (one 1-row fan sinogram of vc views per slice) and
-        #    per-slice backprojection with the slice's angles
-        per_slice = filt.permute(1, 0, 2).contiguous()  # [slices][views][cols]
+        # 3. one pack of the view-major stack (slices as detector rows) and per-slice
+        #    backprojection with the slice's angles: slice s is row s of every view, so its
+        #    operand starts s rows into the stack's (a slice-major copy of the stack first
+        #    cost 0.26 ms of 24 for 140 slices of 512^2)
         fan = self.fan_object(1)
         dg1 = fbp_geometry(fan, dev)
-        packed_obj = copy.copy(fan)
-        packed_obj.view_num = nz * vc
-        dgp = fbp_geometry(packed_obj, dev)
-        packed = ops.pack(dgp, per_slice.view(nz * vc, 1, nu), MCT_F32)
+        packed = ops.pack(pipe.dg, filt.contiguous(), MCT_F32)
         base = (fan.total_scan_angle / vc * np.arange(vc, dtype=np.float32)).astype(np.float32)
         adds = self.added_rotation()
         rots = (np.float32(self.img_rot) + adds.astype(np.float32)).astype(np.float32)
         angles = torch.from_numpy((base[None, :] + rots[:, None]).astype(np.float32)).to(dev)  # [slices][views]
         vol = torch.empty((nz, n, n), dtype=torch.float32, device=dev)
         g = dg1.geom
-        slice_bytes = vc * (nu - 1) * 8
+        row_bytes = (nu - 1) * 8
         for s in range(nz):
-            gs = g.copy(img_rot=float(rots[s]))
+            # nv = nz: the rows from one view's operand to the next
+            gs = g.copy(img_rot=float(rots[s]), nv=nz)
             ts = Tables(angles=angles.data_ptr() + s * vc * 4, u=dg1.tables.u, v=dg1.tables.v)
-            _lib.call("mct_fdk_bp", ctypes.byref(gs), ctypes.byref(ts), ctypes.c_void_p(packed.data_ptr() + s * slice_bytes),
+            _lib.call("mct_fdk_bp", ctypes.byref(gs), ctypes.byref(ts), ctypes.c_void_p(packed.data_ptr() + s * row_bytes),
                       MCT_F32, ctypes.c_void_p(vol.data_ptr() + s * n * n * 4), ops._stream())
         return vol
 
