@@ -172,6 +172,17 @@ struct Quad<h16x4> {
         hi = h16x2_to_float2(q.y);
     }
 };
+// Views between checks whether a column has left the detector (8 and 256 within 0.5 %).
+constexpr int kViewRun = 32;
+
+// 1 / x from the hardware approximation (1 ulp) and one Newton-Raphson step r + r (1 - x r),
+// without the division's branch for special values: 0 and infinities give NaN, which the
+// detector test rejects like the infinite or zero magnification of the division.
+__device__ __forceinline__ float reciprocal(float x) {
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return fmaf(r, fmaf(-x, r, 1.0f), r);
+}
 template <typename PT>
 struct Pair;
 template <>

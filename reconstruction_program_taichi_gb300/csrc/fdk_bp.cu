@@ -83,17 +83,6 @@ __device__ __forceinline__ void fill_view_table(const BpParams& p, const float* 
 //         more than 2^22 rows
 // MODE 1: fan beam in the coronal or sagittal view mode (per-voxel u)
 // MODE 3: projection matrix geometry in any view mode (per-column matrix rows)
-// Views between checks whether a column has left the detector (8 and 256 within 0.5 %).
-constexpr int kViewRun = 32;
-
-// 1 / x from the hardware approximation (1 ulp) and one Newton-Raphson step r + r (1 - x r),
-// without the division's branch for special values: 0 and infinities give NaN, which the
-// detector test rejects like the infinite or zero magnification of the division.
-__device__ __forceinline__ float reciprocal(float x) {
-    float r;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
-    return fmaf(r, fmaf(-x, r, 1.0f), r);
-}
 __device__ __forceinline__ float2 reciprocal2(float2 x) {
     float2 r;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r.x) : "f"(x.x));

@@ -6,6 +6,7 @@
 // GenerateWR :234-243, TVPenaltyVal :245-254, Dt_W_D :267-286, and the NumPy vector
 // algebra of TikhonovSol :188-232.
 #include <cmath>
+#include <type_traits>
 
 #include "common.cuh"
 
@@ -185,16 +186,18 @@ struct CgEpi {
     float s1, s2;
     double* partials;  // one per block, in blockIdx order
 };
-// Resident blocks per SM that the register allocation targets: 3 (80 registers) for
+// Resident blocks per SM that the register allocation targets: 2 (128 registers) for the
+// pipelined loop, which holds a view's gathers and the next one's geometry (16-bit operands
+// with 3 blocks 0.2 % to 1 % slower, 16-byte ones spill).  The other loop: 3 (80 registers) for
 // 8-byte operands and for 16-byte ones without the CG epilogue (with slices in pairs,
 // 512x512x64 / 360 views float32 5.67 ms with 2 blocks of 128 registers, 5.44 ms with
 // 3 blocks, bit-identical), 2 for 16-byte operands with the epilogue.
-template <typename QT, bool EPI>
+template <typename QT, bool EPI, bool PIPE>
 constexpr int ua_min_blocks() {
-    return sizeof(QT) == 8 || !EPI ? 3 : 2;
+    return !PIPE && (sizeof(QT) == 8 || !EPI) ? 3 : 2;
 }
-template <bool CONE, typename QT, typename PT, typename OT = float, bool EPI = false>
-__global__ void __launch_bounds__(UB_TX* UB_TY, ua_min_blocks<QT, EPI>())
+template <bool CONE, typename QT, typename PT, typename OT = float, bool EPI = false, bool PIPE = false>
+__global__ void __launch_bounds__(UB_TX* UB_TY, ua_min_blocks<QT, EPI, PIPE>())
 bp_unmatched_axial_kernel(UbParams p, const float* __restrict__ angles, const float* __restrict__ czv, float cz_const,
                           const void* __restrict__ packed, OT* __restrict__ vol,
                           const uint32_t* __restrict__ f16_max, CgEpi epi = CgEpi{}) {
@@ -231,7 +234,93 @@ bp_unmatched_axial_kernel(UbParams p, const float* __restrict__ angles, const fl
         }
         __syncthreads();
         if (!active || trunc) continue;
-        for (int q = 0; q < nvc; ++q) {
+        if constexpr (PIPE) {
+            // As in fdk_bp_kernel: the next view's geometry is computed between the issue of
+            // this view's gathers and their use, the floor is taken on the FMA pipe, and a
+            // truncated column goes on with a clamped index to the end of its run of views.
+            // One application, ms: 256x256x64 / 180 views float32 0.741 -> 0.648, bf16 0.747 ->
+            // 0.694; 512x512x64 / 360 views float32 5.43 -> 4.90, bf16 5.59 -> 5.31.
+            struct View {
+                const char* base;
+                float ru, wpx, r2, zA, vA, vB;
+            };
+            const float umax = (float)(p.nu - 1);
+            bool off = false;
+            auto geometry = [&](int q) {
+                const float4 tb = tab[q];
+                const float cb = tb.x, sb = tb.y;
+                const float L = p.sid - x * cb - y * sb;
+                const float qx = x - tb.w, qy = y - tab_s[q];
+                const float aqx = fabsf(qx), aqy = fabsf(qy);
+                const float mq = aqx > aqy ? aqx : aqy;
+                const float rr = reciprocal(L * mq);  // for sdd / L and px / max(|qx|, |qy|)
+                const float mag = p.sdd * mq * rr;
+                const float t = -x * sb + y * cb;
+                const float u = __fmul_rn(mag, t);  // rounded on its own, see fdk_bp_kernel
+                const float ui = (u - p.u0) * p.inv_ustep;
+                off |= !(ui >= 0.0f && ui + 1.0f <= umax);
+                const float uf = floorf(ui);
+                const int uc = min(max((int)uf, 0), p.nu - 2);
+                View v;
+                v.ru = ui - uf;
+                v.r2 = qx * qx + qy * qy;
+                v.wpx = p.px * L * rr;
+                v.zA = bz + tb.z;
+                v.vA = (mag * v.zA - p.v0) * p.kv;
+                v.vB = (mag * p.zz) * p.kv;
+                v.base = static_cast<const char*>(packed) + ((int64_t)(jc + q) * p.nv * nq + uc) * (int64_t)sizeof(QT);
+                return v;
+            };
+            const unsigned top = (unsigned)(p.nv - 2);  // rows [0, nv-2] hold a bilinear cell (nv >= 2)
+            const uint32_t stride = (uint32_t)(nq * sizeof(QT));
+            const float2 zz2 = make_float2(p.zz, p.zz);
+            View cur = geometry(0);
+            for (int q0 = 0; q0 < nvc && !off; q0 += kViewRun) {
+                const int q1 = min(q0 + kViewRun, nvc);
+                for (int q = q0; q < q1; ++q) {
+                    const float2 ru2 = make_float2(cur.ru, cur.ru);
+                    const float2 vA2 = make_float2(cur.vA, cur.vA), vB2 = make_float2(cur.vB, cur.vB);
+                    const float M = 12582912.0f;
+                    const unsigned MB = 0x4B400000u;  // M's bits
+                    float2 lo[UA_ZC], hi[UA_ZC];
+                    float rv[UA_ZC];
+                    unsigned row[UA_ZC];
+                    auto load = [&](int k, unsigned r) {
+                        row[k] = r;
+                        Quad<QT>::load(reinterpret_cast<const QT*>(cur.base + (uint64_t)min(r, top) * stride), lo[k], hi[k]);
+                    };
+#pragma unroll
+                    for (int k = 0; k < UA_ZC; k += 2) {
+                        const float2 vi = __ffma2_rn(make_float2((float)k, (float)(k + 1)), vB2, vA2);
+                        const float2 m = __fadd2_rd(vi, make_float2(M, M));
+                        const float2 fl = __fadd2_rn(m, make_float2(-M, -M));
+                        const float2 f = __fadd2_rn(vi, make_float2(-fl.x, -fl.y));
+                        rv[k] = f.x;
+                        rv[k + 1] = f.y;
+                        load(k, __float_as_uint(m.x) - MB);  // rows off the detector: above top
+                        load(k + 1, __float_as_uint(m.y) - MB);
+                    }
+                    const View next = geometry(min(q + 1, nvc - 1));
+                    const float2 zA2 = make_float2(cur.zA, cur.zA), r22 = make_float2(cur.r2, cur.r2);
+                    const float2 wpx2 = make_float2(cur.wpx, cur.wpx);
+#pragma unroll
+                    for (int k = 0; k < UA_ZC; k += 2) {
+                        const float2 kk = make_float2((float)k, (float)(k + 1));
+                        const float2 s0 = __ffma2_rn(ru2, hi[k], lo[k]), s1 = __ffma2_rn(ru2, hi[k + 1], lo[k + 1]);
+                        const float2 z = __ffma2_rn(kk, zz2, zA2);
+                        const float2 d2 = __ffma2_rn(z, z, r22);
+                        float2 w = __fmul2_rn(__fmul2_rn(d2, make_float2(rsqrtf(d2.x), rsqrtf(d2.y))), wpx2);
+                        // a row outside [0, nv-2] contributes nothing
+                        if (row[k] > top) w.x = 0.0f;
+                        if (row[k + 1] > top) w.y = 0.0f;
+                        acc[k] = fmaf(fmaf(rv[k], s0.y, s0.x), w.x, acc[k]);
+                        acc[k + 1] = fmaf(fmaf(rv[k + 1], s1.y, s1.x), w.y, acc[k + 1]);
+                    }
+                    cur = next;
+                }
+            }
+            if (off) trunc = true;
+        } else for (int q = 0; q < nvc; ++q) {
             const int j = jc + q;
             const float4 tb = tab[q];
             const float cb = tb.x, sb = tb.y;
@@ -542,18 +631,45 @@ inline int ew_grid(int64_t n) {
 
 using namespace mct;
 
-template <typename QT, typename PT>
-void launch_unmatched_packed(const mct_geom* g, const UbParams& p, const mct_tables* t, const void* packed,
-                                    float* vol, const uint32_t* f16_max, cudaStream_t s) {
+// The axial cone-beam kernel with output OT, with or without the CG epilogue.
+template <typename OT, bool EPI, bool PIPE, typename QT, typename PT>
+void launch_axial_q(const mct_geom* g, const UbParams& p, const mct_tables* t, const void* packed, OT* out,
+                    const uint32_t* f16_max, const CgEpi& e, cudaStream_t s) {
     dim3 block(UB_TX, UB_TY);
-    if (g->view_mode == 1) {
+    dim3 grid((g->nx + UB_TX - 1) / UB_TX, (g->nx + UB_TY - 1) / UB_TY, (g->nz + UA_ZC - 1) / UA_ZC);
+    bp_unmatched_axial_kernel<true, QT, PT, OT, EPI, PIPE><<<grid, block, 0, s>>>(p, t->angles, t->cz, g->cz, packed, out,
+                                                                                  f16_max, e);
+}
+template <typename OT, bool EPI>
+void launch_axial(const mct_geom* g, const UbParams& p, const mct_tables* t, const void* packed, int dtype, OT* out,
+                  const CgEpi& e, cudaStream_t s) {
+    // the pipelined loop: flat detectors whose row indices the float floor holds exactly
+    const bool pipe = !p.curved && p.nv <= (1 << 22);
+    if (dtype == MCT_F32) {
+        if (pipe) launch_axial_q<OT, EPI, true, float4, float2>(g, p, t, packed, out, nullptr, e, s);
+        else launch_axial_q<OT, EPI, false, float4, float2>(g, p, t, packed, out, nullptr, e, s);
+    } else if (dtype == MCT_BF16) {
+        if (pipe) launch_axial_q<OT, EPI, true, uint2, uint32_t>(g, p, t, packed, out, nullptr, e, s);
+        else launch_axial_q<OT, EPI, false, uint2, uint32_t>(g, p, t, packed, out, nullptr, e, s);
+    } else {
+        const uint32_t* fm = f16_trailer(g, packed);
+        if (pipe) launch_axial_q<OT, EPI, true, h16x4, h16x2>(g, p, t, packed, out, fm, e, s);
+        else launch_axial_q<OT, EPI, false, h16x4, h16x2>(g, p, t, packed, out, fm, e, s);
+    }
+}
+
+// Every view mode and beam with float32 output: the axial cone-beam kernel, the axial
+// fan-beam one, or the general one.
+template <typename QT, typename PT>
+void launch_unmatched_packed(const mct_geom* g, const UbParams& p, const mct_tables* t, const void* packed, int dtype,
+                             float* vol, const uint32_t* f16_max, cudaStream_t s) {
+    dim3 block(UB_TX, UB_TY);
+    if (g->view_mode == 1 && p.cone) {
+        launch_axial<float, false>(g, p, t, packed, dtype, vol, CgEpi{}, s);
+    } else if (g->view_mode == 1) {
         dim3 grid((g->nx + UB_TX - 1) / UB_TX, (g->nx + UB_TY - 1) / UB_TY, (g->nz + UA_ZC - 1) / UA_ZC);
-        if (p.cone)
-            bp_unmatched_axial_kernel<true, QT, PT><<<grid, block, 0, s>>>(p, t->angles, t->cz, g->cz, packed, vol,
-                                                                           f16_max);
-        else
-            bp_unmatched_axial_kernel<false, QT, PT><<<grid, block, 0, s>>>(p, t->angles, t->cz, g->cz, packed, vol,
-                                                                            f16_max);
+        bp_unmatched_axial_kernel<false, QT, PT><<<grid, block, 0, s>>>(p, t->angles, t->cz, g->cz, packed, vol,
+                                                                        f16_max);
     } else {
         dim3 grid((g->nx + UB_TX - 1) / UB_TX, (g->nx + UB_TY - 1) / UB_TY, (g->nz + UB_ZC - 1) / UB_ZC);
         bp_unmatched_kernel<1, QT, PT><<<grid, block, 0, s>>>(p, t->angles, t->cz, g->cz, nullptr, packed, vol,
@@ -589,19 +705,8 @@ int mct_bp_ref_unmatched_packed_out(const mct_geom* g, const mct_tables* t, cons
     MCT_REQUIRE(g->view_mode == 1 && p.cone,
                 "mct_bp_ref_unmatched_packed_out: bf16 output needs the axial view mode and cone beam");
     MCT_REQUIRE((int64_t)g->nv * (g->nu - 1) < ((int64_t)1 << 31), "mct_bp_ref_unmatched_packed_out: detector too large");
-    cudaStream_t s = as_stream(stream);
-    dim3 block(UB_TX, UB_TY);
-    dim3 grid((g->nx + UB_TX - 1) / UB_TX, (g->nx + UB_TY - 1) / UB_TY, (g->nz + UA_ZC - 1) / UA_ZC);
-    __nv_bfloat16* out = static_cast<__nv_bfloat16*>(vol);
-    if (dtype == MCT_F32)
-        bp_unmatched_axial_kernel<true, float4, float2, __nv_bfloat16><<<grid, block, 0, s>>>(
-            p, t->angles, t->cz, g->cz, packed, out, nullptr);
-    else if (dtype == MCT_BF16)
-        bp_unmatched_axial_kernel<true, uint2, uint32_t, __nv_bfloat16><<<grid, block, 0, s>>>(
-            p, t->angles, t->cz, g->cz, packed, out, nullptr);
-    else
-        bp_unmatched_axial_kernel<true, h16x4, h16x2, __nv_bfloat16><<<grid, block, 0, s>>>(
-            p, t->angles, t->cz, g->cz, packed, out, f16_trailer(g, packed));
+    launch_axial<__nv_bfloat16, false>(g, p, t, packed, dtype, static_cast<__nv_bfloat16*>(vol), CgEpi{},
+                                       as_stream(stream));
     return launched("bp_unmatched_kernel");
 }
 
@@ -628,27 +733,11 @@ int mct_bp_ref_unmatched_packed_cg(const mct_geom* g, const mct_tables* t, const
                 "mct_bp_ref_unmatched_packed_cg: q aliases an input");
     MCT_REQUIRE((int64_t)g->nv * (g->nu - 1) < ((int64_t)1 << 31), "mct_bp_ref_unmatched_packed_cg: detector too large");
     cudaStream_t s = as_stream(stream);
-    dim3 block(UB_TX, UB_TY);
-    dim3 grid((g->nx + UB_TX - 1) / UB_TX, (g->nx + UB_TY - 1) / UB_TY, (g->nz + UA_ZC - 1) / UA_ZC);
     const CgEpi e{d, wr1, wr2, s1, s2, partials};
-    const uint32_t* fm = dtype == MCT_F16 ? f16_trailer(g, packed) : nullptr;
-    auto go = [&](auto out_tag) {
-        using OT = decltype(out_tag);
-        OT* out = static_cast<OT*>(q);
-        if (dtype == MCT_F32)
-            bp_unmatched_axial_kernel<true, float4, float2, OT, true><<<grid, block, 0, s>>>(p, t->angles, t->cz, g->cz,
-                                                                                           packed, out, nullptr, e);
-        else if (dtype == MCT_BF16)
-            bp_unmatched_axial_kernel<true, uint2, uint32_t, OT, true><<<grid, block, 0, s>>>(
-                p, t->angles, t->cz, g->cz, packed, out, nullptr, e);
-        else
-            bp_unmatched_axial_kernel<true, h16x4, h16x2, OT, true><<<grid, block, 0, s>>>(p, t->angles, t->cz, g->cz,
-                                                                                         packed, out, fm, e);
-    };
-    if (vec_dtype == MCT_F32) go(float{});
-    else go(__nv_bfloat16{});
+    if (vec_dtype == MCT_F32) launch_axial<float, true>(g, p, t, packed, dtype, static_cast<float*>(q), e, s);
+    else launch_axial<__nv_bfloat16, true>(g, p, t, packed, dtype, static_cast<__nv_bfloat16*>(q), e, s);
     MCT_TRY(launched("bp_unmatched_kernel"));
-    finish_sum_kernel<<<1, RED_THREADS, 0, s>>>(partials, (int)(grid.x * grid.y * grid.z), dq);
+    finish_sum_kernel<<<1, RED_THREADS, 0, s>>>(partials, (int)(mct_bp_cg_partials_size(g) / sizeof(double)), dq);
     return launched("finish_sum_kernel");
 }
 
@@ -662,11 +751,11 @@ int mct_bp_ref_unmatched_packed(const mct_geom* g, const mct_tables* t, const vo
     MCT_REQUIRE((int64_t)g->nv * (g->nu - 1) < ((int64_t)1 << 31), "mct_bp_ref_unmatched_packed: detector too large");
     cudaStream_t s = as_stream(stream);
     if (dtype == MCT_F32)
-        launch_unmatched_packed<float4, float2>(g, p, t, packed, vol, nullptr, s);
+        launch_unmatched_packed<float4, float2>(g, p, t, packed, dtype, vol, nullptr, s);
     else if (dtype == MCT_BF16)
-        launch_unmatched_packed<uint2, uint32_t>(g, p, t, packed, vol, nullptr, s);
+        launch_unmatched_packed<uint2, uint32_t>(g, p, t, packed, dtype, vol, nullptr, s);
     else
-        launch_unmatched_packed<h16x4, h16x2>(g, p, t, packed, vol, f16_trailer(g, packed), s);
+        launch_unmatched_packed<h16x4, h16x2>(g, p, t, packed, dtype, vol, f16_trailer(g, packed), s);
     return launched("bp_unmatched_kernel");
 }
 

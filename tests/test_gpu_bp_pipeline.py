@@ -7,6 +7,7 @@ import pytest
 
 from conftest import rel_l2
 from oracle import fbp_ops as F
+from oracle import ir_ops as I
 from test_gpu_parity import _cone_obj
 
 pytestmark = pytest.mark.gpu
@@ -62,3 +63,27 @@ def test_detector_of_more_than_2_22_rows_gives_the_same_volume(cuda):
     got = ops.fdk_bp(dg, ops.pack(dg, tall))
     assert float((small != 0).float().mean()) > 0.5
     assert torch.equal(got, small)
+
+
+@pytest.mark.parametrize("views,storage", [(2, "f32"), (31, "f32"), (32, "f32"), (33, "f32"), (65, "f32"), (33, "bf16"),
+                                           (33, "f16")])
+def test_solver_backprojection_matches_the_oracle_off_the_detector(views, storage, cuda):
+    """The solver's backprojector in the same loop: columns that leave the detector are zero,
+    rows that leave it are skipped."""
+    import torch
+    from reconstruction_program_taichi_gb300 import geometry, ops
+    o = _cone_obj(n=37, nz=18, nu=34, nv=12, views=views)
+    dg = geometry.ir_geometry(o)
+    rng = np.random.default_rng(views)
+    sgm = rng.normal(0, 1, dg.sgm_shape).astype(np.float32)
+    dtype = {"f32": ops.MCT_F32, "bf16": ops.MCT_BF16, "f16": ops.MCT_F16}[storage]
+    got = ops.bp_unmatched_packed(dg, ops.pack_sinogram(dg, torch.from_numpy(sgm).cuda(), dtype), dtype).cpu().numpy()
+    ref = I.bp_unmatched(sgm, dg.host["angles"], dg.host["u"], dg.host["v"], o.array_img_center_z, nx=o.img_dim,
+                         nz=o.img_dim_z, px=o.img_pix_size, pz=o.img_voxel_height, cx=o.img_center_x, cy=o.img_center_y,
+                         sid=o.source_isocenter_dis, sdd=o.source_det_dis, dv=o.det_elem_height, img_rot=o.img_rot,
+                         cone_beam=True)
+    assert 0.05 < np.mean(ref == 0) < 0.95
+    # voxels within float32 rounding of the detector's edge may fall on either side
+    assert np.mean((got == 0) != (ref == 0)) < 1e-3
+    both = (got != 0) & (ref != 0)
+    assert rel_l2(got[both], ref[both]) < 5 * TOL[storage]  # a row at the edge in or out: one view of `views`
