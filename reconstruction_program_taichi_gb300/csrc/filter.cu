@@ -24,7 +24,8 @@ __global__ void weight_kernel(WeightParams p, const float* __restrict__ in, cons
         const float beta = p.short_scan ? fabsf(angles[p.view_begin + j] - angles[0]) : 0.0f;
         for (int c = threadIdx.x; c < p.nu; c += blockDim.x) {
             const float u = p.u0 + c * p.u_step;
-            dst[c] = weight_value(p, src[c], bh, u, weight_cos(p, u), weight_den(p, u, v), beta);
+            const float gamma = p.short_scan ? parker_gamma(p, u) : 0.0f;
+            dst[c] = weight_value(p, src[c], bh, gamma, weight_cos(p, u), weight_den(p, u, v), beta);
         }
     }
 }
@@ -45,11 +46,11 @@ weight4_kernel(WeightParams p, const float* __restrict__ in, const float* __rest
     const float v = p.v0 + r * p.v_step;
     const int nu4 = p.nu >> 2;
     for (int c4 = threadIdx.x; c4 < nu4; c4 += blockDim.x) {
-        float uu[4], cs[4], den[4];
+        float ga[4], cs[4], den[4];
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
             const float u = p.u0 + (4 * c4 + e) * p.u_step;
-            uu[e] = u;
+            ga[e] = p.short_scan ? parker_gamma(p, u) : 0.0f;
             cs[e] = weight_cos(p, u);
             den[e] = weight_den(p, u, v);
         }
@@ -61,7 +62,7 @@ weight4_kernel(WeightParams p, const float* __restrict__ in, const float* __rest
                 const float beta = p.short_scan ? fabsf(angles[p.view_begin + j] - angles[0]) : 0.0f;
                 float o[4] = {x.x, x.y, x.z, x.w};
 #pragma unroll
-                for (int e = 0; e < 4; ++e) o[e] = weight_value(p, o[e], bh, uu[e], cs[e], den[e], beta);
+                for (int e = 0; e < 4; ++e) o[e] = weight_value(p, o[e], bh, ga[e], cs[e], den[e], beta);
                 *reinterpret_cast<float4*>(out + ((int64_t)r * p.views + j) * p.nu + 4 * c4) =
                     make_float4(o[0], o[1], o[2], o[3]);
             }

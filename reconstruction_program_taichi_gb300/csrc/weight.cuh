@@ -16,11 +16,15 @@ struct WeightParams {
     float num_rounds, remain;  // short-scan constants
 };
 
+// Fan angle of a column in the direction of rotation (short scans).
+__device__ __forceinline__ float parker_gamma(const WeightParams& p, float u) {
+    const float rot_dir = fabsf(p.scan) / p.scan;
+    return p.curved ? ((-1.0f) * u / p.sdd) * rot_dir : atan2f(-u, p.sdd) * rot_dir;
+}
+
 // Parker / over-scan weight of one (view, column), run_mgfbp.py:971-1011.
-__device__ __forceinline__ float parker(const WeightParams& p, float beta, float u) {
+__device__ __forceinline__ float parker(const WeightParams& p, float beta, float gamma) {
     const float PI = (float)kPI;
-    float rot_dir = fabsf(p.scan) / p.scan;
-    float gamma = p.curved ? ((-1.0f) * u / p.sdd) * rot_dir : atan2f(-u, p.sdd) * rot_dir;
     float gmax = p.remain - PI;
     float nr = p.num_rounds, ra = p.remain;
     float w = 0.0f;
@@ -56,8 +60,9 @@ __device__ __forceinline__ float weight_cos(const WeightParams& p, float u) {
 }
 
 // One weighted element: beam-hardening polynomial, cosine weight, Parker weight
-// (beta = |angle - angle_0| of the element's view, used with short scans only).
-__device__ __forceinline__ float weight_value(const WeightParams& p, float val, const float* __restrict__ bh, float u,
+// (beta = |angle - angle_0| of the element's view and gamma, the column's fan angle, are used
+// with short scans only).
+__device__ __forceinline__ float weight_value(const WeightParams& p, float val, const float* __restrict__ bh, float gamma,
                                               float cs, float den, float beta) {
     if (p.n_bh > 0) {
         float acc = 0.0f, pw = val;
@@ -70,7 +75,7 @@ __device__ __forceinline__ float weight_value(const WeightParams& p, float val, 
     const float sdd = p.sdd;
     if (p.curved) val = val * sdd * cs * sdd / den;
     else val = (val * sdd * sdd) / den;
-    if (p.short_scan) val *= parker(p, beta, u);
+    if (p.short_scan) val *= parker(p, beta, gamma);
     return val;
 }
 
