@@ -617,18 +617,207 @@ __device__ __forceinline__ void red_add_v4(float* q, float a, float b, float c, 
                  : "memory");
 }
 
+__device__ __forceinline__ void red_add_v2(float* q, float a, float b) {
+    asm volatile("red.global.add.v2.f32 [%0], {%1, %2};" ::"l"(q), "f"(a), "f"(b) : "memory");
+}
+
+// One ray of the adjoint.  Corners are kept by its direction, 0 behind and 1 ahead on each
+// axis; fx, fy, fz tell where behind is the higher index.  They are template arguments: as
+// run-time values they cost 16 selects per cell.
+template <bool CONE, bool CELLS, bool fx, bool fy, bool fz>
+__device__ __forceinline__ void adjoint_ray(const FpParams& p, const Ray& r, int iv, float yv, float* __restrict__ out) {
+    const int nx = p.nx;
+    const int plane = nx * nx;
+    const int stepx = fx ? -1 : 1, stepy = fy ? -nx : nx, stepz = fz ? -plane : plane;
+    const unsigned xf = fx ? 1u : 0u;                                            // XF of the face behind
+    const unsigned yf = (unsigned)p.nz * (unsigned)plane + (fy ? (unsigned)nx : 0u);  // YF of the face behind
+    int cell = -1;
+    float2 s00 = make_float2(0.f, 0.f), s01 = s00, s10 = s00, s11 = s00;  // s<x><z> = {y behind, y ahead}
+    auto order = [](bool flip, float a, float b) { return flip ? make_float2(b, a) : make_float2(a, b); };
+    auto face = [&](unsigned element, float2 behind, float2 ahead) {  // pairs at z behind and ahead
+        float* q = out + (size_t)element * 4;
+        const float2 lo = fz ? ahead : behind, hi = fz ? behind : ahead;
+        red_add_v4(q, lo.x, lo.y, hi.x, hi.y);
+    };
+    auto flush = [&]() {  // all corners
+        if (cell < 0) return;
+        if constexpr (CONE && CELLS) {
+            face((unsigned)cell + xf, order(fy, s00.x, s00.y), order(fy, s01.x, s01.y));
+            face((unsigned)cell + 1u - xf, order(fy, s10.x, s10.y), order(fy, s11.x, s11.y));
+        } else if constexpr (CELLS) {
+            const float2 lo = order(fx, s00.x, s10.x), hi = order(fx, s00.y, s10.y);  // y behind, ahead
+            red_add_v4(out + (size_t)cell * 4, fy ? hi.x : lo.x, fy ? hi.y : lo.y, fy ? lo.x : hi.x, fy ? lo.y : hi.y);
+        } else {
+            float* b = out + cell;
+            const int x0 = fx ? 1 : 0, y0 = fy ? nx : 0, y1 = nx - y0;
+            float* q = b + (CONE && fz ? plane : 0);
+            atomicAdd(q + x0 + y0, s00.x);
+            atomicAdd(q + 1 - x0 + y0, s10.x);
+            atomicAdd(q + x0 + y1, s00.y);
+            atomicAdd(q + 1 - x0 + y1, s10.y);
+            if (CONE) {
+                q = b + (fz ? 0 : plane);
+                atomicAdd(q + x0 + y0, s01.x);
+                atomicAdd(q + 1 - x0 + y0, s11.x);
+                atomicAdd(q + x0 + y1, s01.y);
+                atomicAdd(q + 1 - x0 + y1, s11.y);
+            }
+        }
+        s00 = s01 = s10 = s11 = make_float2(0.f, 0.f);
+    };
+    auto enter = [&](int off) {
+        if (off == cell) return;
+        const int d = off - cell;
+        if (CONE && CELLS && cell >= 0 && (d == stepx || d == stepy)) {
+            const bool x = d == stepx;
+            const float b0 = x ? s00.y : s10.x, b1 = x ? s01.y : s11.x;  // the face's other corner, z behind and ahead
+            const bool f = x ? fy : fx;
+            face((unsigned)cell + (x ? xf : yf), order(f, s00.x, b0), order(f, s01.x, b1));
+            s00 = make_float2(x ? s10.x : s00.y, x ? s10.y : 0.0f);
+            s10 = make_float2(x ? 0.0f : s10.y, 0.0f);
+            s01 = make_float2(x ? s11.x : s01.y, x ? s11.y : 0.0f);
+            s11 = make_float2(x ? 0.0f : s11.y, 0.0f);
+        } else if (CONE && CELLS && cell >= 0 && d == stepz) {
+            float* q = out + ((size_t)((unsigned)cell + xf) * 4 + (fz ? 2 : 0));
+            const float2 a = order(fy, s00.x, s00.y), b = order(fy, s10.x, s10.y);
+            red_add_v2(q, a.x, a.y);
+            red_add_v2(out + ((size_t)((unsigned)cell + 1u - xf) * 4 + (fz ? 2 : 0)), b.x, b.y);
+            s00 = s01;
+            s10 = s11;
+            s01 = s11 = make_float2(0.f, 0.f);
+        } else {
+            flush();
+        }
+        cell = off;
+    };
+    const float dx = fabsf(r.dfx), dy = fabsf(r.dfy), dzz = fabsf(r.dfz);
+    const float kxy = dx * dy * (1.0f / 12.0f), kxz = dx * dzz * (1.0f / 12.0f), kyz = dy * dzz * (1.0f / 12.0f);
+    // n samples with midpoint fractions (x, y, z) towards the corners ahead
+    auto add = [&](float n, float x, float y, float z) {
+        const float g = n * yv, h = fmaf(n, n, -1.0f), c = h * g;
+        const float a = c * kxy, gy = g * y;
+        const float2 v = make_float2(g - gy, gy);
+        const float2 p1 = __ffma2_rn(make_float2(x, x), v, make_float2(-a, a));  // x ahead, both z
+        const float2 p0 = __fadd2_rn(v, make_float2(-p1.x, -p1.y));
+        if (CONE) {
+            const float b = h * kxz, e = c * kyz, ex = e * x;  // v holds g already
+            const float2 z2 = make_float2(z, z);
+            const float2 t = __ffma2_rn(z2, v, make_float2(-e, e));  // z ahead, both x
+            const float2 q1 = __ffma2_rn(z2, p1, __ffma2_rn(make_float2(b, b), v, make_float2(-ex, ex)));
+            const float2 q0 = __fadd2_rn(t, make_float2(-q1.x, -q1.y));
+            s11 = __fadd2_rn(s11, q1);
+            s01 = __fadd2_rn(s01, q0);
+            s10 = __fadd2_rn(s10, __fadd2_rn(p1, make_float2(-q1.x, -q1.y)));
+            s00 = __fadd2_rn(s00, __fadd2_rn(p0, make_float2(-q0.x, -q0.y)));
+        } else {
+            s10 = __fadd2_rn(s10, p1);
+            s00 = __fadd2_rn(s00, p0);
+        }
+    };
+    // samples at the ends of the range, where the inside test decides
+    auto sample = [&](int k) {
+        const float fk = (float)k;
+        const float px = fmaf(fk, r.dfx, r.fx0), py = fmaf(fk, r.dfy, r.fy0);
+        const float xf_ = floorf(px), yf_ = floorf(py);
+        if (!(xf_ >= 0.0f && xf_ + 1.0f < (float)nx && yf_ >= 0.0f && yf_ + 1.0f < (float)nx)) return;
+        int zi = iv;
+        float zw = 0.0f;
+        if (CONE) {
+            const float pz = fmaf(fk, r.dfz, r.fz0);
+            const float zf_ = floorf(pz);
+            if (!(zf_ >= 0.0f && zf_ + 1.0f < (float)p.nz)) return;
+            zi = (int)zf_;
+            zw = pz - zf_;
+        }
+        enter(zi * plane + (int)yf_ * nx + (int)xf_);
+        const float xw = px - xf_, yw = py - yf_;
+        add(1.0f, fx ? 1.0f - xw : xw, fy ? 1.0f - yw : yw, fz ? 1.0f - zw : zw);
+    };
+    int kis, kie;
+    interior_range(p, r, CONE, kis, kie);
+    if (p.K >= kMaxWalkSteps) {  // step indices would not be exact in float32
+        kis = r.ke + 1;
+        kie = r.ke;
+    }
+    for (int k = r.ks; k < kis; ++k) sample(k);
+    if (kis <= kie) {
+        const float M = 12582912.0f;
+        const unsigned MB = 0x4B400000u;  // bit pattern of M
+        const unsigned obias = CONE ? MB * (unsigned)(plane + nx + 1) : MB * (unsigned)(nx + 1) - (unsigned)(iv * plane);
+        const float2 dxy = make_float2(r.dfx, r.dfy), fxy0 = make_float2(r.fx0, r.fy0);
+        const float2 flip = make_float2(fx ? -1.0f : 1.0f, fy ? -1.0f : 1.0f), base = make_float2(fx ? 1.0f : 0.0f, fy ? 1.0f : 0.0f);
+        const float2 hd = make_float2(0.5f * dx, 0.5f * dy);
+        const float hdz = 0.5f * dzz;
+        const float ix = fminf(1.0f / dx, 1e6f), iy = fminf(1.0f / dy, 1e6f), iz = fminf(1.0f / dzz, 1e6f);
+        const float kend = (float)kie;
+        float fk = (float)kis;
+        while (fk <= kend) {
+            const float2 f = __ffma2_rn(make_float2(fk, fk), dxy, fxy0);
+            const float2 m = __fadd2_rd(f, make_float2(M, M));
+            const float2 fl = __fadd2_rn(m, make_float2(-M, -M));
+            const float2 w = __ffma2_rn(__fadd2_rn(f, make_float2(-fl.x, -fl.y)), flip, base);
+            unsigned off = __float_as_uint(m.x) + __float_as_uint(m.y) * (unsigned)nx - obias;
+            float zw = 0.0f;
+            if (CONE) {
+                const float pz = fmaf(fk, r.dfz, r.fz0);
+                const float mz = __fadd_rd(pz, M);
+                zw = pz - (mz - M);
+                if (fz) zw = 1.0f - zw;
+                off += __float_as_uint(mz) * (unsigned)plane;
+            }
+            // steps to the face ahead
+            float t = fminf(fminf(fmaf(w.x, -ix, ix), fmaf(w.y, -iy, iy)), kend - fk);
+            if (CONE) t = fminf(t, fmaf(zw, -iz, iz));
+            const float n1 = fmaxf(__fadd_rd(t, M) - M, 0.0f);
+            const float2 mid = __ffma2_rn(make_float2(n1, n1), hd, w);
+            enter((int)off);
+            add(n1 + 1.0f, mid.x, mid.y, fmaf(n1, hdz, zw));
+            fk += n1 + 1.0f;
+        }
+    }
+    for (int k = max(kie + 1, kis); k <= r.ke; ++k) sample(k);
+    flush();
+}
+
+template <bool CONE, bool CELLS, bool fx, bool fy>
+__device__ __forceinline__ void adjoint_ray_z(const FpParams& p, const Ray& r, int iv, float yv, float* __restrict__ out) {
+    if (CONE && r.dfz < 0.0f)
+        adjoint_ray<CONE, CELLS, fx, fy, CONE>(p, r, iv, yv, out);
+    else
+        adjoint_ray<CONE, CELLS, fx, fy, false>(p, r, iv, yv, out);
+}
+
 // Exact transpose of fp_kernel: every in-volume sample scatters its trilinear weights
-// times the ray value into the volume.  CELLS: the corner sums go to a cell-space
-// buffer instead (per cell of the 2x2x2 stencil its 8 corner sums, z-low 4 then
-// z-high 4, each group ordered (x,y) (x+1,y) (x,y+1) (x+1,y+1); fan beam: the 4 of the
-// slice), one or two 16-byte reductions per flush; adjoint_gather_kernel then sums
-// each voxel's corner entries from the cells that contain it.
-template <bool CELLS>
+// times the ray value into the volume.  As in the projector, the samples of one cell are
+// taken together: a corner's weights summed over n equally spaced samples with midpoint m
+// are n [u v w (m) + s^2 (du dv w + du dw v + dv dw u)(m)], s^2 = (n^2 - 1) / 12, for the
+// corner's linear weights u, v, w along the axes.
+//
+// CELLS, cone beam: the corner sums leave through two face buffers in the workspace, 16
+// bytes per voxel each: XF(z, y, x) holds the sums of the face {y, y+1} x {z, z+1} at x,
+// YF(z, y, x) those of the face {x, x+1} x {z, z+1} at y, both ordered (lo, lo) (hi, lo)
+// (lo, hi) (hi, hi) with z last.  A ray that crosses into the next cell along x or y is done
+// with the face it leaves behind: one 16-byte reduction; the four corners it shares with the
+// next cell stay in registers.  A crossing along z (rare) puts the four corners left
+// behind into XF as two 8-byte reductions, any other change of cell all eight as two
+// 16-byte ones.  adjoint_gather_kernel then sums each voxel's entries of the faces that
+// contain it.  In fan beam (4 corner sums per cell) and without a workspace (scalar atomics
+// into the volume) a cell's corners leave when the ray does.
+//
+// 250^2 x 45, 501 x 47 x 181 views: 2.5 ms, sample by sample with both 16-byte groups of a
+// cell reduced at every change of cell 4.6 ms.  The reductions bound it: the L2 is at 74 % of
+// its peak (16 bytes for each of 1.3e9 crossings), and neither more warps nor fewer
+// instructions (16 selects less per cell: 2 %) nor an XF with y first, whose entries of
+// neighbouring rays share a sector (0 %), bring much more.  Blocks of 4 rows of rays, not 8:
+// 2 % there, 4 % at 512^2 x 64; 8 where 4 would exceed the grid.
+inline int adjoint_rows(int nv) { return nv <= 4 * 65535 ? 4 : 8; }
+
+template <bool CONE, bool CELLS>
 __global__ void __launch_bounds__(256)
 fp_adjoint_kernel(FpParams p, const float* __restrict__ angles, const float* __restrict__ u_arr,
                   const float* __restrict__ v_arr, const float* __restrict__ czv, const float* __restrict__ pa,
                   const float* __restrict__ pxs, const float* __restrict__ sgm, const float* __restrict__ mask,
-                  float* __restrict__ vol) {
+                  float* __restrict__ out) {
     const int iu = blockIdx.x * blockDim.x + threadIdx.x;
     const int iv = blockIdx.z * blockDim.y + threadIdx.y;
     const int j = blockIdx.y;
@@ -639,79 +828,22 @@ fp_adjoint_kernel(FpParams p, const float* __restrict__ angles, const float* __r
     if (yv == 0.0f) return;
     Ray r;
     if (!setup_ray(p, iu, iv, j, angles, u_arr, v_arr, czv, pa, pxs, true, r)) return;
-    const int nx = p.nx;
-    const int plane = nx * nx;
-    // The 8 corner weights of consecutive samples in the same cell are summed in
-    // registers and scattered once when the ray leaves the cell.
-    int cell = -1;
-    float s00 = 0.f, s01 = 0.f, s10 = 0.f, s11 = 0.f, t00 = 0.f, t01 = 0.f, t10 = 0.f, t11 = 0.f;
-    auto flush = [&]() {
-        if (cell < 0) return;
-        if (CELLS) {
-            float* c = vol + (int64_t)cell * (p.cone ? 8 : 4);
-            red_add_v4(c, s00, s01, s10, s11);
-            if (p.cone) red_add_v4(c + 4, t00, t01, t10, t11);
-            s00 = s01 = s10 = s11 = t00 = t01 = t10 = t11 = 0.f;
-            return;
-        }
-        float* b = vol + cell;
-        atomicAdd(b, s00);
-        atomicAdd(b + 1, s01);
-        atomicAdd(b + nx, s10);
-        atomicAdd(b + nx + 1, s11);
-        if (p.cone) {
-            float* c = b + plane;
-            atomicAdd(c, t00);
-            atomicAdd(c + 1, t01);
-            atomicAdd(c + nx, t10);
-            atomicAdd(c + nx + 1, t11);
-        }
-        s00 = s01 = s10 = s11 = t00 = t01 = t10 = t11 = 0.f;
-    };
-    for (int k = r.ks; k <= r.ke; ++k) {
-        const float fk = (float)k;
-        const float fx = fmaf(fk, r.dfx, r.fx0);
-        const float fy = fmaf(fk, r.dfy, r.fy0);
-        const float xf = floorf(fx), yf = floorf(fy);
-        if (!(xf >= 0.0f && xf + 1.0f < (float)nx && yf >= 0.0f && yf + 1.0f < (float)nx)) continue;
-        const float xw = fx - xf, yw = fy - yf;
-        int zi;
-        float zw = 0.0f;
-        if (p.cone) {
-            const float fz = fmaf(fk, r.dfz, r.fz0);
-            const float zf = floorf(fz);
-            if (!(zf >= 0.0f && zf + 1.0f < (float)p.nz)) continue;
-            zi = (int)zf;
-            zw = fz - zf;
-        } else {
-            zi = iv;
-        }
-        const int off = zi * plane + (int)yf * nx + (int)xf;
-        if (off != cell) {
-            flush();
-            cell = off;
-        }
-        const float wl = p.cone ? (1.0f - zw) * yv : yv;
-        const float w00 = (1.0f - xw) * (1.0f - yw), w01 = xw * (1.0f - yw);
-        const float w10 = (1.0f - xw) * yw, w11 = xw * yw;
-        s00 += w00 * wl;
-        s01 += w01 * wl;
-        s10 += w10 * wl;
-        s11 += w11 * wl;
-        if (p.cone) {
-            const float wh = zw * yv;
-            t00 += w00 * wh;
-            t01 += w01 * wh;
-            t10 += w10 * wh;
-            t11 += w11 * wh;
-        }
+    if (r.dfx < 0.0f) {
+        if (r.dfy < 0.0f)
+            adjoint_ray_z<CONE, CELLS, true, true>(p, r, iv, yv, out);
+        else
+            adjoint_ray_z<CONE, CELLS, true, false>(p, r, iv, yv, out);
+    } else {
+        if (r.dfy < 0.0f)
+            adjoint_ray_z<CONE, CELLS, false, true>(p, r, iv, yv, out);
+        else
+            adjoint_ray_z<CONE, CELLS, false, false>(p, r, iv, yv, out);
     }
-    flush();
 }
 
-// vol[z][y][x] += the corner entries of the (up to) 8 cells that contain voxel
-// (z, y, x), in a fixed order.  C = 8 (cone beam) or 4 (fan beam: one slice per cell).
-template <int C>
+// vol[z][y][x] += its entries of the faces (cone beam, buffers XF and YF above) or cells
+// (fan beam) that contain it, in a fixed order.
+template <bool CONE>
 __global__ void __launch_bounds__(256)
 adjoint_gather_kernel(int nx, int nz, const float* __restrict__ cells, float* __restrict__ vol) {
     const int x = blockIdx.x * blockDim.x + threadIdx.x;
@@ -721,17 +853,26 @@ adjoint_gather_kernel(int nx, int nz, const float* __restrict__ cells, float* __
     const int64_t plane = (int64_t)nx * nx;
     const int64_t v = z * plane + (int64_t)y * nx + x;
     float acc = 0.0f;
+    if (CONE) {
+        const float* yfaces = cells + (int64_t)nz * plane * 4;
 #pragma unroll
-    for (int dz = 0; dz < C / 4; ++dz) {
-        if (z - dz < 0) continue;
+        for (int dz = 0; dz < 2; ++dz) {
+            if (z - dz < 0) continue;
+#pragma unroll
+            for (int d = 0; d < 2; ++d) {
+                const int64_t c = v - dz * plane;
+                if (y - d >= 0) acc += __ldg(cells + (c - (int64_t)d * nx) * 4 + dz * 2 + d);
+                if (x - d >= 0) acc += __ldg(yfaces + (c - d) * 4 + dz * 2 + d);
+            }
+        }
+    } else {
 #pragma unroll
         for (int dy = 0; dy < 2; ++dy) {
             if (y - dy < 0) continue;
 #pragma unroll
             for (int dx = 0; dx < 2; ++dx) {
                 if (x - dx < 0) continue;
-                const int64_t c = v - dz * plane - (int64_t)dy * nx - dx;
-                acc += __ldg(cells + c * C + dz * 4 + dy * 2 + dx);
+                acc += __ldg(cells + (v - (int64_t)dy * nx - dx) * 4 + dy * 2 + dx);
             }
         }
     }
@@ -1091,9 +1232,10 @@ int mct_fp_adjoint(const mct_geom* g, const mct_tables* t, const float* sgm, con
     MCT_TRY(make_params(g, p, "mct_fp_adjoint"));
     MCT_REQUIRE(t && t->angles && t->u && t->v && vol && sgm, "mct_fp_adjoint: NULL buffer");
     MCT_REQUIRE(!p.pmat || (t->pmat_a && t->pmat_xs), "mct_fp_adjoint: projection-matrix tables missing");
-    dim3 block(32, 8), grid((g->nu + 31) / 32, g->views, (g->nv + 7) / 8);
-    fp_adjoint_kernel<false><<<grid, block, 0, as_stream(stream)>>>(p, t->angles, t->u, t->v, t->cz, t->pmat_a,
-                                                                    t->pmat_xs, sgm, mask, vol);
+    const int rows = adjoint_rows(g->nv);
+    dim3 block(32, rows), grid((g->nu + 31) / 32, g->views, (g->nv + rows - 1) / rows);
+    auto go = p.cone ? fp_adjoint_kernel<true, false> : fp_adjoint_kernel<false, false>;
+    go<<<grid, block, 0, as_stream(stream)>>>(p, t->angles, t->u, t->v, t->cz, t->pmat_a, t->pmat_xs, sgm, mask, vol);
     return launched("fp_adjoint_kernel");
 }
 
@@ -1112,18 +1254,18 @@ int mct_fp_adjoint_cells(const mct_geom* g, const mct_tables* t, const float* sg
     MCT_REQUIRE(g->nx <= 65535 * 8 && g->nz <= 65535, "mct_fp_adjoint_cells: at most 524280 x 524280 x 65535 voxels");
     cudaStream_t s = as_stream(stream);
     float* cells = static_cast<float*>(workspace);
-    const int C = p.cone ? 8 : 4;
     MCT_REQUIRE(cudaMemsetAsync(cells, 0, mct_fp_adjoint_workspace_size(g), s) == cudaSuccess,
                 "mct_fp_adjoint_cells: clearing the workspace failed");
-    dim3 block(32, 8), grid((g->nu + 31) / 32, g->views, (g->nv + 7) / 8);
-    fp_adjoint_kernel<true><<<grid, block, 0, s>>>(p, t->angles, t->u, t->v, t->cz, t->pmat_a, t->pmat_xs, sgm,
-                                                   mask, cells);
+    const int rows = adjoint_rows(g->nv);
+    dim3 block(32, rows), grid((g->nu + 31) / 32, g->views, (g->nv + rows - 1) / rows);
+    auto go = p.cone ? fp_adjoint_kernel<true, true> : fp_adjoint_kernel<false, true>;
+    go<<<grid, block, 0, s>>>(p, t->angles, t->u, t->v, t->cz, t->pmat_a, t->pmat_xs, sgm, mask, cells);
     MCT_TRY(launched("fp_adjoint_kernel"));
     dim3 gb(32, 8), gg((g->nx + 31) / 32, (g->nx + 7) / 8, g->nz);
-    if (C == 8)
-        adjoint_gather_kernel<8><<<gg, gb, 0, s>>>(g->nx, g->nz, cells, vol);
+    if (p.cone)
+        adjoint_gather_kernel<true><<<gg, gb, 0, s>>>(g->nx, g->nz, cells, vol);
     else
-        adjoint_gather_kernel<4><<<gg, gb, 0, s>>>(g->nx, g->nz, cells, vol);
+        adjoint_gather_kernel<false><<<gg, gb, 0, s>>>(g->nx, g->nz, cells, vol);
     return launched("adjoint_gather_kernel");
 }
 
