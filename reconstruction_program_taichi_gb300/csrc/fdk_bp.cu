@@ -25,20 +25,25 @@
 namespace mct {
 namespace {
 
-constexpr int BP_TX = 32, BP_TY = 8, BP_ZC = 16, BP_VCHUNK = 1024;
+// Blocks of two warps: with 8 warps (32 x 8 columns) a small volume's 256 blocks left a third
+// of the SMs half empty, and the warps of a block waited for each other at every chunk of
+// views.  128x128x64 / 180 views, FDK: 284 -> 275 us; 333x333x101 / 500 views, curved 5.03 ->
+// 4.72 ms; 512x512x256 / 1080 views 49.3 -> 46.6 ms; 256^3 / 360 views coronal, bf16 4.07 ms
+// both (one warp: 4.19 ms there, the others as with two; four warps 278 us, 4.82, 47.7 ms).
+constexpr int BP_TX = 8, BP_TY = 8, BP_ZC = 16, BP_VCHUNK = 256;
 constexpr int BP_WX = 4;  // columns along x per warp (32 / BP_WX along y)
 static_assert(BP_TX % BP_WX == 0 && BP_TY % (32 / BP_WX) == 0, "warps tile the block");
 static_assert(BP_ZC % 2 == 0, "the 16-bit axial loop takes slices in pairs");
-// Minimum resident blocks per SM, i.e. a register budget of 65536 / (256 * minb) per
+// Minimum resident blocks per SM, i.e. a register budget of 65536 / (64 * minb) per
 // thread.  The axial kernel needs enough registers to issue all BP_ZC stencil gathers
 // of a view before their arithmetic (that hides the gather latency): measured at
-// 512x512x256 / 1080 views, float32 stencils run fastest with 128 registers (2
-// blocks), bf16 stencils with 80 (3 blocks); 16-bit stencils of a curved detector spill
-// there (512x512x128 / 360 views, FDK: 15.9 ms with 3 blocks, 8.4 with 2).  The general
-// modes use 2.
+// 512x512x256 / 1080 views, float32 stencils run fastest with 128 registers (8
+// blocks), bf16 stencils with 80 (12 blocks); 16-bit stencils of a curved detector spill
+// there (512x512x128 / 360 views, FDK: 15.9 ms with 12 blocks, 8.4 with 8).  The general
+// modes use 8.
 template <int MODE, typename QT, bool CURVED>
 constexpr int bp_min_blocks() {
-    return (MODE == 0 || MODE == 2) && sizeof(QT) == 8 && !CURVED ? 3 : 2;
+    return (MODE == 0 || MODE == 2) && sizeof(QT) == 8 && !CURVED ? 12 : 8;
 }
 
 struct BpParams {
@@ -100,11 +105,11 @@ fdk_bp_kernel(BpParams p, const float* __restrict__ angles, const float* __restr
     __shared__ float4 tab[VCH];  // {cos b, sin b, dbeta*div, unused}
     __shared__ __align__(16) float pms[MODE == 3 ? 12 * VCH : 4];
     const int tid = threadIdx.y * BP_TX + threadIdx.x;
-    // A warp is 4 columns along x x 8 along y of the block's 32 x 8: for one view its
+    // A warp is 4 columns along x x 8 along y of the block's 8 x 8: for one view its
     // columns project onto fewer detector columns than a row of 32 (about 4|sin| + 8|cos|
     // + 1 against 32|sin| + 1), so each gather touches fewer L1 lines.  At 512x512x256 /
     // 1080 views: 52.19 -> 50.22 ms (float32), 49.07 -> 47.17 ms (bf16); warps of 16 x 2
-    // 51.62 / 48.50, 8 x 4 50.78 / 47.70; blocks of 16 x 16 or 8 x 32 no better.
+    // 51.62 / 48.50, 8 x 4 50.78 / 47.70 (blocks of 32 x 8; in today's 8 x 8, 8 x 4 costs 1 %).
     const int warp = tid >> 5, lane = tid & 31;
     const int ix = blockIdx.x * BP_TX + (warp % (BP_TX / BP_WX)) * BP_WX + (lane % BP_WX);
     const int iy = blockIdx.y * BP_TY + (warp / (BP_TX / BP_WX)) * (32 / BP_WX) + lane / BP_WX;

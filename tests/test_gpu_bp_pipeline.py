@@ -87,3 +87,27 @@ def test_solver_backprojection_matches_the_oracle_off_the_detector(views, storag
     assert np.mean((got == 0) != (ref == 0)) < 1e-3
     both = (got != 0) & (ref != 0)
     assert rel_l2(got[both], ref[both]) < 5 * TOL[storage]  # a row at the edge in or out: one view of `views`
+
+
+@pytest.mark.parametrize("n,nz,views,kw", [
+    (7, 5, 255, {}), (8, 16, 256, {}), (9, 17, 257, {"CurvedDetector": True}), (17, 3, 513, {"ReconViewMode": "coronal"})])
+def test_backprojection_at_the_edges_of_blocks_and_view_tables(n, nz, views, kw, cuda):
+    """Volumes of one column less and more than a block, scans of one view less and more than
+    the block's table of views."""
+    import torch
+    from reconstruction_program_taichi_gb300 import geometry, ops
+    o = _cone_obj(n=n, nz=nz, nu=3 * n, nv=2 * nz, views=views, **kw)
+    dg = geometry.fbp_geometry(o)
+    g = dg.geom
+    f = np.random.default_rng(views).normal(0, 1, (views, g.nv, g.nu)).astype(np.float32)
+    got = ops.fdk_bp(dg, ops.pack(dg, torch.from_numpy(f).cuda())).cpu().numpy()
+    u, v, ang = geometry.fbp_arrays(o)
+    ref = F.fdk_bp(f.transpose(1, 0, 2), ang, u, v, nx=o.img_dim, nz=o.img_dim_z, px=o.img_pix_size,
+                   pz=o.img_voxel_height, cx=o.img_center_x, cy=o.img_center_y, cz=o.img_center_z,
+                   sid=o.source_isocenter_dis, sdd=o.source_det_dis, dv=o.det_elem_height, img_rot=o.img_rot,
+                   total_scan_angle=o.total_scan_angle, short_scan=o.short_scan, cone_beam=True,
+                   curved=o.curved_dect, view_mode=o.recon_view_mode)
+    assert np.mean((got == 0) != (ref == 0)) < 1e-3
+    both = (got != 0) & (ref != 0)
+    assert both.sum() > 0.2 * both.size
+    assert rel_l2(got[both], ref[both]) < TOL["f32"]
