@@ -209,11 +209,11 @@ enum Walk { kCells, kWindows, kSamples };
 // Resident blocks per SM that the register allocation of fp_kernel targets: 5 (48
 // registers) with copies.  512x512x256 / 1080 views, float32: 4 blocks 160.6 ms, 5
 // 158.9, 6 164.7; 512x512x64 / 360 views, bf16: 4 blocks 13.55 ms, 5 13.41, 6 14.27.
-// The fan-beam path needs 40 registers (6 blocks), the walk by samples 62 (4; 5 blocks
-// cost it 10 %).
-template <bool CONE, int WALK>
+// The fan-beam path needs 40 registers (6 blocks), the walk of 16-bit cells by samples 62
+// (4; 5 blocks cost it 10 %); that of float32 quads is 3 to 4 % faster with 5 than with 4.
+template <bool CONE, typename ZT, int WALK>
 constexpr int fp_min_blocks() {
-    return WALK == kSamples ? 4 : CONE ? 5 : 6;
+    return WALK == kSamples && sizeof(ZT) == 16 && !std::is_same<ZT, Quad16>::value ? 4 : CONE ? 5 : 6;
 }
 
 // Above this many steps a ray's indices are no longer exact in float32 (and would not
@@ -250,11 +250,12 @@ constexpr int kWinPlanes = 64;
 //     512x512x64, 360 views, bf16          18.32 / 13.41 / 14.9 (windows: 16-bit cells lose)
 //     512^2 fan beam, 720 views            1.34 / 0.80 / 0.66
 //     256x256x128, 360 views, step 0.1     18.83 / 7.19;  step 0.5: 6.20 / 5.95
-// 16-bit cells, which the walk by samples reloads with one load and which cells hold twice
-// the arithmetic for, are walked by samples from the step on where it is the faster
-// (walk_by_samples below): each keeps its cell in registers until it enters another.
+// Where a step leaves about one sample per cell or fewer, the sum over cells saves nothing
+// and costs its second-order terms: from the step on where it is the faster
+// (walk_by_samples below), a ray is walked by samples and keeps its cell in registers until
+// it enters another.
 template <bool CONE, bool ZP, typename ZT, int WALK>
-__global__ void __launch_bounds__(256, fp_min_blocks<CONE, WALK>())
+__global__ void __launch_bounds__(256, fp_min_blocks<CONE, ZT, WALK>())
 fp_kernel(FpParams p, const float* __restrict__ angles, const float* __restrict__ u_arr,
           const float* __restrict__ v_arr, const float* __restrict__ czv, const float* __restrict__ pa,
           const float* __restrict__ pxs, const float* __restrict__ vol, const float* __restrict__ vol_t,
@@ -1025,13 +1026,19 @@ inline int copy_pitch(const mct_geom* g) {
     const int pitch = ((g->nx + 7) & ~7) + 3;
     return g->nx >= 128 && (int64_t)g->nz * g->nx * pitch < ((int64_t)1 << 31) ? pitch : g->nx;
 }
-// Whether 16-bit cells are walked by samples: few samples per cell (the ray's cell
+// Whether float32 quads are walked in windows (fan beam always is: its warps span more cells).
+inline bool walk_in_windows(const mct_geom* g) { return g->nx >= 256; }
+// Whether a ray with copies is walked by samples: few samples per cell (the ray's cell
 // crossings per voxel length are 1.33 on average over a scan).  256x256x64, 360 views, by
 // samples / by cells, ms: bf16 step 0.2 (2.2 samples per cell) 4.84 / 3.46, 0.3 (1.4) 3.22 /
 // 3.31 (140 columns, 300 views: 0.929 / 0.966), 0.5 (0.9) 2.1 / 2.95; float16, which pays
-// more per load, 0.3 3.8 / 3.60, 0.5 2.33 / 3.19.
+// more per load, 0.3 3.8 / 3.60, 0.5 2.33 / 3.19.  float32, us: 123x123x51, 686 views, 0.3
+// 1320 / 1261, 0.4 (1.1) 1106 / 1193, 0.5 974 / 1119; 224x224x64, 120 views, 0.4 901 / 897,
+// 0.5 795 / 841, 0.7 664 / 654; 64^3, 180 views, 0.4 139 / 153, 0.5 126 / 144.  With windows,
+// from 256 columns on, cells stay: 512x512x64, 90 views, 0.5 3567 / 3252, 0.7 3024 / 2524
+// (300 columns, 300 views: 2164 / 2250, 1772 / 1817).
 inline bool walk_by_samples(const mct_geom* g, int32_t dtype) {
-    if (dtype == MCT_F32) return false;
+    if (dtype == MCT_F32 && walk_in_windows(g)) return false;
     const double step = g->fp_step * std::sqrt(2.0 + ((double)g->pz / g->px) * ((double)g->pz / g->px));
     return 1.0 / (1.33 * step) < (dtype == MCT_BF16 ? 1.5 : 1.2);
 }
@@ -1129,26 +1136,27 @@ int fp_storage_impl(const mct_geom* g, const mct_tables* t, const TIN* vol_in, c
     dim3 tb(32, 8), tg((g->nx + 31) / 32, (g->nx + 31) / 32, g->nz);
     // Ray tiles: 16 detector columns x 16 consecutive views of one row, warps of 2^wcs
     // columns.  The rays of neighbouring views cross nearly the same cells, the more so the
-    // closer the views, so long scans take warps of 4 columns x 8 views and short ones 16
-    // columns x 2 views.  float32, ms with 4 / 16 columns per warp: 512x512x256, 1080 views
-    // 159.0 / 168.7; 128x128x64, 270 views 0.698 / 0.741; 512x512x64: 180 views 8.68 / 8.28,
-    // 90 views 5.23 / 4.86, 60 views 3.74 / 3.48.  16-bit cells take 4 views x 4 rows: bf16
-    // 512x512x128, 90 views 7.60 ms against 7.73 with 16 views; 256x256x64, 360 views 3.457
-    // against 3.480; by samples they keep warps of 4 columns.  Fan
-    // beam: warps of 8 columns x 4 views (512^2, 720 views, 4 / 8 / 16 columns: 0.604 /
-    // 0.596 / 0.595; 128^2 x 16, 360 views 0.327 / 0.324 / 0.339; one row of 32 columns x 8
-    // rows, 7 of them idle for one slice: 0.664).
+    // closer the views, so scans of at least 256 views, or of a view per image column, take
+    // warps of 4 columns x 8 views and others 16 columns x 2 views.  float32, ms with 4 / 16
+    // columns per warp: 512x512x256, 1080 views 159.0 / 168.7; 512x512x64: 180 views 8.68 /
+    // 8.28, 90 views 5.23 / 4.86, 60 views 3.74 / 3.48; 224x224x64, 300 views 2.04 / 2.14;
+    // 128x128x64, 270 views 0.698 / 0.741; 123x123x51: 140 views 0.325 / 0.335, 90 views 0.241
+    // / 0.240; 100x100x40, 200 views 0.228 / 0.245; 64^3, 180 views 0.158 / 0.169.  16-bit
+    // cells take 4 views x 4 rows: bf16 512x512x128, 90 views 7.60 ms against 7.73 with 16
+    // views; 256x256x64, 360 views 3.457 against 3.480; by samples they keep warps of 4
+    // columns.  Fan beam: warps of 8 columns x 4 views (512^2, 720 views, 4 / 8 / 16 columns:
+    // 0.604 / 0.596 / 0.595; 128^2 x 16, 360 views 0.327 / 0.324 / 0.339; one row of 32
+    // columns x 8 rows, 7 of them idle for one slice: 0.664).
     // With copies, 4 row tiles are taken in turn per view group: neighbouring rows' rays
     // cross nearly the same cells, and the outer rows' slab (up to ~50 planes) does not fit
     // L2 across all views.  Otherwise row tiles are only grouped where the grid needs it.
     const bool copies = p.cone && workspace;
-    const bool long_scan = g->views >= 256, by_samples = copies && walk_by_samples(g, dtype);
+    const bool long_scan = g->views >= 256 || g->views >= g->nx, by_samples = copies && walk_by_samples(g, dtype);
     p.bcs = 4;
     p.vshift = copies && dtype != MCT_F32 ? 2 : 4;
     p.wcs = !p.cone ? 3 : long_scan || by_samples ? 2 : 4;
     p.rs = copies ? (p.vshift == 4 ? 2 : 0) : (g->nv > 65535 ? 3 : 0);
     if (copies) p.pitch = copy_pitch(g);
-    const bool windows = g->nx >= 256;  // float32 quads; fan beam always (its warps span more cells)
     const int vb = 1 << p.vshift, rb = 1 << (8 - p.bcs - p.vshift + p.rs), cb = 1 << p.bcs;
     dim3 block(32, 8), grid((g->nu + cb - 1) / cb, ((g->views + vb - 1) / vb) << p.rs, (g->nv + rb - 1) / rb);
     const size_t n = copy_elems(g);
@@ -1183,7 +1191,9 @@ int fp_storage_impl(const mct_geom* g, const mct_tables* t, const TIN* vol_in, c
         quad32_kernel<<<tg, tb, 0, s>>>(g->nx, g->nz, p.pitch, vol_in, reinterpret_cast<float4*>(cx),
                                         reinterpret_cast<float4*>(cy));
         MCT_TRY(launched("quad32_kernel"));
-        auto go = windows ? fp_kernel<true, true, Quad16, kWindows> : fp_kernel<true, true, Quad16, kCells>;
+        auto go = by_samples           ? fp_kernel<true, true, Quad16, kSamples>
+                  : walk_in_windows(g) ? fp_kernel<true, true, Quad16, kWindows>
+                                       : fp_kernel<true, true, Quad16, kCells>;
         go<<<grid, block, 0, s>>>(p, t->angles, t->u, t->v, t->cz, t->pmat_a, t->pmat_xs, vol, nullptr, cx, cy, mask, sgm,
                                   nullptr);
     } else if constexpr (kIn32) {

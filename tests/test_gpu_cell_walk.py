@@ -52,3 +52,11 @@ def test_projection_by_cells_matches_the_sum_over_samples(n, nz, nu, nv, views, 
                     for j in some], axis=1)
     for g in got:
         assert rel_l2(g.cpu().numpy()[:, some], ref) < TOL[storage]
+
+
+@pytest.mark.parametrize("n,nz,nu,nv,views,step", [
+    (40, 8, 35, 9, 39, 0.36), (40, 8, 35, 9, 39, 0.37), (40, 8, 35, 9, 40, 0.5), (128, 6, 17, 5, 9, 0.5),
+    (255, 6, 17, 3, 5, 0.5), (256, 6, 17, 3, 5, 0.5), (9, 5, 33, 3, 20, 1.7)])
+def test_float32_projection_by_samples_matches_the_sum_over_samples(n, nz, nu, nv, views, step, cuda):
+    """Both sides of the step, width and view count that decide how float32 quads are walked."""
+    test_projection_by_cells_matches_the_sum_over_samples(n, nz, nu, nv, views, step, "f32", True, cuda)
