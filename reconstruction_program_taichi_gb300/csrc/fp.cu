@@ -20,6 +20,7 @@ namespace mct {
 namespace {
 
 struct FpParams {
+    bool by_samples;  // the adjoint takes samples one by one
     int nx, nz, nu, nv, views, K, cone, curved, pmat;
     float sid, sdd, cx, cy, cz;
     float stepvd, l_min, inv_px, inv_pz;
@@ -630,6 +631,7 @@ __device__ __forceinline__ void adjoint_ray(const FpParams& p, const Ray& r, int
     const int nx = p.nx;
     const int plane = nx * nx;
     const int stepx = fx ? -1 : 1, stepy = fy ? -nx : nx, stepz = fz ? -plane : plane;
+    const int first = (fx ? 1 : 0) + (fy ? nx : 0) + (CONE && fz ? plane : 0);  // from the cell to its corner behind on all axes
     const unsigned xf = fx ? 1u : 0u;                                            // XF of the face behind
     const unsigned yf = (unsigned)p.nz * (unsigned)plane + (fy ? (unsigned)nx : 0u);  // YF of the face behind
     int cell = -1;
@@ -649,19 +651,17 @@ __device__ __forceinline__ void adjoint_ray(const FpParams& p, const Ray& r, int
             const float2 lo = order(fx, s00.x, s10.x), hi = order(fx, s00.y, s10.y);  // y behind, ahead
             red_add_v4(out + (size_t)cell * 4, fy ? hi.x : lo.x, fy ? hi.y : lo.y, fy ? lo.x : hi.x, fy ? lo.y : hi.y);
         } else {
-            float* b = out + cell;
-            const int x0 = fx ? 1 : 0, y0 = fy ? nx : 0, y1 = nx - y0;
-            float* q = b + (CONE && fz ? plane : 0);
-            atomicAdd(q + x0 + y0, s00.x);
-            atomicAdd(q + 1 - x0 + y0, s10.x);
-            atomicAdd(q + x0 + y1, s00.y);
-            atomicAdd(q + 1 - x0 + y1, s10.y);
+            float* q = out + (cell + first);
+            atomicAdd(q, s00.x);
+            atomicAdd(q + stepx, s10.x);
+            atomicAdd(q + stepy, s00.y);
+            atomicAdd(q + stepx + stepy, s10.y);
             if (CONE) {
-                q = b + (fz ? 0 : plane);
-                atomicAdd(q + x0 + y0, s01.x);
-                atomicAdd(q + 1 - x0 + y0, s11.x);
-                atomicAdd(q + x0 + y1, s01.y);
-                atomicAdd(q + 1 - x0 + y1, s11.y);
+                q += stepz;
+                atomicAdd(q, s01.x);
+                atomicAdd(q + stepx, s11.x);
+                atomicAdd(q + stepy, s01.y);
+                atomicAdd(q + stepx + stepy, s11.y);
             }
         }
         s00 = s01 = s10 = s11 = make_float2(0.f, 0.f);
@@ -669,20 +669,39 @@ __device__ __forceinline__ void adjoint_ray(const FpParams& p, const Ray& r, int
     auto enter = [&](int off) {
         if (off == cell) return;
         const int d = off - cell;
-        if (CONE && CELLS && cell >= 0 && (d == stepx || d == stepy)) {
+        if ((CONE || !CELLS) && cell >= 0 && (d == stepx || d == stepy)) {
             const bool x = d == stepx;
             const float b0 = x ? s00.y : s10.x, b1 = x ? s01.y : s11.x;  // the face's other corner, z behind and ahead
-            const bool f = x ? fy : fx;
-            face((unsigned)cell + (x ? xf : yf), order(f, s00.x, b0), order(f, s01.x, b1));
+            if constexpr (CELLS) {
+                const bool f = x ? fy : fx;
+                face((unsigned)cell + (x ? xf : yf), order(f, s00.x, b0), order(f, s01.x, b1));
+            } else {
+                float* q = out + (cell + first);
+                const int t = x ? stepy : stepx;
+                atomicAdd(q, s00.x);
+                atomicAdd(q + t, b0);
+                if (CONE) {
+                    atomicAdd(q + stepz, s01.x);
+                    atomicAdd(q + stepz + t, b1);
+                }
+            }
             s00 = make_float2(x ? s10.x : s00.y, x ? s10.y : 0.0f);
             s10 = make_float2(x ? 0.0f : s10.y, 0.0f);
             s01 = make_float2(x ? s11.x : s01.y, x ? s11.y : 0.0f);
             s11 = make_float2(x ? 0.0f : s11.y, 0.0f);
-        } else if (CONE && CELLS && cell >= 0 && d == stepz) {
-            float* q = out + ((size_t)((unsigned)cell + xf) * 4 + (fz ? 2 : 0));
-            const float2 a = order(fy, s00.x, s00.y), b = order(fy, s10.x, s10.y);
-            red_add_v2(q, a.x, a.y);
-            red_add_v2(out + ((size_t)((unsigned)cell + 1u - xf) * 4 + (fz ? 2 : 0)), b.x, b.y);
+        } else if (CONE && cell >= 0 && d == stepz) {
+            if constexpr (CELLS) {
+                float* q = out + ((size_t)((unsigned)cell + xf) * 4 + (fz ? 2 : 0));
+                const float2 a = order(fy, s00.x, s00.y), b = order(fy, s10.x, s10.y);
+                red_add_v2(q, a.x, a.y);
+                red_add_v2(out + ((size_t)((unsigned)cell + 1u - xf) * 4 + (fz ? 2 : 0)), b.x, b.y);
+            } else {
+                float* q = out + (cell + first);
+                atomicAdd(q, s00.x);
+                atomicAdd(q + stepy, s00.y);
+                atomicAdd(q + stepx, s10.x);
+                atomicAdd(q + stepx + stepy, s10.y);
+            }
             s00 = s01;
             s10 = s11;
             s01 = s11 = make_float2(0.f, 0.f);
@@ -736,7 +755,7 @@ __device__ __forceinline__ void adjoint_ray(const FpParams& p, const Ray& r, int
     };
     int kis, kie;
     interior_range(p, r, CONE, kis, kie);
-    if (p.K >= kMaxWalkSteps) {  // step indices would not be exact in float32
+    if (p.K >= kMaxWalkSteps || p.by_samples) {  // kMaxWalkSteps: step indices would not be exact in float32
         kis = r.ke + 1;
         kie = r.ke;
     }
@@ -794,25 +813,28 @@ __device__ __forceinline__ void adjoint_ray_z(const FpParams& p, const Ray& r, i
 // are n [u v w (m) + s^2 (du dv w + du dw v + dv dw u)(m)], s^2 = (n^2 - 1) / 12, for the
 // corner's linear weights u, v, w along the axes.
 //
-// CELLS, cone beam: the corner sums leave through two face buffers in the workspace, 16
-// bytes per voxel each: XF(z, y, x) holds the sums of the face {y, y+1} x {z, z+1} at x,
-// YF(z, y, x) those of the face {x, x+1} x {z, z+1} at y, both ordered (lo, lo) (hi, lo)
-// (lo, hi) (hi, hi) with z last.  A ray that crosses into the next cell along x or y is done
-// with the face it leaves behind: one 16-byte reduction; the four corners it shares with the
-// next cell stay in registers.  A crossing along z (rare) puts the four corners left
-// behind into XF as two 8-byte reductions, any other change of cell all eight as two
-// 16-byte ones.  adjoint_gather_kernel then sums each voxel's entries of the faces that
-// contain it.  In fan beam (4 corner sums per cell) and without a workspace (scalar atomics
-// into the volume) a cell's corners leave when the ray does.
+// A ray that crosses into the next cell along x or y is done with the face it leaves
+// behind: that face's corners are reduced, the ones it shares with the next cell stay in
+// registers.  A crossing along z (rare) does the same with the corners left behind, any
+// other change of cell reduces all.  Without CELLS the corners are added to the volume one
+// by one.  CELLS, cone beam: the faces' sums go to two buffers in the workspace, 16 bytes
+// per voxel each: XF(z, y, x) holds the face {y, y+1} x {z, z+1} at x, YF(z, y, x) the face
+// {x, x+1} x {z, z+1} at y, both ordered (lo, lo) (hi, lo) (lo, hi) (hi, hi) with z last:
+// one 16-byte reduction a face, two of 8 bytes in XF for a crossing along z;
+// adjoint_gather_kernel then sums each voxel's entries of the faces that contain it.
+// CELLS, fan beam: the 4 corner sums of a cell are one 16-byte reduction anyway (two edges
+// of 8 bytes cost more: a reduction of 8 bytes takes the L2 as long as one of 16).
 //
 // 250^2 x 45, 501 x 47 x 181 views: 2.5 ms, sample by sample with both 16-byte groups of a
 // cell reduced at every change of cell 4.6 ms.  The reductions bound it: the L2 is at 74 % of
 // its peak (16 bytes for each of 1.3e9 crossings), and neither more warps nor fewer
 // instructions (16 selects less per cell: 2 %) nor an XF with y first, whose entries of
-// neighbouring rays share a sector (0 %), bring much more.  Blocks of 4 rows of rays, not 8:
-// 2 % there, 4 % at 512^2 x 64; 8 where 4 would exceed the grid.
-inline int adjoint_rows(int nv) { return nv <= 4 * 65535 ? 4 : 8; }
-
+// neighbouring rays share a sector (0 %), bring much more.  Without CELLS, ms before /
+// after: 123x123x51, 300 views 7.95 / 5.16, step 0.5 6.06 / 5.05; fan beam 300^2 x 4, 360
+// views 2.35 / 1.40.  Blocks of 8 rows of rays (4 cost the scalar additions 2 to 10 %); of 4
+// for cone beam with CELLS (grad above 2 %, 512^2 x 64 4 %), where the grid allows it.
+// Fan beam with CELLS goes by samples where a cell holds about one (300^2 x 4, 360 views,
+// by samples / by cells, ms: step 0.2 1.02 / 0.71, 0.4 0.64 / 0.66, 0.5 0.60 / 0.64).
 template <bool CONE, bool CELLS>
 __global__ void __launch_bounds__(256)
 fp_adjoint_kernel(FpParams p, const float* __restrict__ angles, const float* __restrict__ u_arr,
@@ -1028,8 +1050,12 @@ inline int copy_pitch(const mct_geom* g) {
 }
 // Whether float32 quads are walked in windows (fan beam always is: its warps span more cells).
 inline bool walk_in_windows(const mct_geom* g) { return g->nx >= 256; }
-// Whether a ray with copies is walked by samples: few samples per cell (the ray's cell
-// crossings per voxel length are 1.33 on average over a scan).  256x256x64, 360 views, by
+// Samples of a ray per cell: its cell crossings per voxel length are 1.33 on average over a scan.
+inline double samples_per_cell(const mct_geom* g) {
+    const double step = g->fp_step * std::sqrt(2.0 + ((double)g->pz / g->px) * ((double)g->pz / g->px));
+    return 1.0 / (1.33 * step);
+}
+// Whether a ray with copies is walked by samples: few samples per cell.  256x256x64, 360 views, by
 // samples / by cells, ms: bf16 step 0.2 (2.2 samples per cell) 4.84 / 3.46, 0.3 (1.4) 3.22 /
 // 3.31 (140 columns, 300 views: 0.929 / 0.966), 0.5 (0.9) 2.1 / 2.95; float16, which pays
 // more per load, 0.3 3.8 / 3.60, 0.5 2.33 / 3.19.  float32, us: 123x123x51, 686 views, 0.3
@@ -1039,8 +1065,7 @@ inline bool walk_in_windows(const mct_geom* g) { return g->nx >= 256; }
 // (300 columns, 300 views: 2164 / 2250, 1772 / 1817).
 inline bool walk_by_samples(const mct_geom* g, int32_t dtype) {
     if (dtype == MCT_F32 && walk_in_windows(g)) return false;
-    const double step = g->fp_step * std::sqrt(2.0 + ((double)g->pz / g->px) * ((double)g->pz / g->px));
-    return 1.0 / (1.33 * step) < (dtype == MCT_BF16 ? 1.5 : 1.2);
+    return samples_per_cell(g) < (dtype == MCT_BF16 ? 1.5 : 1.2);
 }
 inline size_t copy_elems(const mct_geom* g) { return (size_t)g->nz * g->nx * copy_pitch(g); }
 
@@ -1242,8 +1267,7 @@ int mct_fp_adjoint(const mct_geom* g, const mct_tables* t, const float* sgm, con
     MCT_TRY(make_params(g, p, "mct_fp_adjoint"));
     MCT_REQUIRE(t && t->angles && t->u && t->v && vol && sgm, "mct_fp_adjoint: NULL buffer");
     MCT_REQUIRE(!p.pmat || (t->pmat_a && t->pmat_xs), "mct_fp_adjoint: projection-matrix tables missing");
-    const int rows = adjoint_rows(g->nv);
-    dim3 block(32, rows), grid((g->nu + 31) / 32, g->views, (g->nv + rows - 1) / rows);
+    dim3 block(32, 8), grid((g->nu + 31) / 32, g->views, (g->nv + 7) / 8);
     auto go = p.cone ? fp_adjoint_kernel<true, false> : fp_adjoint_kernel<false, false>;
     go<<<grid, block, 0, as_stream(stream)>>>(p, t->angles, t->u, t->v, t->cz, t->pmat_a, t->pmat_xs, sgm, mask, vol);
     return launched("fp_adjoint_kernel");
@@ -1266,7 +1290,8 @@ int mct_fp_adjoint_cells(const mct_geom* g, const mct_tables* t, const float* sg
     float* cells = static_cast<float*>(workspace);
     MCT_REQUIRE(cudaMemsetAsync(cells, 0, mct_fp_adjoint_workspace_size(g), s) == cudaSuccess,
                 "mct_fp_adjoint_cells: clearing the workspace failed");
-    const int rows = adjoint_rows(g->nv);
+    p.by_samples = !p.cone && samples_per_cell(g) < 1.2;
+    const int rows = p.cone && g->nv <= 4 * 65535 ? 4 : 8;
     dim3 block(32, rows), grid((g->nu + 31) / 32, g->views, (g->nv + rows - 1) / rows);
     auto go = p.cone ? fp_adjoint_kernel<true, true> : fp_adjoint_kernel<false, true>;
     go<<<grid, block, 0, s>>>(p, t->angles, t->u, t->v, t->cz, t->pmat_a, t->pmat_xs, sgm, mask, cells);

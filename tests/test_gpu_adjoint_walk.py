@@ -45,3 +45,8 @@ def test_adjoint_by_cells_matches_the_sum_over_samples(n, nz, nu, nv, views, ste
     for ws in (True, None):
         got = ops.fp_adjoint(dg, yt, mask=m, workspace=ws).cpu().numpy()
         assert rel_l2(got[inner], ref[inner]) < TOL
+
+
+@pytest.mark.parametrize("step", [0.36, 0.37, 0.44, 0.45])
+def test_fan_beam_adjoint_on_both_sides_of_the_walk_by_samples(step, cuda):
+    test_adjoint_by_cells_matches_the_sum_over_samples(34, 3, 37, 3, 30, step, False, cuda)
