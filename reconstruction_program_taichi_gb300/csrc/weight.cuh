@@ -51,9 +51,10 @@ __device__ __forceinline__ float parker(const WeightParams& p, float beta, float
 }
 
 // Distance factor's denominator and the curved detector's cosine (per row v, column u).
+template <bool PLAIN = false>
 __device__ __forceinline__ float weight_den(const WeightParams& p, float u, float v) {
     const float sdd = p.sdd;
-    return p.curved ? sqrtf(sdd * sdd + v * v) : sqrtf(sdd * sdd + u * u + v * v);
+    return !PLAIN && p.curved ? sqrtf(sdd * sdd + v * v) : sqrtf(sdd * sdd + u * u + v * v);
 }
 __device__ __forceinline__ float weight_cos(const WeightParams& p, float u) {
     return p.curved ? cosf((-1.0f) * u / p.sdd) : 0.0f;
@@ -62,9 +63,11 @@ __device__ __forceinline__ float weight_cos(const WeightParams& p, float u) {
 // One weighted element: beam-hardening polynomial, cosine weight, Parker weight
 // (beta = |angle - angle_0| of the element's view and gamma, the column's fan angle, are used
 // with short scans only).
+// PLAIN: a flat detector, no polynomial and no short scan.
+template <bool PLAIN = false>
 __device__ __forceinline__ float weight_value(const WeightParams& p, float val, const float* __restrict__ bh, float gamma,
                                               float cs, float den, float beta) {
-    if (p.n_bh > 0) {
+    if (!PLAIN && p.n_bh > 0) {
         float acc = 0.0f, pw = val;
         for (int t = 0; t < p.n_bh; ++t) {
             acc += bh[t] * pw;
@@ -73,9 +76,9 @@ __device__ __forceinline__ float weight_value(const WeightParams& p, float val, 
         val = acc;
     }
     const float sdd = p.sdd;
-    if (p.curved) val = val * sdd * cs * sdd / den;
+    if (!PLAIN && p.curved) val = val * sdd * cs * sdd / den;
     else val = (val * sdd * sdd) / den;
-    if (p.short_scan) val *= parker(p, beta, gamma);
+    if (!PLAIN && p.short_scan) val *= parker(p, beta, gamma);
     return val;
 }
 
