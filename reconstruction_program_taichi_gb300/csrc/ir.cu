@@ -455,9 +455,8 @@ template <typename T>
 __global__ void tv_weights_kernel(int nx, int nz, float beta, const T* __restrict__ x, float* __restrict__ wr) {
     const int64_t n = (int64_t)nz * nx * nx;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        const int ix = (int)(i % nx);
-        const int iy = (int)((i / nx) % nx);
-        const int iz = (int)(i / ((int64_t)nx * nx));
+        int ix, iy;
+        const int iz = (int)split_index(split_index(i, nx, ix), nx, iy);
         Grad g = grad_at(x, nx, nz, iz, iy, ix);
         wr[i] = 1.0f / sqrtf(g.gy * g.gy + g.gx * g.gx + g.gz * g.gz + beta);
     }
@@ -472,8 +471,8 @@ __global__ void admm_shrink_kernel(int nx, int nz, const float* __restrict__ x, 
                                    float* __restrict__ px) {
     const int64_t n = (int64_t)nz * nx * nx;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        const int ix = (int)(i % nx);
-        const int iy = (int)((i / nx) % nx);
+        int ix, iy;
+        split_index(split_index(i, nx, ix), nx, iy);
         const float c = x[i];
         const float dy = iy < nx - 1 ? x[i + nx] - c : 0.0f;
         const float dx = ix < nx - 1 ? x[i + 1] - c : 0.0f;
@@ -496,8 +495,8 @@ __global__ void admm_rhs_kernel(int nx, int nz, const float* __restrict__ bpb, c
                                 const float* __restrict__ px, float rho, float* __restrict__ out) {
     const int64_t n = (int64_t)nz * nx * nx;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        const int ix = (int)(i % nx);
-        const int iy = (int)((i / nx) % nx);
+        int ix, iy;
+        split_index(split_index(i, nx, ix), nx, iy);
         const bool iny = iy >= 1 && iy <= nx - 2, inx = ix >= 1 && ix <= nx - 2;
         const float tvy = iny ? vy[i - nx] - vy[i] : 0.0f, tvx = inx ? vx[i - 1] - vx[i] : 0.0f;
         const float tpy = iny ? py[i - nx] - py[i] : 0.0f, tpx = inx ? px[i - 1] - px[i] : 0.0f;
@@ -515,12 +514,10 @@ __global__ void __launch_bounds__(256)
 dtwd_kernel(int nx, int nz, const T* __restrict__ x, const float* __restrict__ wr, float s,
             const T* out_in, float a, T* out, double* __restrict__ partials) {
     const int64_t n = (int64_t)nz * nx * nx;
-    const int64_t plane = (int64_t)nx * nx;
     double dsum = 0.0;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        const int ix = (int)(i % nx);
-        const int iy = (int)((i / nx) % nx);
-        const int iz = (int)(i / plane);
+        int ix, iy;
+        const int iz = (int)split_index(split_index(i, nx, ix), nx, iy);
         const float c = ldv(x, i);
         const float r = dtwd_at(x, wr, nx, nz, i, iz, iy, ix);
         float v = s * r;
@@ -576,9 +573,8 @@ tv_partial_kernel(int nx, int nz, float beta, const float* __restrict__ x, doubl
     const int64_t n = (int64_t)nz * nx * nx;
     double s = 0.0;
     for (int64_t i = blockIdx.x * (int64_t)RED_THREADS + threadIdx.x; i < n; i += (int64_t)gridDim.x * RED_THREADS) {
-        const int ix = (int)(i % nx);
-        const int iy = (int)((i / nx) % nx);
-        const int iz = (int)(i / ((int64_t)nx * nx));
+        int ix, iy;
+        const int iz = (int)split_index(split_index(i, nx, ix), nx, iy);
         Grad g = grad_at(x, nx, nz, iz, iy, ix);
         s += sqrt((double)g.gy * g.gy + (double)g.gx * g.gx + (double)g.gz * g.gz + (double)beta);
     }
