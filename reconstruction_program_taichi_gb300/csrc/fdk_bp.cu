@@ -33,16 +33,16 @@ namespace {
 constexpr int BP_TX = 8, BP_TY = 8, BP_ZC = 16, BP_VCHUNK = 256;
 constexpr int BP_WX = 4;  // columns along x per warp (32 / BP_WX along y)
 static_assert(BP_TX % BP_WX == 0 && BP_TY % (32 / BP_WX) == 0, "warps tile the block");
-static_assert(BP_ZC % 2 == 0, "the 16-bit axial loop takes slices in pairs");
 // Minimum resident blocks per SM, i.e. a register budget of 65536 / (64 * minb) per
 // thread.  The axial kernel needs enough registers to issue all BP_ZC stencil gathers
 // of a view before their arithmetic (that hides the gather latency): measured at
 // 512x512x256 / 1080 views, float32 stencils run fastest with 128 registers (8
 // blocks), bf16 stencils with 80 (12 blocks); 16-bit stencils of a curved detector spill
 // there (512x512x128 / 360 views, FDK: 15.9 ms with 12 blocks, 8.4 with 8).  The general
-// modes use 8.
-template <int MODE, typename QT, bool CURVED>
+// modes use 8, columns of 8 slices 10 (12 with 16-bit stencils).
+template <int MODE, typename QT, bool CURVED, int ZC>
 constexpr int bp_min_blocks() {
+    if (ZC == 8 && (sizeof(QT) == 16 || CURVED)) return 10;
     return (MODE == 0 || MODE == 2) && sizeof(QT) == 8 && !CURVED ? 12 : 8;
 }
 
@@ -95,8 +95,8 @@ __device__ __forceinline__ float2 reciprocal2(float2 x) {
     return __ffma2_rn(r, __ffma2_rn(make_float2(-x.x, -x.y), r, make_float2(1.0f, 1.0f)), r);
 }
 
-template <int MODE, bool CONE, typename QT, typename PT, bool CURVED = false>
-__global__ void __launch_bounds__(BP_TX* BP_TY, bp_min_blocks<MODE, QT, CURVED>())
+template <int MODE, bool CONE, typename QT, typename PT, bool CURVED = false, int ZC = BP_ZC>
+__global__ void __launch_bounds__(BP_TX* BP_TY, bp_min_blocks<MODE, QT, CURVED, ZC>())
 fdk_bp_kernel(BpParams p, const float* __restrict__ angles, const float* __restrict__ pmat,
               const void* __restrict__ packed, float* __restrict__ vol, const uint32_t* __restrict__ f16_max) {
     // views per chunk of the shared tables; with projection matrices the chunk's 3x4
@@ -113,7 +113,7 @@ fdk_bp_kernel(BpParams p, const float* __restrict__ angles, const float* __restr
     const int warp = tid >> 5, lane = tid & 31;
     const int ix = blockIdx.x * BP_TX + (warp % (BP_TX / BP_WX)) * BP_WX + (lane % BP_WX);
     const int iy = blockIdx.y * BP_TY + (warp / (BP_TX / BP_WX)) * (32 / BP_WX) + lane / BP_WX;
-    const int zb = blockIdx.z * BP_ZC;
+    const int zb = blockIdx.z * ZC;
     const bool active = ix < p.nx && iy < p.ncb;
     const int nq = p.nu - 1;  // packed columns; packed rows per view: nv (cone: row nv-1 is NaN)
 
@@ -122,9 +122,9 @@ fdk_bp_kernel(BpParams p, const float* __restrict__ angles, const float* __restr
     const float c0y = p.o_y + ix * p.px_y + iy * p.py_y + zb * p.pz_y;
     const float c0z = p.o_z + ix * p.px_z + iy * p.py_z + zb * p.pz_z;
 
-    float acc[BP_ZC];
+    float acc[ZC];
 #pragma unroll
-    for (int k = 0; k < BP_ZC; ++k) acc[k] = 0.0f;
+    for (int k = 0; k < ZC; ++k) acc[k] = 0.0f;
     uint32_t dead = 0;  // bit k: slice zb+k projected off the detector in some view
 
     // float16 operands hold values scaled by 2^e: fold 2^-e (exact) into the view weight
@@ -149,7 +149,7 @@ fdk_bp_kernel(BpParams p, const float* __restrict__ angles, const float* __restr
             // views.  512x512x256 / 1080 views, FDK: float32 53.7 -> 49.2 ms; 256^3 / 360
             // views coronal, bf16: 4.55 -> 4.08 ms; 333x333x101 / 500 views, curved 6.42 ->
             // 5.30 ms (bit-identical).  L1 wavefronts bind now (82 % for float32).
-            static_assert(CONE, "cone-beam modes");
+            static_assert(CONE && ZC % 2 == 0, "cone-beam modes, slices in pairs");
             struct View {
                 const char* base;  // the view's cell (row 0, column floor(u))
                 float ru, w, vA, vB;  // column fraction, weight; row of slice k = vA + k vB
@@ -187,8 +187,8 @@ fdk_bp_kernel(BpParams p, const float* __restrict__ angles, const float* __restr
                 const int q1 = min(q0 + kViewRun, nvc);
                 for (int q = q0; q < q1; ++q) {
                     const float2 ru2 = make_float2(cur.ru, cur.ru);
-                    float2 lo[BP_ZC], hi[BP_ZC];
-                    float rv[BP_ZC];
+                    float2 lo[ZC], hi[ZC];
+                    float rv[ZC];
                     auto load = [&](int k, unsigned row) {
                         Quad<QT>::load(reinterpret_cast<const QT*>(cur.base + (uint64_t)min(row, nan_row) * stride), lo[k],
                                        hi[k]);
@@ -202,7 +202,7 @@ fdk_bp_kernel(BpParams p, const float* __restrict__ angles, const float* __restr
                     const unsigned MB = 0x4B400000u;  // M's bits
                     if constexpr (MODE == 2) {
 #pragma unroll
-                        for (int k = 0; k < BP_ZC; ++k) {
+                        for (int k = 0; k < ZC; ++k) {
                             const float vi = fmaf((float)k, cur.vB, cur.vA);
                             const float vf = floorf(vi);
                             rv[k] = vi - vf;
@@ -211,7 +211,7 @@ fdk_bp_kernel(BpParams p, const float* __restrict__ angles, const float* __restr
                     } else if constexpr (sizeof(QT) == 16) {
                         const float2 vA2 = make_float2(cur.vA, cur.vA), vB2 = make_float2(cur.vB, cur.vB);
 #pragma unroll
-                        for (int k = 0; k < BP_ZC; k += 2) {
+                        for (int k = 0; k < ZC; k += 2) {
                             const float2 vi = __ffma2_rn(make_float2((float)k, (float)(k + 1)), vB2, vA2);
                             const float2 m = __fadd2_rd(vi, make_float2(M, M));
                             const float2 fl = __fadd2_rn(m, make_float2(-M, -M));
@@ -223,7 +223,7 @@ fdk_bp_kernel(BpParams p, const float* __restrict__ angles, const float* __restr
                         }
                     } else {
 #pragma unroll
-                        for (int k = 0; k < BP_ZC; ++k) {
+                        for (int k = 0; k < ZC; ++k) {
                             const float vi = fmaf((float)k, cur.vB, cur.vA);
                             const float m = __fadd_rd(vi, M);
                             rv[k] = vi - (m - M);
@@ -233,7 +233,7 @@ fdk_bp_kernel(BpParams p, const float* __restrict__ angles, const float* __restr
                     const View next = geometry(min(q + 1, nvc - 1));
                     const float w = cur.w;
 #pragma unroll
-                    for (int k = 0; k < BP_ZC; ++k) {
+                    for (int k = 0; k < ZC; ++k) {
                         const float2 s2 = __ffma2_rn(ru2, hi[k], lo[k]);
                         acc[k] = fmaf(w, fmaf(rv[k], s2.y, s2.x), acc[k]);
                     }
@@ -268,7 +268,7 @@ fdk_bp_kernel(BpParams p, const float* __restrict__ angles, const float* __restr
                 const float w = (p.sid * dw) * tb.z;
                 const unsigned nan_row = (unsigned)(p.nv - 1);  // rows outside [0, nv-2] read the NaN row
                 const QT* view = reinterpret_cast<const QT*>(packed) + (int64_t)j * p.nv * nq;
-                const float tiny = 0x1p-26f / (float)BP_ZC;
+                const float tiny = 0x1p-26f / (float)ZC;
                 if (fabsf(Bu) <= tiny * fabsf(Au) && fabsf(Bw) <= tiny * fabsf(Aw)) {
                     const float mag = 1.0f / Aw;
                     const float ui = Au * mag;
@@ -281,7 +281,7 @@ fdk_bp_kernel(BpParams p, const float* __restrict__ angles, const float* __restr
                     const QT* base = view + (int)uf;
                     const float2 ru2 = make_float2(ru, ru);
 #pragma unroll
-                    for (int k = 0; k < BP_ZC; ++k) {
+                    for (int k = 0; k < ZC; ++k) {
                         const float vi = fmaf((float)k, Bv, Av) * mag;  // as in the per-slice branch
                         const float vf = floorf(vi);
                         const unsigned vr = min((unsigned)(int)vf, nan_row);
@@ -293,7 +293,7 @@ fdk_bp_kernel(BpParams p, const float* __restrict__ angles, const float* __restr
                     }
                 } else {
 #pragma unroll
-                    for (int k = 0; k < BP_ZC; ++k) {
+                    for (int k = 0; k < ZC; ++k) {
                         if ((dead >> k) & 1u) continue;
                         const float fk = (float)k;
                         const float mag = 1.0f / fmaf(fk, Bw, Aw);
@@ -322,7 +322,7 @@ fdk_bp_kernel(BpParams p, const float* __restrict__ angles, const float* __restr
                 const float L0 = p.sid - c0x * cb - c0y * sb, dL = -(p.pz_x * cb + p.pz_y * sb);
                 const float t0 = -c0x * sb + c0y * cb, dt = -p.pz_x * sb + p.pz_y * cb;
 #pragma unroll
-                for (int k = 0; k < BP_ZC; ++k) {
+                for (int k = 0; k < ZC; ++k) {
                     if (zb + k >= p.nsl || (dead >> k) & 1u) continue;
                     const float L = fmaf((float)k, dL, L0);
                     const float t = fmaf((float)k, dt, t0);
@@ -348,7 +348,7 @@ fdk_bp_kernel(BpParams p, const float* __restrict__ angles, const float* __restr
     if (!active) return;
     float* out = vol + (int64_t)zb * p.ss + (int64_t)iy * p.sb + ix;
 #pragma unroll
-    for (int k = 0; k < BP_ZC; ++k) {
+    for (int k = 0; k < ZC; ++k) {
         if (zb + k < p.nsl) {
             const bool off_detector = ((dead >> k) & 1u) || acc[k] != acc[k];
             if (p.accumulate)  // a voxel off the detector in any chunk stays NaN until mct_fdk_bp_finish
@@ -562,15 +562,15 @@ void launch_bp_fan(const BpParams& p, const mct_geom* g, cudaStream_t s, const f
         fdk_bp_fan_kernel<ZC, CURVED, float2><<<grid, block, 0, s>>>(p, angles, packed, vol, nullptr);
 }
 
-template <int MODE, bool CONE, bool CURVED = false>
+template <int MODE, bool CONE, bool CURVED = false, int ZC = BP_ZC>
 void launch_bp(const BpParams& p, dim3 grid, dim3 block, cudaStream_t s, const float* angles, const float* pmat,
                const void* packed, int dtype, float* vol, const uint32_t* f16_max) {
     if (dtype == MCT_BF16)
-        fdk_bp_kernel<MODE, CONE, uint2, uint32_t, CURVED><<<grid, block, 0, s>>>(p, angles, pmat, packed, vol, nullptr);
+        fdk_bp_kernel<MODE, CONE, uint2, uint32_t, CURVED, ZC><<<grid, block, 0, s>>>(p, angles, pmat, packed, vol, nullptr);
     else if (dtype == MCT_F16)
-        fdk_bp_kernel<MODE, CONE, h16x4, h16x2, CURVED><<<grid, block, 0, s>>>(p, angles, pmat, packed, vol, f16_max);
+        fdk_bp_kernel<MODE, CONE, h16x4, h16x2, CURVED, ZC><<<grid, block, 0, s>>>(p, angles, pmat, packed, vol, f16_max);
     else
-        fdk_bp_kernel<MODE, CONE, float4, float2, CURVED><<<grid, block, 0, s>>>(p, angles, pmat, packed, vol, nullptr);
+        fdk_bp_kernel<MODE, CONE, float4, float2, CURVED, ZC><<<grid, block, 0, s>>>(p, angles, pmat, packed, vol, nullptr);
 }
 
 }  // namespace
@@ -644,6 +644,17 @@ extern "C" int mct_fdk_bp(const mct_geom* g, const mct_tables* t, const void* pa
     p.ss = permuted ? g->nx : plane;
     dim3 block(BP_TX, BP_TY);
     dim3 grid((g->nx + BP_TX - 1) / BP_TX, (p.ncb + BP_TY - 1) / BP_TY, (p.nsl + BP_ZC - 1) / BP_ZC);
+    // Columns of 8 slices where 16 leave the SMs short of warps or too many of the last
+    // slices empty; otherwise their geometry, which 8 slices pay as often as 16, costs 8 to 12 %.
+    // FDK with columns of 16 / 8: 96x96x64, 180 views 125 / 110 us (576 blocks of 16 slices),
+    // bf16 157 / 122; 112x112x64 (784 blocks) 144 / 167, bf16 170 / 174; 64^3 113 / 92;
+    // 256x256, 360 views: 24 slices 528 / 480, 40 823 / 776 (bf16 842 / 757, curved 850 / 860),
+    // 56 1082 / 1056, 72 1323 / 1323; 512x512x8, 360 views 966 / 546.
+    const int64_t pad16 = (p.nsl + 15) / 16 * 16, pad8 = (p.nsl + 7) / 8 * 8;
+    const bool few = (int64_t)grid.x * grid.y * grid.z <= 152 * 4;
+    const bool slices8 = cone && !pm && g->nv <= (1 << 22) && (few || (p.curved ? pad16 * 4 > pad8 * 5 : pad16 * 8 > pad8 * 9)) &&
+                         (p.nsl + 7) / 8 <= 65535;
+    if (slices8) grid.z = (unsigned)((p.nsl + 7) / 8);
     MCT_REQUIRE(grid.y <= 65535 && grid.z <= 65535, "mct_fdk_bp: volume too large for the launch grid");
     cudaStream_t s = as_stream(stream);
     const uint32_t* fm = dtype == MCT_F16 ? f16_trailer(g, packed) : nullptr;
@@ -652,6 +663,9 @@ extern "C" int mct_fdk_bp(const mct_geom* g, const mct_tables* t, const void* pa
         launch_bp<2, true, true>(p, grid, block, s, t->angles, nullptr, packed, dtype, vol, fm);
     else if (cone && g->nv > (1 << 22))
         launch_bp<2, true>(p, grid, block, s, t->angles, nullptr, packed, dtype, vol, fm);
+    else if (slices8 && p.curved)
+        launch_bp<0, true, true, 8>(p, grid, block, s, t->angles, nullptr, packed, dtype, vol, fm);
+    else if (slices8) launch_bp<0, true, false, 8>(p, grid, block, s, t->angles, nullptr, packed, dtype, vol, fm);
     else if (cone && p.curved) launch_bp<0, true, true>(p, grid, block, s, t->angles, nullptr, packed, dtype, vol, fm);
     else if (cone) launch_bp<0, true>(p, grid, block, s, t->angles, nullptr, packed, dtype, vol, fm);
     else if (g->view_mode == 1 && g->nu <= (1 << 22)) {  // column indices exact in the float floor

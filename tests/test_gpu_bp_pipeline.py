@@ -111,3 +111,29 @@ def test_backprojection_at_the_edges_of_blocks_and_view_tables(n, nz, views, kw,
     both = (got != 0) & (ref != 0)
     assert both.sum() > 0.2 * both.size
     assert rel_l2(got[both], ref[both]) < TOL["f32"]
+
+
+@pytest.mark.parametrize("n,nz,storage,kw", [
+    (16, 8, "f32", {}), (20, 16, "f32", {}), (20, 17, "bf16", {}), (20, 25, "f32", {"CurvedDetector": True}),
+    (33, 9, "f16", {"ReconViewMode": "sagittal"}), (200, 16, "f32", {}), (200, 24, "f32", {}), (200, 17, "f32", {"CurvedDetector": True})])
+def test_columns_of_8_and_of_16_slices_match_the_oracle(n, nz, storage, kw, cuda):
+    """Both sides of the rule that picks the slices of a column: few and many blocks, last
+    slices that fill 16 or half of them."""
+    import torch
+    from reconstruction_program_taichi_gb300 import geometry, ops
+    o = _cone_obj(n=n, nz=nz, nu=40, nv=2 * nz, views=5, PixelSize=24.0 / n, DetectorElementWidth=1.6, **kw)
+    dg = geometry.fbp_geometry(o)
+    g = dg.geom
+    f = np.random.default_rng(n + nz).normal(0, 1, (5, g.nv, g.nu)).astype(np.float32)
+    dtype = {"f32": ops.MCT_F32, "bf16": ops.MCT_BF16, "f16": ops.MCT_F16}[storage]
+    got = ops.fdk_bp(dg, ops.pack(dg, torch.from_numpy(f).cuda(), dtype), dtype).cpu().numpy()
+    u, v, ang = geometry.fbp_arrays(o)
+    ref = F.fdk_bp(f.transpose(1, 0, 2), ang, u, v, nx=o.img_dim, nz=o.img_dim_z, px=o.img_pix_size,
+                   pz=o.img_voxel_height, cx=o.img_center_x, cy=o.img_center_y, cz=o.img_center_z,
+                   sid=o.source_isocenter_dis, sdd=o.source_det_dis, dv=o.det_elem_height, img_rot=o.img_rot,
+                   total_scan_angle=o.total_scan_angle, short_scan=o.short_scan, cone_beam=True,
+                   curved=o.curved_dect, view_mode=o.recon_view_mode)
+    assert np.mean((got == 0) != (ref == 0)) < 1e-3
+    both = (got != 0) & (ref != 0)
+    assert both.sum() > 0.2 * both.size
+    assert rel_l2(got[both], ref[both]) < TOL[storage]
