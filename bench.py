@@ -306,7 +306,7 @@ def run_gpu(args, w):
                           gather=n_samples * (32 if fp_dtype == ops.MCT_F32 else 16),
                           what="copies of the volume (32 B per voxel, both orientations) read once, the "
                                "projection written once; gathers: one 32-byte (16-bit: 16-byte) cell per "
-                               "in-volume sample"),
+                               "in-volume sample (a ray loads a cell once for all its samples there)"),
         "fdk_bp_kernel": dict(ms=float(st[2]), compulsory=cells * bp_elem + nvox * 4,
                               gather=nvox * w["views"] * bp_elem,
                               what="packed operand (16 B float32 / 8 B 16-bit per detector cell) read once, the "
