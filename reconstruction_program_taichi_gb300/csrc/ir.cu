@@ -192,41 +192,44 @@ struct CgEpi {
 // 8-byte operands and for 16-byte ones without the CG epilogue (with slices in pairs,
 // 512x512x64 / 360 views float32 5.67 ms with 2 blocks of 128 registers, 5.44 ms with
 // 3 blocks, bit-identical), 2 for 16-byte operands with the epilogue.
-template <typename QT, bool EPI, bool PIPE>
+// Per block of 64 threads (TX = 8) four times as many, and 10 for columns of 8 slices.
+template <typename QT, bool EPI, bool PIPE, int TX, int ZC>
 constexpr int ua_min_blocks() {
-    return !PIPE && (sizeof(QT) == 8 || !EPI) ? 3 : 2;
+    return ZC == 8 ? 10 : (!PIPE && (sizeof(QT) == 8 || !EPI) ? 3 : 2) * (UB_TX / TX);
 }
-template <bool CONE, typename QT, typename PT, typename OT = float, bool EPI = false, bool PIPE = false>
-__global__ void __launch_bounds__(UB_TX* UB_TY, ua_min_blocks<QT, EPI, PIPE>())
+template <bool CONE, typename QT, typename PT, typename OT = float, bool EPI = false, bool PIPE = false, int TX = UB_TX,
+          int ZC = UA_ZC>
+__global__ void __launch_bounds__(TX* UB_TY, ua_min_blocks<QT, EPI, PIPE, TX, ZC>())
 bp_unmatched_axial_kernel(UbParams p, const float* __restrict__ angles, const float* __restrict__ czv, float cz_const,
                           const void* __restrict__ packed, OT* __restrict__ vol,
                           const uint32_t* __restrict__ f16_max, CgEpi epi = CgEpi{}) {
     const int nq = p.nu - 1;  // packed: nv rows of nu-1 coefficient sets per view
-    __shared__ float4 tab[UB_VCHUNK];  // {cos b, sin b, cz_j, sid*cos b}
-    __shared__ float tab_s[UB_VCHUNK];  // sid*sin b
-    // a warp is 4 columns along x x 8 along y of the block's 32 x 8 (a view's gathers
+    constexpr int VCH = TX == 8 ? UB_VCHUNK / 2 : UB_VCHUNK;
+    __shared__ float4 tab[VCH];  // {cos b, sin b, cz_j, sid*cos b}
+    __shared__ float tab_s[VCH];  // sid*sin b
+    // a warp is 4 columns along x x 8 along y of the block's TX x 8 (a view's gathers
     // then span fewer detector columns; 512x512x64 / 360 views: float32 6.01 -> 5.79 ms,
     // bf16 5.94 -> 5.91)
     constexpr int WX = 4;
-    const int tid = threadIdx.y * UB_TX + threadIdx.x;
+    const int tid = threadIdx.y * TX + threadIdx.x;
     const int wq = tid >> 5, lq = tid & 31;
-    const int ix = blockIdx.x * UB_TX + (wq % (UB_TX / WX)) * WX + (lq % WX);
-    const int iy = blockIdx.y * UB_TY + (wq / (UB_TX / WX)) * (32 / WX) + lq / WX;
-    const int zb = blockIdx.z * UA_ZC;
+    const int ix = blockIdx.x * TX + (wq % (TX / WX)) * WX + (lq % WX);
+    const int iy = blockIdx.y * UB_TY + (wq / (TX / WX)) * (32 / WX) + lq / WX;
+    const int zb = blockIdx.z * ZC;
     const bool active = ix < p.nx && iy < p.nx;
     // same expressions as the general kernel with the axial mode's zero z-terms
     const float x = p.o_x + ix * p.ex_x + iy * p.ey_x + zb * p.ez_x;
     const float y = p.o_y + ix * p.ex_y + iy * p.ey_y + zb * p.ez_y;
     const float bz = p.z0 + ix * p.zx + iy * p.zy + zb * p.zz;
-    float acc[UA_ZC];
+    float acc[ZC];
 #pragma unroll
-    for (int k = 0; k < UA_ZC; ++k) acc[k] = 0.0f;
+    for (int k = 0; k < ZC; ++k) acc[k] = 0.0f;
     bool trunc = false;
 
-    for (int jc = 0; jc < p.views; jc += UB_VCHUNK) {
-        const int nvc = min(UB_VCHUNK, p.views - jc);
+    for (int jc = 0; jc < p.views; jc += VCH) {
+        const int nvc = min(VCH, p.views - jc);
         __syncthreads();
-        for (int q = tid; q < nvc; q += UB_TX * UB_TY) {
+        for (int q = tid; q < nvc; q += TX * UB_TY) {
             float s, c;
             sincosf(angles[jc + q] - p.img_rot, &s, &c);
             tab[q] = make_float4(c, s, czv ? czv[jc + q] : cz_const, p.sid * c);
@@ -282,15 +285,15 @@ bp_unmatched_axial_kernel(UbParams p, const float* __restrict__ angles, const fl
                     const float2 vA2 = make_float2(cur.vA, cur.vA), vB2 = make_float2(cur.vB, cur.vB);
                     const float M = 12582912.0f;
                     const unsigned MB = 0x4B400000u;  // M's bits
-                    float2 lo[UA_ZC], hi[UA_ZC];
-                    float rv[UA_ZC];
-                    unsigned row[UA_ZC];
+                    float2 lo[ZC], hi[ZC];
+                    float rv[ZC];
+                    unsigned row[ZC];
                     auto load = [&](int k, unsigned r) {
                         row[k] = r;
                         Quad<QT>::load(reinterpret_cast<const QT*>(cur.base + (uint64_t)min(r, top) * stride), lo[k], hi[k]);
                     };
 #pragma unroll
-                    for (int k = 0; k < UA_ZC; k += 2) {
+                    for (int k = 0; k < ZC; k += 2) {
                         const float2 vi = __ffma2_rn(make_float2((float)k, (float)(k + 1)), vB2, vA2);
                         const float2 m = __fadd2_rd(vi, make_float2(M, M));
                         const float2 fl = __fadd2_rn(m, make_float2(-M, -M));
@@ -304,7 +307,7 @@ bp_unmatched_axial_kernel(UbParams p, const float* __restrict__ angles, const fl
                     const float2 zA2 = make_float2(cur.zA, cur.zA), r22 = make_float2(cur.r2, cur.r2);
                     const float2 wpx2 = make_float2(cur.wpx, cur.wpx);
 #pragma unroll
-                    for (int k = 0; k < UA_ZC; k += 2) {
+                    for (int k = 0; k < ZC; k += 2) {
                         const float2 kk = make_float2((float)k, (float)(k + 1));
                         const float2 s0 = __ffma2_rn(ru2, hi[k], lo[k]), s1 = __ffma2_rn(ru2, hi[k + 1], lo[k + 1]);
                         const float2 z = __ffma2_rn(kk, zz2, zA2);
@@ -356,9 +359,9 @@ bp_unmatched_axial_kernel(UbParams p, const float* __restrict__ angles, const fl
                 const float2 vA2 = make_float2(vA, vA), vB2 = make_float2(vB, vB);
                 const float2 zA2 = make_float2(zA, zA), zz2 = make_float2(p.zz, p.zz);
                 const float2 r22 = make_float2(r2, r2), wpx2 = make_float2(wpx, wpx);
-                static_assert(UA_ZC % 2 == 0, "slices are taken in pairs");
+                static_assert(ZC % 2 == 0, "slices are taken in pairs");
 #pragma unroll
-                for (int k = 0; k < UA_ZC; k += 2) {
+                for (int k = 0; k < ZC; k += 2) {
                     const float2 kk = make_float2((float)k, (float)(k + 1));
                     const float2 vi = __ffma2_rn(kk, vB2, vA2);
                     const float vf0 = floorf(vi.x), vf1 = floorf(vi.y);
@@ -378,7 +381,7 @@ bp_unmatched_axial_kernel(UbParams p, const float* __restrict__ angles, const fl
             } else {
                 const PT* base = reinterpret_cast<const PT*>(packed) + ((int64_t)j * p.nv + zb) * nq + uc;
 #pragma unroll
-                for (int k = 0; k < UA_ZC; ++k) {
+                for (int k = 0; k < ZC; ++k) {
                     if (zb + k < p.nz) {
                         const float z = fmaf((float)k, p.zz, bz) + tb.z;
                         const float2 pr = Pair<PT>::load(base + k * nq);
@@ -402,10 +405,10 @@ bp_unmatched_axial_kernel(UbParams p, const float* __restrict__ angles, const fl
         double dsum = 0.0;
         if (active) {
 #pragma unroll
-            for (int k = 0; k < UA_ZC; ++k)
+            for (int k = 0; k < ZC; ++k)
                 if (zb + k < p.nz) stv(vol, (zb + k) * plane + (int64_t)iy * p.nx + ix, trunc ? 0.0f : acc[k] * unscale);
 #pragma unroll 1
-            for (int k = 0; k < UA_ZC && zb + k < p.nz; ++k) {
+            for (int k = 0; k < ZC && zb + k < p.nz; ++k) {
                 const int64_t i = (zb + k) * plane + (int64_t)iy * p.nx + ix;
                 float v = ldv(vol, i);  // this thread's own store
                 if (epi.w1) v = __fadd_rn(__fmul_rn(epi.s1, dtwd_at(d, epi.w1, p.nx, p.nz, i, zb + k, iy, ix)), v);
@@ -415,7 +418,7 @@ bp_unmatched_axial_kernel(UbParams p, const float* __restrict__ angles, const fl
             }
         }
         // block sum over the 256 threads, then one partial per block
-        __shared__ double red[UB_TX * UB_TY / 32];
+        __shared__ double red[TX * UB_TY / 32];
         const int lane = tid & 31, w = tid >> 5;
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) dsum += __shfl_down_sync(0xffffffffu, dsum, o);
@@ -424,14 +427,14 @@ bp_unmatched_axial_kernel(UbParams p, const float* __restrict__ angles, const fl
         if (tid == 0) {
             double t = 0.0;
 #pragma unroll
-            for (int q = 0; q < UB_TX * UB_TY / 32; ++q) t += red[q];
+            for (int q = 0; q < TX * UB_TY / 32; ++q) t += red[q];
             epi.partials[((int64_t)blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x] = t;
         }
         return;
     }
     if (!active) return;
 #pragma unroll
-    for (int k = 0; k < UA_ZC; ++k)
+    for (int k = 0; k < ZC; ++k)
         if (zb + k < p.nz) stv(vol, (zb + k) * plane + (int64_t)iy * p.nx + ix, trunc ? 0.0f : acc[k] * unscale);
 }
 
@@ -628,13 +631,33 @@ inline int ew_grid(int64_t n) {
 using namespace mct;
 
 // The axial cone-beam kernel with output OT, with or without the CG epilogue.
+template <typename OT, bool EPI, bool PIPE, typename QT, typename PT, int TX, int ZC>
+void launch_axial_shape(const mct_geom* g, const UbParams& p, const mct_tables* t, const void* packed, OT* out,
+                        const uint32_t* f16_max, const CgEpi& e, cudaStream_t s) {
+    dim3 block(TX, UB_TY);
+    dim3 grid((g->nx + TX - 1) / TX, (g->nx + UB_TY - 1) / UB_TY, (g->nz + ZC - 1) / ZC);
+    bp_unmatched_axial_kernel<true, QT, PT, OT, EPI, PIPE, TX, ZC><<<grid, block, 0, s>>>(p, t->angles, t->cz, g->cz,
+                                                                                          packed, out, f16_max, e);
+}
+// Blocks of two warps, as in the FDK kernel, except with the epilogue, whose partial sums are
+// one per 32 x 8 columns; columns of 8 slices by the FDK kernel's rule.  CGLS of 3 iterations,
+// ms, blocks of 8 warps / 2 warps / 2 warps with 8 slices: 128x128x48, 120 views 1.958 / 1.836
+// / 1.893; 64^3, 120 views 1.103 / 1.064 / 0.901; 96x96x64 1.547 / 1.551 / 1.484; 112x112x64
+// 2.029 / 1.914 / 1.969; 200x200, 180 views: 24 slices 3.622 / 3.342 / 2.963, 56 6.650 / 6.460
+// / 6.210; 256x256x64, 180 views, with a TV reweighting 21.17 / 21.11 / 21.37.
 template <typename OT, bool EPI, bool PIPE, typename QT, typename PT>
 void launch_axial_q(const mct_geom* g, const UbParams& p, const mct_tables* t, const void* packed, OT* out,
                     const uint32_t* f16_max, const CgEpi& e, cudaStream_t s) {
-    dim3 block(UB_TX, UB_TY);
-    dim3 grid((g->nx + UB_TX - 1) / UB_TX, (g->nx + UB_TY - 1) / UB_TY, (g->nz + UA_ZC - 1) / UA_ZC);
-    bp_unmatched_axial_kernel<true, QT, PT, OT, EPI, PIPE><<<grid, block, 0, s>>>(p, t->angles, t->cz, g->cz, packed, out,
-                                                                                  f16_max, e);
+    if constexpr (!EPI && PIPE) {
+        const int64_t pad16 = (g->nz + 15) / 16 * 16, pad8 = (g->nz + 7) / 8 * 8;
+        const int64_t columns = (int64_t)((g->nx + 7) / 8) * ((g->nx + 7) / 8);
+        if ((columns * (pad16 / 16) <= 152 * 4 || pad16 * 8 > pad8 * 9) && pad8 / 8 <= 65535)
+            launch_axial_shape<OT, EPI, PIPE, QT, PT, 8, 8>(g, p, t, packed, out, f16_max, e, s);
+        else
+            launch_axial_shape<OT, EPI, PIPE, QT, PT, 8, 16>(g, p, t, packed, out, f16_max, e, s);
+    } else {
+        launch_axial_shape<OT, EPI, PIPE, QT, PT, UB_TX, UA_ZC>(g, p, t, packed, out, f16_max, e, s);
+    }
 }
 template <typename OT, bool EPI>
 void launch_axial(const mct_geom* g, const UbParams& p, const mct_tables* t, const void* packed, int dtype, OT* out,

@@ -137,3 +137,24 @@ def test_columns_of_8_and_of_16_slices_match_the_oracle(n, nz, storage, kw, cuda
     both = (got != 0) & (ref != 0)
     assert both.sum() > 0.2 * both.size
     assert rel_l2(got[both], ref[both]) < TOL[storage]
+
+
+@pytest.mark.parametrize("n,nz,views,storage", [
+    (7, 8, 255, "f32"), (9, 16, 257, "f32"), (20, 17, 40, "bf16"), (200, 16, 5, "f32"), (201, 17, 5, "f32"), (200, 30, 5, "f16")])
+def test_solver_backprojection_at_the_edges_of_its_blocks(n, nz, views, storage, cuda):
+    """Blocks of 8 x 8 columns, view tables of 256 entries, columns of 8 and of 16 slices."""
+    import torch
+    from reconstruction_program_taichi_gb300 import geometry, ops
+    o = _cone_obj(n=n, nz=nz, nu=60, nv=2 * nz, views=views, PixelSize=12.0 / n, DetectorElementWidth=1.0)
+    dg = geometry.ir_geometry(o)
+    sgm = np.random.default_rng(n + views).normal(0, 1, dg.sgm_shape).astype(np.float32)
+    dtype = {"f32": ops.MCT_F32, "bf16": ops.MCT_BF16, "f16": ops.MCT_F16}[storage]
+    got = ops.bp_unmatched_packed(dg, ops.pack_sinogram(dg, torch.from_numpy(sgm).cuda(), dtype), dtype).cpu().numpy()
+    ref = I.bp_unmatched(sgm, dg.host["angles"], dg.host["u"], dg.host["v"], o.array_img_center_z, nx=o.img_dim,
+                         nz=o.img_dim_z, px=o.img_pix_size, pz=o.img_voxel_height, cx=o.img_center_x, cy=o.img_center_y,
+                         sid=o.source_isocenter_dis, sdd=o.source_det_dis, dv=o.det_elem_height, img_rot=o.img_rot,
+                         cone_beam=True)
+    assert np.mean((got == 0) != (ref == 0)) < 1e-3
+    both = (got != 0) & (ref != 0)
+    assert both.sum() > 0.2 * both.size
+    assert rel_l2(got[both], ref[both]) < 5 * TOL[storage]  # a row at the edge in or out, as above
