@@ -1111,6 +1111,7 @@ int mct_fp_adjoint(const mct_geom* g, const mct_tables* t, const float* sgm, con
     MCT_TRY(make_params(g, p, "mct_fp_adjoint"));
     MCT_REQUIRE(t && t->angles && t->u && t->v && vol && sgm, "mct_fp_adjoint: NULL buffer");
     MCT_REQUIRE(!p.pmat || (t->pmat_a && t->pmat_xs), "mct_fp_adjoint: projection-matrix tables missing");
+    if (p.cone && g->nz < 2) return MCT_OK;  // no cell, so mct_fp sums nothing: its transpose adds nothing
     dim3 block(32, 8), grid((g->nu + 31) / 32, g->views, (g->nv + 7) / 8);
     auto go = p.cone ? fp_adjoint_kernel<true, false> : fp_adjoint_kernel<false, false>;
     go<<<grid, block, 0, as_stream(stream)>>>(p, t->angles, t->u, t->v, t->cz, t->pmat_a, t->pmat_xs, sgm, mask, vol);
@@ -1130,6 +1131,7 @@ int mct_fp_adjoint_cells(const mct_geom* g, const mct_tables* t, const float* sg
     MCT_REQUIRE(!p.pmat || (t->pmat_a && t->pmat_xs), "mct_fp_adjoint_cells: projection-matrix tables missing");
     MCT_REQUIRE(((uintptr_t)workspace & 15) == 0, "mct_fp_adjoint_cells: workspace must be 16-byte aligned");
     MCT_REQUIRE(g->nx <= 65535 * 8 && g->nz <= 65535, "mct_fp_adjoint_cells: at most 524280 x 524280 x 65535 voxels");
+    if (p.cone && g->nz < 2) return MCT_OK;  // as in mct_fp_adjoint
     cudaStream_t s = as_stream(stream);
     float* cells = static_cast<float*>(workspace);
     MCT_REQUIRE(cudaMemsetAsync(cells, 0, mct_fp_adjoint_workspace_size(g), s) == cudaSuccess,

@@ -114,6 +114,7 @@ MCT_HD void interior_range(const FpParams& p, const Ray& r, bool test_z, int& ki
     bool empty = false;
     auto axis = [&](float f0, float df, float n) {
         const float a = eps, b = n - 1.0f - eps;
+        if (!(a <= b)) empty = true;  // one plane: no cell (t1, t2 would span the plane's two sides)
         if (fabsf(df) < 1e-20f) {
             if (!(f0 >= a && f0 <= b)) empty = true;
             return;

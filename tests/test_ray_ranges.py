@@ -85,3 +85,12 @@ def check_inside(g, steps, terms):
 def test_every_sample_of_the_range_lies_in_a_cell(nx, nz, nu, nv, views, step, cone, host_lib):
     g, t = geom(nx, nz, nu, nv, views, step, cone)
     assert check_inside(g, *ranges(host_lib, g, t)).sum() > 0
+
+
+@pytest.mark.parametrize("nx,nu,nv,views,high,cz", [(256, 48, 32, 4, 8.0, 0.22), (32, 40, 33, 12, 4.0, 0.1), (3, 9, 9, 13, 6.0, 0.267)])
+def test_a_cone_beam_volume_of_one_slice_has_no_cells(nx, nu, nv, views, high, cz, host_lib):
+    """Its only plane lies on both z faces at once: no sample passes the inside test."""
+    g, t = geom(nx, 1, nu, nv, views, px=0.8, pz=0.4, high=high, cz=cz)
+    steps, terms = ranges(host_lib, g, t)
+    assert (steps[:, 0] <= steps[:, 1]).any()  # rays reach the plane
+    assert not (steps[:, 2] <= steps[:, 3]).any()
