@@ -249,7 +249,7 @@ fp_kernel(FpParams p, const float* __restrict__ angles, const float* __restrict_
             acc += ok ? v : 0.0f;
         };
         int kis, kie;
-        interior_range(p, r, CONE, kis, kie);
+        if (!interior_range(p, r, CONE, kis, kie)) acc = __int_as_float(0x7fffffff);  // its values have no weights
         if (p.K >= kMaxWalkSteps) {  // step indices would not be exact in float32
             kis = r.ke + 1;
             kie = r.ke;

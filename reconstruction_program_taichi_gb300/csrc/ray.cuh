@@ -107,12 +107,15 @@ MCT_HD bool setup_ray(const FpParams& p, int iu, int iv, int j, const float* __r
 
 // Steps [kis, kie] whose sample lies at least 1e-3 voxel inside the box on every
 // tested axis (and one more step in from both ends): for them the reference's inside
-// test certainly passes, far beyond float rounding, so it can be skipped.
-MCT_HD void interior_range(const FpParams& p, const Ray& r, bool test_z, int& kis, int& kie) {
+// test certainly passes, far beyond float rounding, so it can be skipped.  A ray with a term
+// that is no finite number (from an angle, a centre, a matrix) has no such steps, so no index
+// is taken from it; false is returned if the terms that are finite would leave it some.
+MCT_HD bool interior_range(const FpParams& p, const Ray& r, bool test_z, int& kis, int& kie) {
     const float eps = 1e-3f;
     float lo = -3.0e38f, hi = 3.0e38f;
-    bool empty = false;
+    bool empty = false, finite = true;
     auto axis = [&](float f0, float df, float n) {
+        finite = finite && fabsf(f0) <= 3.4e38f && fabsf(df) <= 3.4e38f;
         const float a = eps, b = n - 1.0f - eps;
         if (!(a <= b)) empty = true;  // one plane: no cell (t1, t2 would span the plane's two sides)
         if (fabsf(df) < 1e-20f) {
@@ -128,17 +131,18 @@ MCT_HD void interior_range(const FpParams& p, const Ray& r, bool test_z, int& ki
     if (test_z) axis(r.fz0, r.dfz, (float)p.nz);
     lo = fmaxf(lo, (float)r.ks - 2.0f);
     hi = fminf(hi, (float)r.ke + 2.0f);
-    if (empty || !(lo <= hi)) {
+    kis = 1;
+    kie = 0;
+    if (!empty && lo <= hi) {
+        kis = max(r.ks, (int)ceilf(lo) + 1);
+        kie = min(r.ke, (int)floorf(hi) - 1);
+    }
+    const bool lost = !finite && kis <= kie;
+    if (lost || kis > kie) {
         kis = r.ke + 1;
         kie = r.ke;
-        return;
     }
-    kis = max(r.ks, (int)ceilf(lo) + 1);
-    kie = min(r.ke, (int)floorf(hi) - 1);
-    if (kis > kie) {
-        kis = r.ke + 1;
-        kie = r.ke;
-    }
+    return !lost;
 }
 
 // Above this many steps a ray's indices are no longer exact in float32 (and would not

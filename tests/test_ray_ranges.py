@@ -94,3 +94,33 @@ def test_a_cone_beam_volume_of_one_slice_has_no_cells(nx, nu, nv, views, high, c
     steps, terms = ranges(host_lib, g, t)
     assert (steps[:, 0] <= steps[:, 1]).any()  # rays reach the plane
     assert not (steps[:, 2] <= steps[:, 3]).any()
+
+
+@pytest.mark.parametrize("bad", [np.nan, np.inf, -np.inf])
+@pytest.mark.parametrize("table", ["angles", "cz", "u", "v", "pa", "pxs"])
+def test_a_ray_without_a_position_has_no_range(table, bad, host_lib):
+    """A table entry that is no finite number takes the ranges of its rays, and of no others."""
+    g, t = geom(32, 9, 16, 7, 8)
+    t["cz"] = np.linspace(-0.1, 0.1, 8)
+    if table in ("pa", "pxs"):  # matrices that put the rays where the circular scan has them
+        g.flags |= _lib.MCT_PMATRIX
+        m = np.zeros((8, 9))
+        for j, a in enumerate(t["angles"].astype(np.float64)):
+            for i, (w, eu, ev) in enumerate(((-550.0, 0.0, 0.0), (t["u"][0], g.du, 0.0), (t["v"][0], 0.0, g.dv))):
+                m[j, 3 * i:3 * i + 3] = eu, ev, w
+            c, s = np.cos(a), np.sin(a)
+            x, y = m[j, 0:3].copy(), m[j, 3:6].copy()
+            m[j, 0:3], m[j, 3:6] = c * x - s * y, s * x + c * y
+        t["pa"] = m
+        t["pxs"] = np.stack([300 * np.cos(t["angles"]), 300 * np.sin(t["angles"]), 0 * t["angles"]], 1)
+    good, terms = ranges(host_lib, g, t)
+    assert check_inside(g, good, terms).mean() > 0.3
+    a = t[table]
+    a[3 if a.ndim == 1 else (3, 0)] = bad
+    steps, _ = ranges(host_lib, g, t)
+    has = (steps[:, 2] <= steps[:, 3]).reshape(8, 7, 16)
+    hit = {"u": np.s_[:, :, 3], "v": np.s_[:, 3]}.get(table, np.s_[3])
+    rest = np.ones_like(has)
+    rest[hit] = False
+    assert not has[hit].any()
+    assert (steps.reshape(8, 7, 16, 4)[rest] == good.reshape(8, 7, 16, 4)[rest]).all()
