@@ -21,6 +21,7 @@
 #include <type_traits>
 
 #include "common.cuh"
+#include "fan.cuh"
 
 namespace mct {
 namespace {
@@ -439,18 +440,11 @@ fdk_bp_fan_kernel(BpParams p, const float* __restrict__ angles, const void* __re
     const float M = 12582912.0f;
     const unsigned MB = 0x4B400000u;  // M's bits
     const unsigned last = (unsigned)(p.nu - 2);
-    // A pixel at distance rho from the axis is seen at most asin(rho / sid) off the central
-    // ray: where that stays a column inside the detector for all the warp's pixels, no view
-    // needs the test or the clamp.
+    // the warp's pixels are inside the detector in every view: no test, no clamp
     bool in = true;
 #pragma unroll
-    for (int r = 0; r < R; ++r) {
-        const float rho2 = fmaxf(x2[r].x * x2[r].x + y2[r].x * y2[r].x, x2[r].y * x2[r].y + y2[r].y * y2[r].y);
-        const float c2 = p.sid * p.sid - rho2;
-        const float reach = CURVED ? p.sdd * asinf(sqrtf(rho2) / p.sid) : p.sdd * sqrtf(rho2 / c2);
-        const float i0 = (-reach - p.u0) * p.inv_ustep, i1 = (reach - p.u0) * p.inv_ustep;
-        in = in && c2 > 0.0f && fminf(i0, i1) >= 1.0f && fmaxf(i0, i1) <= (float)(p.nu - 3);
-    }
+    for (int r = 0; r < R; ++r)
+        in = in && fan_pair_inside<CURVED>(x2[r].x, y2[r].x, x2[r].y, y2[r].y, p.sid, p.sdd, p.u0, p.inv_ustep, p.nu);
     const bool inside = __all_sync(0xffffffffu, in);
     if (inside) {  // no index was recorded: any valid one
 #pragma unroll
@@ -458,13 +452,15 @@ fdk_bp_fan_kernel(BpParams p, const float* __restrict__ angles, const void* __re
     }
     for (int jc = 0; jc < p.views; jc += FB_VCHUNK) {
         const int nvc = min(FB_VCHUNK, p.views - jc);
+        bool angles_ok = true;  // an angle that is no finite number has NaN indices: its views are tested
         __syncthreads();
         for (int q = tid; q < nvc; q += 32 * FB_G) {
             const float4 e = view_entry(p, angles, jc + q, unscale);
             tab[q] = make_float4(e.x, e.x, e.y, e.y);
             tabw[q] = two(p.sid * e.z);
+            angles_ok = angles_ok && fabsf(e.x) <= 1.0f && fabsf(e.y) <= 1.0f;
         }
-        __syncthreads();
+        angles_ok = __syncthreads_and(angles_ok);
         if (!active) continue;
         auto views = [&](auto inside_tag) {
             constexpr bool kInside = decltype(inside_tag)::value;
@@ -512,7 +508,7 @@ fdk_bp_fan_kernel(BpParams p, const float* __restrict__ angles, const void* __re
                 }
             }
         };
-        if (inside) views(std::true_type{});
+        if (inside && angles_ok) views(std::true_type{});
         else views(std::false_type{});
     }
     const float umax = (float)(p.nu - 1);

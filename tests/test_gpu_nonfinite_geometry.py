@@ -68,3 +68,56 @@ def test_rays_without_a_position(table, cone, step, bad, cuda):
         # the same additions in another order: 24 views of at most about 10 per voxel
         assert rel_l2(out.cpu().numpy(), want.cpu().numpy()) < 1e-6
     assert ops.fp_count_samples(dg) == ops.fp_count_samples(good, mask=keep)
+
+
+def _fan(n, nz, views, curved=False, wide=2.0, **kw):
+    from reconstruction_program_taichi_gb300 import geometry
+    o = _cone_obj(n=n, nz=nz, nu=90, nv=nz, views=views, ConeBeam=False, CurvedDetector=curved,
+                  DetectorElementWidth=wide * n * 0.5 * 550 / 300 / 90, **kw)
+    return geometry.fbp_geometry(o)
+
+
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+@pytest.mark.parametrize("n,nz,views,curved,view", [(33, 1, 40, False, 7), (33, 1, 40, True, 39), (64, 1, 600, False, 0),
+                                                    (34, 9, 40, False, 7), (34, 3, 40, True, 20)])
+def test_a_fan_beam_view_without_an_angle_leaves_no_pixel(n, nz, views, curved, view, bad, cuda):
+    """It sees every pixel off the detector, so all are written as 0; in chunks too, where the
+    other chunks' pixels are inside the detector in each of their views."""
+    import torch
+    from reconstruction_program_taichi_gb300 import ops
+    dg = _fan(n, nz, views, curved)
+    f = torch.rand((views, nz, 90), device="cuda", generator=torch.Generator("cuda").manual_seed(1)) + 0.5
+    for dtype in (ops.MCT_F32, ops.MCT_BF16):
+        good = ops.fdk_bp(dg, ops.pack(dg, f, dtype), dtype)
+        assert (good != 0).float().mean() > 0.9
+    dg._keep["angles"][view] = bad
+    for dtype in (ops.MCT_F32, ops.MCT_BF16, ops.MCT_F16):
+        out, rest = _front(dg.vol_shape, 3.0)
+        ops.fdk_bp(dg, ops.pack(dg, f, dtype), dtype, out=out)
+        assert not out.any() and (rest == 3.0).all()
+    vol = torch.zeros(dg.vol_shape, device="cuda")
+    for b in range(0, views, 30):
+        c = ops.ViewChunk(dg, b, min(30, views - b), accumulate=True)
+        ops.fdk_bp(c, ops.pack(c, f[b:b + 30].contiguous()), out=vol)
+    assert not ops.fdk_bp_finish(dg, vol).any()
+
+
+@pytest.mark.parametrize("curved", [False, True])
+def test_fan_beam_of_a_far_source_drops_the_pixels_off_the_detector(curved, cuda):
+    """sid^2 is beyond float32; the rays are parallel, the magnification 2."""
+    import torch
+    from reconstruction_program_taichi_gb300 import ops
+    dg = _fan(64, 1, 40, curved, wide=0.5)
+    dg.geom.sid, dg.geom.sdd = 2e19, 4e19
+    g = dg.geom
+    f = torch.ones((40, 1, 90), device="cuda")
+    got = ops.fdk_bp(dg, ops.pack(dg, f)).cpu().numpy()[0]
+    i = np.arange(64)
+    x = (i[None, :] - 31.5) * g.px + g.cx
+    y = -(i[:, None] - 31.5) * g.px + g.cy
+    a = dg.host["angles"][:, None, None]
+    index = (2 * (y * np.cos(a) - x * np.sin(a)) - g.u0) / g.u_step
+    edge = np.minimum(np.abs(index), np.abs(index - 88)).min(0) < 1e-3
+    seen = ((index >= 0) & (index + 1 <= 89)).all(0)
+    assert 0.1 < seen.mean() < 0.9
+    assert not got[~seen & ~edge].any()
