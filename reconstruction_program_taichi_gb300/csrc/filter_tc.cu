@@ -445,9 +445,10 @@ tc_filter_kernel(TcDims d, int nv, int views, float du, Parts a, Parts b, float*
             at = ((int64_t)j * nv + r) * d.nu;
         }
         const uint32_t lanes = tmem + ((uint32_t)(warp * 32) << 16);
+        const int cols = min(BN, d.nu - nbk * BN);  // this tile's, at least 1
         if ((d.nu & 3) == 0) {
             // rows are 16-byte aligned: each lane stores its row
-            for (int c0 = 0; c0 < BN; c0 += 16) {
+            for (int c0 = 0; c0 < cols; c0 += 16) {
                 float v[16];
                 tmem_ld16(lanes + (uint32_t)c0, v);
                 const int n0 = nbk * BN + c0;
@@ -469,7 +470,7 @@ tc_filter_kernel(TcDims d, int nv, int views, float du, Parts a, Parts b, float*
             // columns at a time through this warp's part of the ring (its copies and
             // MMAs are done), so that a warp stores 32 consecutive floats of a row
             float* t = reinterpret_cast<float*>(smem) + warp * (32 * 33);
-            for (int c0 = 0; c0 < BN; c0 += 32) {
+            for (int c0 = 0; c0 < cols; c0 += 32) {
                 const int n = nbk * BN + c0 + lane;
 #pragma unroll
                 for (int h = 0; h < 32; h += 16) {
