@@ -238,14 +238,19 @@ __global__ void absmax_kernel(int nu, int nv, int views, int64_t rs, int64_t vs,
 // Row nv-1 is all NaN: the backprojector sends every off-detector row there, so an
 // off-detector voxel ends up NaN and is written as 0.
 //
-// The copy's writes bound it.  Blocks take tiles of PACK_COLS columns x PACK_ROWS rows of a
+// The copy's writes bound it.  Blocks take tiles of PACK_COLS columns x 16 rows of a
 // view and each thread PACK_RUN rows of a column, which it loads once each; element by
 // element, two 64-bit divisions per element took 78 % of the issue slots at small sizes
 // (float32, 180 views of 64 x 256: 22.8 us, 1080 of 256 x 1024: 1.08 ms; by tiles 13.7 us, 0.82
 // ms = 6.8 TB/s, the same bits).
-constexpr int PACK_COLS = 64, PACK_RUN = 4, PACK_ROWS = 256 / PACK_COLS * PACK_RUN;
+// Detectors of fewer than 13 rows take blocks of as many rows as they have.
+constexpr int PACK_COLS = 64, PACK_RUN = 4;
+inline int pack_threads(const mct_geom* g) {
+    return PACK_COLS * std::min((g->nv + PACK_RUN - 1) / PACK_RUN, 256 / PACK_COLS);
+}
 inline int64_t pack_tiles(const mct_geom* g) {
-    return (int64_t)g->views * ((g->nv + PACK_ROWS - 1) / PACK_ROWS) * ((g->nu - 1 + PACK_COLS - 1) / PACK_COLS);
+    const int rows = pack_threads(g) / PACK_COLS * PACK_RUN;
+    return (int64_t)g->views * ((g->nv + rows - 1) / rows) * ((g->nu - 1 + PACK_COLS - 1) / PACK_COLS);
 }
 template <typename QT>
 __global__ void __launch_bounds__(256)
@@ -253,12 +258,13 @@ pack_quad_kernel(int nu, int nv, int views, int64_t rs, int64_t vs, const float*
                  const uint32_t* __restrict__ maxbits) {
     const int nq = nu - 1;
     const float sc = IsF16<QT>::value ? ldexpf(1.0f, f16_scale_exp(*maxbits)) : 1.0f;
-    const int ct = (nq + PACK_COLS - 1) / PACK_COLS, rt = (nv + PACK_ROWS - 1) / PACK_ROWS;
+    const int rows = (int)blockDim.x / PACK_COLS * PACK_RUN;
+    const int ct = (nq + PACK_COLS - 1) / PACK_COLS, rt = (nv + rows - 1) / rows;
     for (int64_t t = blockIdx.x; t < (int64_t)views * rt * ct; t += gridDim.x) {
         int tc, tr;
         const int64_t j = split_index(split_index(t, ct, tc), rt, tr);
         const int c = tc * PACK_COLS + (int)(threadIdx.x % PACK_COLS);
-        const int r0 = tr * PACK_ROWS + (int)(threadIdx.x / PACK_COLS) * PACK_RUN;
+        const int r0 = tr * rows + (int)(threadIdx.x / PACK_COLS) * PACK_RUN;
         if (c >= nq || r0 >= nv) continue;
         const float* f = F + r0 * rs + j * vs + c;
         QT* q = Q + (j * nv + r0) * nq + c;
@@ -288,24 +294,69 @@ pack_quad_kernel(int nu, int nv, int views, int64_t rs, int64_t vs, const float*
 
 // fan: P[j][r][c] = {A', F(j,r,c+1) - A'} with A' = F(j,r,c) as stored, c < nu-1.  A block
 // takes a line at a time (element by element, the index divisions bound it: 140 slices of
-// 720 views x 1024 columns, float32, 0.32 ms, by lines 0.19 ms).
-constexpr int PAIR_THREADS = 128;
-template <typename PT>
+// 720 views x 1024 columns, float32, 0.32 ms, by lines 0.19 ms).  SHORT: lines of up to 128
+// elements, w lanes and PAIR_RUN lines per thread: a block for each of them costs more than
+// the divisions did (21476 lines of 70 elements: element by element 9.6 us, a line a block
+// 12.0 us, now 6.8 us; 10704 lines of 49: 4.4, 6.6, 3.4 us).
+constexpr int PAIR_THREADS = 128, PAIR_RUN = 4;
+inline int pair_lanes(int nq) {  // lanes per short line: a power of two, or a multiple of 32
+    int w = 4;
+    while (w < nq && w < 64) w *= 2;
+    return nq > 64 ? (nq + 31) / 32 * 32 : w;
+}
+template <typename PT, bool SHORT>
 __global__ void __launch_bounds__(PAIR_THREADS)
-pack_pair_kernel(int nu, int nv, int views, int64_t rs, int64_t vs, const float* __restrict__ F,
-                                 PT* __restrict__ P, const uint32_t* __restrict__ maxbits) {
+pack_pair_kernel(int nu, int nv, int views, int64_t rs, int64_t vs, const float* __restrict__ F, PT* __restrict__ P,
+                 const uint32_t* __restrict__ maxbits, int w) {
     const int nq = nu - 1;
     const float sc = IsF16<PT>::value ? ldexpf(1.0f, f16_scale_exp(*maxbits)) : 1.0f;
     const int64_t lines = (int64_t)views * nv;
-    for (int64_t l = blockIdx.x; l < lines; l += gridDim.x) {
-        int r;
-        const int64_t j = split_index(l, nv, r);
-        const float* f = F + r * rs + j * vs;
-#pragma unroll 4
-        for (int c = threadIdx.x; c < nq; c += PAIR_THREADS) {
-            const float a = stored_base<PT>(f[c] * sc);
-            P[l * nq + c] = make_pair<PT>(a, f[c + 1] * sc - a);
+    if constexpr (SHORT) {
+        const int per = blockDim.x / w, c = threadIdx.x % w;
+        if (c >= nq) return;
+        for (int64_t l0 = (int64_t)blockIdx.x * per * PAIR_RUN; l0 < lines; l0 += (int64_t)gridDim.x * per * PAIR_RUN) {
+            float x0[PAIR_RUN], x1[PAIR_RUN];  // all loads before the first store
+            const int64_t l = l0 + threadIdx.x / w;
+#pragma unroll
+            for (int k = 0; k < PAIR_RUN; ++k) {
+                int r;
+                const int64_t j = split_index(min(l + k * per, lines - 1), nv, r);
+                const float* f = F + r * rs + j * vs + c;
+                x0[k] = __ldg(f) * sc;
+                x1[k] = __ldg(f + 1) * sc;
+            }
+#pragma unroll
+            for (int k = 0; k < PAIR_RUN; ++k) {
+                const float a = stored_base<PT>(x0[k]);
+                if (l + k * per < lines) P[(l + k * per) * nq + c] = make_pair<PT>(a, x1[k] - a);
+            }
         }
+    } else {
+        for (int64_t l = blockIdx.x; l < lines; l += gridDim.x) {
+            int r;
+            const int64_t j = split_index(l, nv, r);
+            const float* f = F + r * rs + j * vs;
+#pragma unroll 4
+            for (int c = threadIdx.x; c < nq; c += PAIR_THREADS) {
+                const float a = stored_base<PT>(f[c] * sc);
+                P[l * nq + c] = make_pair<PT>(a, f[c + 1] * sc - a);
+            }
+        }
+    }
+}
+template <typename PT>
+void launch_pack_pair(const mct_geom* g, int64_t rs, int64_t vs, const float* F, void* packed, const uint32_t* maxbits,
+                      cudaStream_t s) {
+    const int64_t lines = (int64_t)g->views * g->nv;
+    const int nq = g->nu - 1;
+    PT* P = static_cast<PT*>(packed);
+    if (nq <= PAIR_THREADS) {
+        const int w = pair_lanes(nq), per = PAIR_THREADS / w;
+        const int blocks = (int)std::min<int64_t>((lines + per * PAIR_RUN - 1) / (per * PAIR_RUN), 1 << 30);
+        pack_pair_kernel<PT, true><<<blocks, w * per, 0, s>>>(g->nu, g->nv, g->views, rs, vs, F, P, maxbits, w);
+    } else {
+        pack_pair_kernel<PT, false><<<(int)std::min<int64_t>(lines, 1 << 30), PAIR_THREADS, 0, s>>>(
+            g->nu, g->nv, g->views, rs, vs, F, P, maxbits, 0);
     }
 }
 
@@ -381,7 +432,7 @@ int mct_pack_strided(const mct_geom* g, const float* src, int64_t row_stride, in
     const int64_t rs = row_stride, vs = view_stride;
     const bool cone = (g->flags & MCT_CONE) != 0;
     MCT_REQUIRE(!cone || g->nv >= 2, "mct_pack: cone beam needs at least 2 detector rows");
-    const int lines = (int)std::min<int64_t>((int64_t)g->views * g->nv, 1 << 30);
+    const int threads = pack_threads(g);
     const int tiles = (int)std::min<int64_t>(std::max<int64_t>(pack_tiles(g), 1), 1 << 30);
     uint32_t* maxbits = nullptr;
     if (dtype == MCT_F16) {
@@ -396,24 +447,18 @@ int mct_pack_strided(const mct_geom* g, const float* src, int64_t row_stride, in
     }
     if (cone) {
         if (dtype == MCT_F32)
-            pack_quad_kernel<float4><<<tiles, 256, 0, s>>>(g->nu, g->nv, g->views, rs, vs, src, (float4*)packed,
+            pack_quad_kernel<float4><<<tiles, threads, 0, s>>>(g->nu, g->nv, g->views, rs, vs, src, (float4*)packed,
                                                                  maxbits);
         else if (dtype == MCT_BF16)
-            pack_quad_kernel<uint2><<<tiles, 256, 0, s>>>(g->nu, g->nv, g->views, rs, vs, src, (uint2*)packed,
+            pack_quad_kernel<uint2><<<tiles, threads, 0, s>>>(g->nu, g->nv, g->views, rs, vs, src, (uint2*)packed,
                                                                 maxbits);
         else
-            pack_quad_kernel<h16x4><<<tiles, 256, 0, s>>>(g->nu, g->nv, g->views, rs, vs, src, (h16x4*)packed,
+            pack_quad_kernel<h16x4><<<tiles, threads, 0, s>>>(g->nu, g->nv, g->views, rs, vs, src, (h16x4*)packed,
                                                                 maxbits);
     } else {
-        if (dtype == MCT_F32)
-            pack_pair_kernel<float2><<<lines, PAIR_THREADS, 0, s>>>(g->nu, g->nv, g->views, rs, vs, src, (float2*)packed,
-                                                                 maxbits);
-        else if (dtype == MCT_BF16)
-            pack_pair_kernel<uint32_t><<<lines, PAIR_THREADS, 0, s>>>(g->nu, g->nv, g->views, rs, vs, src,
-                                                                   (uint32_t*)packed, maxbits);
-        else
-            pack_pair_kernel<h16x2><<<lines, PAIR_THREADS, 0, s>>>(g->nu, g->nv, g->views, rs, vs, src, (h16x2*)packed,
-                                                                maxbits);
+        if (dtype == MCT_F32) launch_pack_pair<float2>(g, rs, vs, src, packed, maxbits, s);
+        else if (dtype == MCT_BF16) launch_pack_pair<uint32_t>(g, rs, vs, src, packed, maxbits, s);
+        else launch_pack_pair<h16x2>(g, rs, vs, src, packed, maxbits, s);
     }
     return launched("pack_kernel");
 }
