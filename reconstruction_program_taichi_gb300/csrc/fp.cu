@@ -39,8 +39,8 @@ __device__ __forceinline__ bool spread_along_y(const FpParams& p, int j, const f
 // detector tiles.  Blocks are scheduled x, then y, then z, so the blocks resident at
 // one time cover many views of the same detector rows; those rays cross only a thin
 // z-slab of the volume, which then stays in L2 across views.  fp_kernel takes tiles of
-// 16 columns x 2^vshift consecutive views x 2^(4 - vshift) rows (x = column tiles, y =
-// view groups, z = row tiles).
+// 16 columns, several consecutive views and rows (x = column tiles, y = view groups, z =
+// row tiles).
 //
 // One thread per ray (u, v) of view j.  vol is [z][y][x]; vol_t, when
 // given, is the same volume as [z][x][y]: views whose detector columns spread along
@@ -132,13 +132,13 @@ fp_kernel(FpParams p, const float* __restrict__ angles, const float* __restrict_
     // of 2^wcs columns x 2^(5 - wcs) slots
     const int tid = threadIdx.y * 32 + threadIdx.x;
     const int warp = tid >> 5, lane = tid & 31;
-    const int gpr = p.bcs - p.wcs;  // log2 of the warps across the tile's columns
+    const int gpr = 4 - p.wcs;  // log2 of the warps across the tile's columns
     const int tx = ((warp & ((1 << gpr) - 1)) << p.wcs) + (lane & ((1 << p.wcs) - 1));
     const int ty = ((warp >> gpr) << (5 - p.wcs)) + (lane >> p.wcs);
-    const int iu = (blockIdx.x << p.bcs) + tx;
+    const int iu = (blockIdx.x << 4) + tx;
     const int vs = p.vshift;
     const int vg = blockIdx.y >> p.rs, rsub = blockIdx.y & ((1 << p.rs) - 1);  // view group, row tile in it
-    const int iv = ((((int)blockIdx.z << p.rs) + rsub) << (8 - p.bcs - vs)) + (ty >> vs);
+    const int iv = ((((int)blockIdx.z << p.rs) + rsub) << (p.ls - 4 - vs)) + (ty >> vs);
     const int j = (vg << vs) + (ty & ((1 << vs) - 1));
     if (iu >= p.nu || iv >= p.nv || j >= p.views) return;
     const int64_t oidx = ((int64_t)iv * p.views + j) * p.nu + iu;
@@ -921,17 +921,27 @@ inline double samples_per_cell(const mct_geom* g) {
     const double step = g->fp_step * std::sqrt(2.0 + ((double)g->pz / g->px) * ((double)g->pz / g->px));
     return 1.0 / (1.33 * step);
 }
-// Whether a ray with copies is walked by samples: few samples per cell.  256x256x64, 360 views, by
-// samples / by cells, ms: bf16 step 0.2 (2.2 samples per cell) 4.84 / 3.46, 0.3 (1.4) 3.22 /
-// 3.31 (140 columns, 300 views: 0.929 / 0.966), 0.5 (0.9) 2.1 / 2.95; float16, which pays
-// more per load, 0.3 3.8 / 3.60, 0.5 2.33 / 3.19.  float32, us: 123x123x51, 686 views, 0.3
-// 1320 / 1261, 0.4 (1.1) 1106 / 1193, 0.5 974 / 1119; 224x224x64, 120 views, 0.4 901 / 897,
-// 0.5 795 / 841, 0.7 664 / 654; 64^3, 180 views, 0.4 139 / 153, 0.5 126 / 144.  With windows,
-// from 256 columns on, cells stay: 512x512x64, 90 views, 0.5 3567 / 3252, 0.7 3024 / 2524
-// (300 columns, 300 views: 2164 / 2250, 1772 / 1817).
-inline bool walk_by_samples(const mct_geom* g, int32_t dtype) {
-    if (dtype == MCT_F32 && walk_in_windows(g)) return false;
-    return samples_per_cell(g) < (dtype == MCT_BF16 ? 1.5 : 1.2);
+// Scans whose neighbouring views cross nearly the same cells.
+inline bool long_scan(const mct_geom* g) { return g->views >= 256 || g->views >= g->nx; }
+// Whether a ray is walked by samples: few samples per cell.  us, by samples / by cells (what
+// the walk by samples was before the walk by cells came):
+//   bf16 256x256x64, 360 views, step 0.3 (1.4 samples per cell) 3220 / 3310, 0.5 (0.9) 2100 / 2950;
+//   float16, which pays more per load: 32x32x23, 35 views, 0.3 23.2 / 30.8 (27.0), 170x170x19, 37
+//     views 90.6 / 108.5 (94.5); from 256 columns 0.3 is even, 0.5 2330 / 3190;
+//   float32 123x123x51, 686 views, 0.3 1320 / 1261, 0.4 (1.1) 1106 / 1193, 0.5 974 / 1119;
+//     224x224x64, 120 views, 0.4 901 / 897, 0.5 795 / 841; without copies 81x81x3, 171 views,
+//     0.5 27.5 / 32.3 (26.8), 54x54x36, 23 views, 1.2 14.5 / 17.9 (16.4);
+//   fan beam 491 columns, 147 views, 0.5 (1.1) 194 / 223 (207), 253 columns, 52 views, 1.2
+//     43.7 / 49.1 (45.3); step 0.3 (1.8) costs samples 1.5 to 1.9 times as much.
+// With windows, from 256 columns on, float32 cells stay for short scans (512x512x64, 90 views, 0.5
+// 3567 / 3252); long ones go by samples where a cell holds about one (319x319x109, 617 views,
+// 0.5 13570 / 14380 (13964); 426 columns, 0.7 (0.6) 15725 / 15290 but 270 columns 1933 / 2094
+// (1990); 1.0 (0.4) 2 % more for samples).  Without copies they stay (even at 0.5).
+inline bool walk_by_samples(const mct_geom* g, int32_t dtype, bool copies) {
+    const bool cone = (g->flags & MCT_CONE) != 0, wide = walk_in_windows(g);
+    const double n = samples_per_cell(g);
+    if (dtype == MCT_F32 && cone && wide) return copies && long_scan(g) && n >= 0.6 && n < 1.2;
+    return n < (dtype == MCT_BF16 || (dtype == MCT_F16 && !wide) ? 1.5 : 1.2);
 }
 inline size_t copy_elems(const mct_geom* g) { return (size_t)g->nz * g->nx * copy_pitch(g); }
 
@@ -1012,22 +1022,38 @@ int fp_storage_impl(const mct_geom* g, const mct_tables* t, const TIN* vol_in, c
     // 128x128x64, 270 views 0.698 / 0.741; 123x123x51: 140 views 0.325 / 0.335, 90 views 0.241
     // / 0.240; 100x100x40, 200 views 0.228 / 0.245; 64^3, 180 views 0.158 / 0.169.  16-bit
     // cells take 4 views x 4 rows: bf16 512x512x128, 90 views 7.60 ms against 7.73 with 16
-    // views; 256x256x64, 360 views 3.457 against 3.480; by samples they keep warps of 4
-    // columns.  Fan beam: warps of 8 columns x 4 views (512^2, 720 views, 4 / 8 / 16 columns:
-    // 0.604 / 0.596 / 0.595; 128^2 x 16, 360 views 0.327 / 0.324 / 0.339; one row of 32
-    // columns x 8 rows, 7 of them idle for one slice: 0.664).
-    // With copies, 4 row tiles are taken in turn per view group: neighbouring rows' rays
+    // views; 256x256x64, 360 views 3.457 against 3.480.  Fan beam: warps of 8 columns x 4
+    // views (512^2, 720 views, 4 / 8 / 16 columns: 0.604 / 0.596 / 0.595; 128^2 x 16, 360
+    // views 0.327 / 0.324 / 0.339; one row of 32 columns x 8 rows, 7 of them idle for one
+    // slice: 0.664).  By samples, blocks of 128 rays, 16 columns x 8 views, in warps of 4 (long
+    // scans) or 8 columns: 170x170x19, 37 views, float16 90.6 us against 97.7 with 4 views x 4
+    // rows; 68x68x18, 224 views, bf16 13 % less, fan beam 246 columns, 134 views 53.9 us against
+    // 60.4; only wide long scans keep 16 views (float32 388 columns, 885 views 26.6 / 27.3 ms).
+    // Where the tile leaves a fifth of its rays outside the scan, 8 or 4 views x 2 or 4 rows
+    // (fan beam 210 columns x 16 rows, 23 views 200 -> 153 us).
+    // With copies, 4 rows are taken in turn per view group: neighbouring rows' rays
     // cross nearly the same cells, and the outer rows' slab (up to ~50 planes) does not fit
     // L2 across all views.  Otherwise row tiles are only grouped where the grid needs it.
-    const bool copies = p.cone && workspace;
-    const bool long_scan = g->views >= 256 || g->views >= g->nx, by_samples = copies && walk_by_samples(g, dtype);
-    p.bcs = 4;
-    p.vshift = copies && dtype != MCT_F32 ? 2 : 4;
-    p.wcs = !p.cone ? 3 : long_scan || by_samples ? 2 : 4;
-    p.rs = copies ? (p.vshift == 4 ? 2 : 0) : (g->nv > 65535 ? 3 : 0);
+    const bool copies = p.cone && workspace, by_samples = walk_by_samples(g, dtype, copies);
+    const bool small_tile = by_samples && !(dtype == MCT_F32 && p.cone && walk_in_windows(g)) && g->nv <= 65535;
+    p.ls = small_tile ? 7 : 8;
+    p.vshift = small_tile ? 3 : copies && dtype != MCT_F32 ? 2 : 4;
+    p.wcs = !p.cone ? 3 : long_scan(g) ? 2 : by_samples ? 3 : 4;
+    if (!small_tile) {
+        auto rays = [&](int vs) {  // of the tiles of 2^vs views, in and outside the scan
+            const int64_t v = (1 << vs) - 1, r = (1 << (4 - vs)) - 1;
+            return ((g->views + v) & ~v) * ((g->nv + r) & ~r);
+        };
+        int best = 4;
+        for (int vs = 3; vs >= 2; --vs)
+            if (rays(vs) < rays(best)) best = vs;
+        if (rays(p.vshift) * 4 > rays(best) * 5) p.vshift = best;
+    }
+    const int row_bits = p.ls - 4 - p.vshift;
+    p.rs = copies ? (row_bits < 2 ? 2 - row_bits : 0) : (g->nv > 65535 ? 3 : 0);
     if (copies) p.pitch = copy_pitch(g);
-    const int vb = 1 << p.vshift, rb = 1 << (8 - p.bcs - p.vshift + p.rs), cb = 1 << p.bcs;
-    dim3 block(32, 8), grid((g->nu + cb - 1) / cb, ((g->views + vb - 1) / vb) << p.rs, (g->nv + rb - 1) / rb);
+    const int vb = 1 << p.vshift, rb = 1 << (row_bits + p.rs);
+    dim3 block(32, 1 << (p.ls - 5)), grid((g->nu + 15) / 16, ((g->views + vb - 1) / vb) << p.rs, (g->nv + rb - 1) / rb);
     const size_t n = copy_elems(g);
     if (copies && dtype == MCT_BF16) {
         uint4* cx = static_cast<uint4*>(workspace);
@@ -1071,14 +1097,10 @@ int fp_storage_impl(const mct_geom* g, const mct_tables* t, const TIN* vol_in, c
             transpose_xy_kernel<<<tg, tb, 0, s>>>(g->nx, g->nz, vol, vt);
             MCT_TRY(launched("transpose_xy_kernel"));
         }
-        if (p.cone)
-            fp_kernel<true, false, float2, kCells><<<grid, block, 0, s>>>(p, t->angles, t->u, t->v, t->cz, t->pmat_a,
-                                                                  t->pmat_xs, vol, vt, nullptr, nullptr, mask, sgm,
-                                                                  nullptr);
-        else
-            fp_kernel<false, false, float2, kWindows><<<grid, block, 0, s>>>(p, t->angles, t->u, t->v, t->cz, t->pmat_a,
-                                                                   t->pmat_xs, vol, vt, nullptr, nullptr, mask, sgm,
-                                                                   nullptr);
+        auto go = p.cone ? (by_samples ? fp_kernel<true, false, float2, kSamples> : fp_kernel<true, false, float2, kCells>)
+                         : (by_samples ? fp_kernel<false, false, float2, kSamples> : fp_kernel<false, false, float2, kWindows>);
+        go<<<grid, block, 0, s>>>(p, t->angles, t->u, t->v, t->cz, t->pmat_a, t->pmat_xs, vol, vt, nullptr, nullptr, mask, sgm,
+                                  nullptr);
     }
     return launched("fp_kernel");
 }

@@ -17,11 +17,11 @@ struct FpParams {
     float stepvd, l_min, inv_px, inv_pz;
     float x0, y0, zoff;  // voxel (0,0) centre x, y; z0 = zoff + cz_view
     float zpv;
-    // fp_kernel ray tiling: a block of 256 rays is 2^bcs detector columns x 2^vshift
-    // views x 2^(8 - bcs - vshift) detector rows, a warp 2^wcs columns x 2^(5 - wcs)
-    // of the block's (view, row) slots; blockIdx.y runs over 2^rs row tiles within
-    // each view group (the block order is column tile, row tile, view group, row group)
-    int vshift, bcs, wcs, rs;
+    // fp_kernel's ray tiles: a block of 2^ls rays is 16 detector columns x 2^vshift views x
+    // 2^(ls - 4 - vshift) detector rows, a warp 2^wcs columns x 2^(5 - wcs) of the block's
+    // (view, row) slots; blockIdx.y runs over 2^rs row tiles within each view group (the
+    // block order is column tile, row tile, view group, row group)
+    int ls, vshift, wcs, rs;
     int pitch;  // elements per row of the volume or its copies (a plane is nx rows)
 };
 
@@ -149,7 +149,7 @@ MCT_HD bool interior_range(const FpParams& p, const Ray& r, bool test_z, int& ki
 // advance one by one): such rays are sampled one sample at a time.
 constexpr int kMaxWalkSteps = 1 << 23;
 
-// The launch parameters of a geometry, with the ray tile of the plain ray kernels.
+// The launch parameters of a geometry, without a ray tile.
 inline FpParams ray_params(const mct_geom* g) {
     FpParams p{};
     p.nx = g->nx; p.nz = g->nz; p.nu = g->nu; p.nv = g->nv; p.views = g->views; p.K = g->fp_steps;
@@ -169,10 +169,6 @@ inline FpParams ray_params(const mct_geom* g) {
     p.y0 = (float)(-(g->nx - 1.0) / 2.0 * (-px) + g->cy);
     p.zoff = (float)(-(g->nz - 1.0) / 2.0 * (double)g->pz);
     p.zpv = g->fp_z_per_view;
-    p.vshift = 0;
-    p.bcs = 5;  // 32 columns x 8 rows of one view, warps of 32 columns
-    p.wcs = 5;
-    p.rs = 0;
     p.pitch = g->nx;
     return p;
 }

@@ -40,3 +40,67 @@ def test_one_slice_projects_nothing(n, nu, nv, views, cz, cuda):
         assert not _adjoint(dg, y, None, ws).any()
         assert not ops.fp(dg, x, workspace=ws).any()
     assert ops.fp_count_samples(dg) == 0
+
+
+def _clear_rays(o, dg, step):
+    """1 for the rays all of whose samples keep 1e-3 voxel from the volume's faces: there an
+    inside test flips with the rounding of the position."""
+    g = dg.geom
+    h = dg.host
+    n, nz, px, pz = g.nx, g.nz, o.img_pix_size, o.img_voxel_height
+    lmin = g.sid - np.sqrt(2 * (n * px) ** 2 + (nz * pz) ** 2) / 2
+    l = np.arange(g.fp_steps) * step * np.sqrt(2 * px * px + pz * pz) + lmin
+    out = np.ones(dg.sgm_shape, np.float32)
+    for j in range(g.views):
+        sz, ux, uy, uz, _ = P._ray_dirs(h["u"], h["v"], g.nv, g.sid, g.sdd, False, 0.0, j)
+        c, s = np.cos(h["angles"][j]), np.sin(h["angles"][j])
+        x, y, z = g.sid + ux[..., None] * l, uy[..., None] * l, sz + uz[..., None] * l
+        fx = (x * c - y * s + (n - 1) / 2 * px - g.cx) / px
+        fy = (y * c + x * s - (n - 1) / 2 * px - g.cy) / -px
+        fz = (z + (nz - 1) / 2 * pz - o.array_img_center_z[j]) / pz
+        near = np.zeros(fx.shape, bool)
+        for f, m in ((fx, n), (fy, n), (fz, nz)):
+            near |= (np.abs(f) < 1e-3) | (np.abs(f - (m - 1)) < 1e-3)
+        # only where the other axes do not already put the sample outside
+        reach = np.ones(fx.shape, bool)
+        for f, m in ((fx, n), (fy, n), (fz, nz)):
+            reach &= (f > -1e-3) & (f < m - 1 + 1e-3)
+        out[:, j] = 1.0 - (near & reach).any(-1)
+    return out
+
+
+# float32 sample positions are within 3 * 2^-24 * n of the float64 ones (1.2e-5 voxel at n = 64);
+# with values and differences of the same size that bounds a ray's relative error by about as
+# much, a voxel's by 3 times that (weights of 0.35).  Storage rounds by 2^-11 / 2^-8 at most.
+TOL = {"f32": 5e-5, "f16": 2.0 ** -11, "bf16": 2.0 ** -8}
+
+
+@pytest.mark.parametrize("nz,nv", [(2, 7), (3, 8)])
+@pytest.mark.parametrize("step", [0.05, 0.2, 0.5, 1.3])
+def test_one_and_two_layers_of_cells(nz, nv, step, cuda):
+    import torch
+    from reconstruction_program_taichi_gb300 import ops
+    n, nu, views = 40, 35, 24
+    o, dg = _scan(n, nz, nu, nv, views, step, 1.1, ImageCenterZ=0.13)
+    mask = _clear_rays(o, dg, step)
+    assert mask.mean() > 0.5
+    rng = np.random.default_rng(nz)
+    vol = (rng.uniform(-1, 1, dg.vol_shape) + 0.5).astype(np.float32)
+    y = (rng.uniform(-1, 1, dg.sgm_shape) + 0.5).astype(np.float32)
+
+    def march(j, **kw):
+        return P.march(vol if "out" not in kw else None, j, dg.host["angles"], dg.host["u"], dg.host["v"], nx=n, nz=nz,
+                       px=o.img_pix_size, pz=o.img_voxel_height, cx=o.img_center_x, cy=o.img_center_y,
+                       cz_view=o.array_img_center_z[j], sid=o.source_isocenter_dis, sdd=o.source_det_dis, step=step,
+                       cone_beam=True, rows=nv, K=dg.geom.fp_steps, mask=mask[:, j], **kw)
+
+    ref = np.stack([march(j) for j in range(views)], axis=1)
+    back = np.zeros(dg.vol_shape)
+    for j in range(views):
+        march(j, mode="adjoint", ray_values=y[:, j], out=back)
+    x, m, yt = torch.from_numpy(vol).cuda(), torch.from_numpy(mask).cuda(), torch.from_numpy(y).cuda()
+    for storage, kw in (("f32", {}), ("f32", dict(workspace=None)), ("bf16", dict(dtype=ops.MCT_BF16)),
+                        ("f16", dict(dtype=ops.MCT_F16))):
+        assert rel_l2(ops.fp(dg, x, mask=m, **kw).cpu().numpy(), ref) < TOL[storage]
+    for ws in (True, None):
+        assert rel_l2(_adjoint(dg, yt, m, ws), back) < 3 * TOL["f32"]
