@@ -266,9 +266,12 @@ fp_kernel(FpParams p, const float* __restrict__ angles, const float* __restrict_
                 CONE ? MB * (unsigned)(plane + sy + sx) : MB * (unsigned)(sy + sx) - (unsigned)(iv * plane);
             const float2 M2 = make_float2(M, M), nM2 = make_float2(-M, -M);
             const float2 dxy = make_float2(r.dfx, r.dfy), fxy0 = make_float2(r.fx0, r.fy0);
-            // steps from fraction w to the face that the ray leaves the cell through: A + w * B
-            const float ix = fminf(1.0f / fabsf(r.dfx), 1e6f), iy = fminf(1.0f / fabsf(r.dfy), 1e6f);
-            const float iz = fminf(1.0f / fabsf(r.dfz), 1e6f);
+            // steps from fraction w to the face that the ray leaves the cell through: A + w * B.
+            // The bound keeps an axis without motion finite and is far enough that it never ends
+            // a run (at 1e6 a ray along a plane, whose fraction rounds to 1 - 2^-24, took its
+            // samples one by one: bf16 141x141x3, 129 views of 3 rows 115 us, now 66; float32 132, 73).
+            const float ix = fminf(1.0f / fabsf(r.dfx), 1e30f), iy = fminf(1.0f / fabsf(r.dfy), 1e30f);
+            const float iz = fminf(1.0f / fabsf(r.dfz), 1e30f);
             const float2 B2 = make_float2(r.dfx < 0.0f ? ix : -ix, r.dfy < 0.0f ? iy : -iy);
             const float2 A2 = make_float2(r.dfx < 0.0f ? 0.0f : ix, r.dfy < 0.0f ? 0.0f : iy);
             const float Bz = r.dfz < 0.0f ? iz : -iz, Az = r.dfz < 0.0f ? 0.0f : iz;
@@ -634,7 +637,7 @@ __device__ __forceinline__ void adjoint_ray(const FpParams& p, const Ray& r, int
         const float2 flip = make_float2(fx ? -1.0f : 1.0f, fy ? -1.0f : 1.0f), base = make_float2(fx ? 1.0f : 0.0f, fy ? 1.0f : 0.0f);
         const float2 hd = make_float2(0.5f * dx, 0.5f * dy);
         const float hdz = 0.5f * dzz;
-        const float ix = fminf(1.0f / dx, 1e6f), iy = fminf(1.0f / dy, 1e6f), iz = fminf(1.0f / dzz, 1e6f);
+        const float ix = fminf(1.0f / dx, 1e30f), iy = fminf(1.0f / dy, 1e30f), iz = fminf(1.0f / dzz, 1e30f);  // as in fp_kernel
         const float kend = (float)kie;
         float fk = (float)kis;
         while (fk <= kend) {

@@ -104,3 +104,34 @@ def test_one_and_two_layers_of_cells(nz, nv, step, cuda):
         assert rel_l2(ops.fp(dg, x, mask=m, **kw).cpu().numpy(), ref) < TOL[storage]
     for ws in (True, None):
         assert rel_l2(_adjoint(dg, yt, m, ws), back) < 3 * TOL["f32"]
+
+
+@pytest.mark.parametrize("n,nz,nu,nv,step", [(41, 3, 41, 3, 0.2), (41, 9, 41, 7, 0.1), (9, 41, 41, 41, 0.3), (40, 5, 41, 1, 0.9)])
+def test_rays_along_planes(n, nz, nu, nv, step, cuda):
+    """A centred scan of an odd number of planes, rows and columns: the middle row's rays stay
+    on a plane, some views' middle column's on a column of voxels, with fractions that round to
+    0 or to 1 - 2^-24."""
+    import torch
+    from reconstruction_program_taichi_gb300 import ops
+    views = 8
+    o, dg = _scan(n, nz, nu, nv, views, step, 0.8, ImageCenterZ=0.0, DetectorOffsetVertical=0.0, ImageCenter=[0.0, 0.0],
+                  DetectorOffsetHorizontal=0.0, ImageRotation=0)
+    mask = _clear_rays(o, dg, step)
+    assert mask[nv // 2].mean() > 0.5
+    rng = np.random.default_rng(n)
+    vol = (rng.uniform(-1, 1, dg.vol_shape) + 0.5).astype(np.float32)
+    y = (rng.uniform(-1, 1, dg.sgm_shape) + 0.5).astype(np.float32)
+    kw = dict(nx=n, nz=nz, px=o.img_pix_size, pz=o.img_voxel_height, cx=0.0, cy=0.0, sid=o.source_isocenter_dis,
+              sdd=o.source_det_dis, step=step, cone_beam=True, rows=nv, K=dg.geom.fp_steps)
+    tables = dg.host["angles"], dg.host["u"], dg.host["v"]
+    ref = np.stack([P.march(vol, j, *tables, cz_view=o.array_img_center_z[j], mask=mask[:, j], **kw) for j in range(views)], 1)
+    back = np.zeros(dg.vol_shape)
+    for j in range(views):
+        P.march(None, j, *tables, cz_view=o.array_img_center_z[j], mask=mask[:, j], mode="adjoint", ray_values=y[:, j],
+                out=back, **kw)
+    x, m, yt = torch.from_numpy(vol).cuda(), torch.from_numpy(mask).cuda(), torch.from_numpy(y).cuda()
+    for storage, a in (("f32", {}), ("f32", dict(workspace=None)), ("bf16", dict(dtype=ops.MCT_BF16)),
+                       ("f16", dict(dtype=ops.MCT_F16))):
+        assert rel_l2(ops.fp(dg, x, mask=m, **a).cpu().numpy(), ref) < TOL[storage]
+    for ws in (True, None):
+        assert rel_l2(_adjoint(dg, yt, m, ws), back) < 3 * TOL["f32"]
