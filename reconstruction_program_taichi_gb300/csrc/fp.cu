@@ -624,7 +624,7 @@ __device__ __forceinline__ void adjoint_ray(const FpParams& p, const Ray& r, int
     };
     int kis, kie;
     interior_range(p, r, CONE, kis, kie);
-    if (p.K >= kMaxWalkSteps || p.by_samples) {  // kMaxWalkSteps: step indices would not be exact in float32
+    if (p.K >= kMaxWalkSteps) {  // step indices would not be exact in float32
         kis = r.ke + 1;
         kie = r.ke;
     }
@@ -702,8 +702,7 @@ __device__ __forceinline__ void adjoint_ray_z(const FpParams& p, const Ray& r, i
 // after: 123x123x51, 300 views 7.95 / 5.16, step 0.5 6.06 / 5.05; fan beam 300^2 x 4, 360
 // views 2.35 / 1.40.  Blocks of 8 rows of rays (4 cost the scalar additions 2 to 10 %); of 4
 // for cone beam with CELLS (grad above 2 %, 512^2 x 64 4 %), where the grid allows it.
-// Fan beam with CELLS goes by samples where a cell holds about one (300^2 x 4, 360 views,
-// by samples / by cells, ms: step 0.2 1.02 / 0.71, 0.4 0.64 / 0.66, 0.5 0.60 / 0.64).
+// Where a cell holds few samples, fp_adjoint_samples_kernel below (adjoint_by_samples).
 template <bool CONE, bool CELLS>
 __global__ void __launch_bounds__(256)
 fp_adjoint_kernel(FpParams p, const float* __restrict__ angles, const float* __restrict__ u_arr,
@@ -731,6 +730,93 @@ fp_adjoint_kernel(FpParams p, const float* __restrict__ angles, const float* __r
         else
             adjoint_ray_z<CONE, CELLS, false, false>(p, r, iv, yv, out);
     }
+}
+
+// The adjoint sample by sample, for rays with few cells or about a sample per cell: a cell's corner
+// sums are kept in registers and all added when the ray enters another, into the buffers of
+// fp_adjoint_kernel with CELLS (cone beam: the faces behind and ahead along x).
+template <bool CONE, bool CELLS>
+__global__ void __launch_bounds__(256)
+fp_adjoint_samples_kernel(FpParams p, const float* __restrict__ angles, const float* __restrict__ u_arr,
+                          const float* __restrict__ v_arr, const float* __restrict__ czv, const float* __restrict__ pa,
+                          const float* __restrict__ pxs, const float* __restrict__ sgm, const float* __restrict__ mask,
+                          float* __restrict__ out) {
+    const int iu = blockIdx.x * blockDim.x + threadIdx.x;
+    const int iv = blockIdx.z * blockDim.y + threadIdx.y;
+    const int j = blockIdx.y;
+    if (iu >= p.nu || iv >= p.nv) return;
+    const int64_t oidx = ((int64_t)iv * p.views + j) * p.nu + iu;
+    if (mask && mask[oidx] != 1.0f) return;
+    const float yv = sgm[oidx] * p.stepvd;
+    if (yv == 0.0f) return;
+    Ray r;
+    if (!setup_ray(p, iu, iv, j, angles, u_arr, v_arr, czv, pa, pxs, true, r)) return;
+    const int nx = p.nx;
+    const int plane = nx * nx;
+    int cell = -1;
+    float s00 = 0.f, s01 = 0.f, s10 = 0.f, s11 = 0.f, t00 = 0.f, t01 = 0.f, t10 = 0.f, t11 = 0.f;  // <y><x>; t: z ahead
+    auto flush = [&]() {
+        if (cell < 0) return;
+        if constexpr (CELLS) {
+            float* c = out + (int64_t)cell * 4;
+            if (CONE) {
+                red_add_v4(c, s00, s10, t00, t10);
+                red_add_v4(c + 4, s01, s11, t01, t11);
+            } else {
+                red_add_v4(c, s00, s01, s10, s11);
+            }
+        } else {
+            float* b = out + cell;
+            atomicAdd(b, s00);
+            atomicAdd(b + 1, s01);
+            atomicAdd(b + nx, s10);
+            atomicAdd(b + nx + 1, s11);
+            if (CONE) {
+                float* c = b + plane;
+                atomicAdd(c, t00);
+                atomicAdd(c + 1, t01);
+                atomicAdd(c + nx, t10);
+                atomicAdd(c + nx + 1, t11);
+            }
+        }
+        s00 = s01 = s10 = s11 = t00 = t01 = t10 = t11 = 0.f;
+    };
+    for (int k = r.ks; k <= r.ke; ++k) {
+        const float fk = (float)k;
+        const float fx = fmaf(fk, r.dfx, r.fx0), fy = fmaf(fk, r.dfy, r.fy0);
+        const float xf = floorf(fx), yf = floorf(fy);
+        if (!(xf >= 0.0f && xf + 1.0f < (float)nx && yf >= 0.0f && yf + 1.0f < (float)nx)) continue;
+        const float xw = fx - xf, yw = fy - yf;
+        int zi = iv;
+        float zw = 0.0f;
+        if (CONE) {
+            const float fz = fmaf(fk, r.dfz, r.fz0);
+            const float zf = floorf(fz);
+            if (!(zf >= 0.0f && zf + 1.0f < (float)p.nz)) continue;
+            zi = (int)zf;
+            zw = fz - zf;
+        }
+        const int off = zi * plane + (int)yf * nx + (int)xf;
+        if (off != cell) {
+            flush();
+            cell = off;
+        }
+        const float wl = CONE ? (1.0f - zw) * yv : yv;
+        const float w00 = (1.0f - xw) * (1.0f - yw), w01 = xw * (1.0f - yw);
+        const float w10 = (1.0f - xw) * yw, w11 = xw * yw;
+        s00 += w00 * wl;
+        s01 += w01 * wl;
+        s10 += w10 * wl;
+        s11 += w11 * wl;
+        if (CONE) {
+            const float wh = zw * yv;
+            t00 += w00 * wh;
+            t01 += w01 * wh;
+            t10 += w10 * wh;
+            t11 += w11 * wh;
+        }
+    }
+    flush();
 }
 
 // vol[z][y][x] += its entries of the faces (cone beam, buffers XF and YF above) or cells
@@ -946,6 +1032,28 @@ inline bool walk_by_samples(const mct_geom* g, int32_t dtype, bool copies) {
     if (dtype == MCT_F32 && cone && wide) return copies && long_scan(g) && n >= 0.6 && n < 1.2;
     return n < (dtype == MCT_BF16 || (dtype == MCT_F16 && !wide) ? 1.5 : 1.2);
 }
+// Whether the adjoint goes by samples; figures by samples / by cells.
+// A thread pays for a walk by cells before its first sample, so grids that leave the GPU
+// waiting go by samples where a cell holds about one: 66x66x2, 55 views of 2 x 123, step 1.2,
+// without a workspace 7.8 / 13.6 us; 90x90x4, 73 views of 4 x 174, step 0.5, with one 36 / 42 us.
+// Fan beam with a workspace: the reductions are the same either way (445^2 x 2, 179 views, step
+// 0.5 417 / 425 us, 0.3 492 / 449).
+// Otherwise it is the faces that the walk by cells saves.  Without a workspace it pays until a
+// cell holds half a sample (123x123x51, 300 views, step 0.7 5.7 / 5.1 ms, 1.0 3.97 / 4.02, 1.5
+// 2.71 / 2.81; fan beam 300^2 x 4, 360 views, 1.0 1.49 / 1.33, 1.5 0.98 / 0.97).  With one, whose
+// reductions carry four values, the longer the wider the volume (51x51x19, 95 views, 0.8 31 / 46
+// us; 115x115x40, 674 views, 0.8 2.27 / 2.07 ms; 64^3, 180 views, 0.5 0.36 / 0.30 ms, 2.5 83 /
+// 103 us), and less where columns a voxel and more apart share few faces (67x67x100, 292 views
+// of 111 x 61, 1.2 259 / 316 us).
+inline bool adjoint_by_samples(const mct_geom* g, bool cells) {
+    const bool cone = (g->flags & MCT_CONE) != 0;
+    const double n = samples_per_cell(g);
+    const int64_t rays = sgm_elems(*g);
+    if ((!cone && cells) || rays < 60000) return n < (rays < 4000 ? 1.6 : 1.2);
+    if (!cone) return false;
+    if (!cells) return n < (g->nx < 64 ? 0.6 : 0.45);
+    return n < (g->nx < 32 ? 1.5 : g->nx < 64 ? 1.2 : g->nx < 112 ? 0.6 : 4LL * g->nu <= 5LL * g->nx ? 0.4 : 0.0);
+}
 inline size_t copy_elems(const mct_geom* g) { return (size_t)g->nz * g->nx * copy_pitch(g); }
 
 int make_params(const mct_geom* g, FpParams& p, const char* who) {
@@ -1026,9 +1134,10 @@ int fp_storage_impl(const mct_geom* g, const mct_tables* t, const TIN* vol_in, c
     // / 0.240; 100x100x40, 200 views 0.228 / 0.245; 64^3, 180 views 0.158 / 0.169.  16-bit
     // cells take 4 views x 4 rows: bf16 512x512x128, 90 views 7.60 ms against 7.73 with 16
     // views; 256x256x64, 360 views 3.457 against 3.480.  Fan beam: warps of 8 columns x 4
-    // views (512^2, 720 views, 4 / 8 / 16 columns: 0.604 / 0.596 / 0.595; 128^2 x 16, 360
-    // views 0.327 / 0.324 / 0.339; one row of 32 columns x 8 rows, 7 of them idle for one
-    // slice: 0.664).  By samples, blocks of 128 rays, 16 columns x 8 views, in warps of 4 (long
+    // views (512^2, 720 views, 4 / 8 / 16 columns: 0.604 / 0.596 / 0.595; 128^2 x
+    // 16, 360 views 0.327 / 0.324 / 0.339; one row of 32 columns x 8 rows, 7 of them idle for one
+    // slice: 0.664), of 16 x 2 where the views are far apart and there are slices enough (243^2 x
+    // 65, 46 views, step 0.8 0.420 / 0.368; 258^2 x 4, 67 views, step 0.1 0.124 / 0.114).  By samples, blocks of 128 rays, 16 columns x 8 views, in warps of 4 (long
     // scans) or 8 columns: 170x170x19, 37 views, float16 90.6 us against 97.7 with 4 views x 4
     // rows; 68x68x18, 224 views, bf16 13 % less, fan beam 246 columns, 134 views 53.9 us against
     // 60.4; only wide long scans keep 16 views (float32 388 columns, 885 views 26.6 / 27.3 ms).
@@ -1041,7 +1150,8 @@ int fp_storage_impl(const mct_geom* g, const mct_tables* t, const TIN* vol_in, c
     const bool small_tile = by_samples && !(dtype == MCT_F32 && p.cone && walk_in_windows(g)) && g->nv <= 65535;
     p.ls = small_tile ? 7 : 8;
     p.vshift = small_tile ? 3 : copies && dtype != MCT_F32 ? 2 : 4;
-    p.wcs = !p.cone ? 3 : long_scan(g) ? 2 : by_samples ? 3 : 4;
+    if (p.cone) p.wcs = long_scan(g) ? 2 : by_samples ? 3 : 4;
+    else p.wcs = g->nv >= 4 && 2 * g->views < g->nx ? 4 : 3;
     if (!small_tile) {
         auto rays = [&](int vs) {  // of the tiles of 2^vs views, in and outside the scan
             const int64_t v = (1 << vs) - 1, r = (1 << (4 - vs)) - 1;
@@ -1138,7 +1248,9 @@ int mct_fp_adjoint(const mct_geom* g, const mct_tables* t, const float* sgm, con
     MCT_REQUIRE(!p.pmat || (t->pmat_a && t->pmat_xs), "mct_fp_adjoint: projection-matrix tables missing");
     if (p.cone && g->nz < 2) return MCT_OK;  // no cell, so mct_fp sums nothing: its transpose adds nothing
     dim3 block(32, 8), grid((g->nu + 31) / 32, g->views, (g->nv + 7) / 8);
-    auto go = p.cone ? fp_adjoint_kernel<true, false> : fp_adjoint_kernel<false, false>;
+    const bool by_samples = adjoint_by_samples(g, false);
+    auto go = p.cone ? (by_samples ? fp_adjoint_samples_kernel<true, false> : fp_adjoint_kernel<true, false>)
+                     : (by_samples ? fp_adjoint_samples_kernel<false, false> : fp_adjoint_kernel<false, false>);
     go<<<grid, block, 0, as_stream(stream)>>>(p, t->angles, t->u, t->v, t->cz, t->pmat_a, t->pmat_xs, sgm, mask, vol);
     return launched("fp_adjoint_kernel");
 }
@@ -1161,10 +1273,11 @@ int mct_fp_adjoint_cells(const mct_geom* g, const mct_tables* t, const float* sg
     float* cells = static_cast<float*>(workspace);
     MCT_REQUIRE(cudaMemsetAsync(cells, 0, mct_fp_adjoint_workspace_size(g), s) == cudaSuccess,
                 "mct_fp_adjoint_cells: clearing the workspace failed");
-    p.by_samples = !p.cone && samples_per_cell(g) < 1.2;
+    const bool by_samples = adjoint_by_samples(g, true);
     const int rows = p.cone && g->nv <= 4 * 65535 ? 4 : 8;
     dim3 block(32, rows), grid((g->nu + 31) / 32, g->views, (g->nv + rows - 1) / rows);
-    auto go = p.cone ? fp_adjoint_kernel<true, true> : fp_adjoint_kernel<false, true>;
+    auto go = p.cone ? (by_samples ? fp_adjoint_samples_kernel<true, true> : fp_adjoint_kernel<true, true>)
+                     : (by_samples ? fp_adjoint_samples_kernel<false, true> : fp_adjoint_kernel<false, true>);
     go<<<grid, block, 0, s>>>(p, t->angles, t->u, t->v, t->cz, t->pmat_a, t->pmat_xs, sgm, mask, cells);
     MCT_TRY(launched("fp_adjoint_kernel"));
     dim3 gb(32, 8), gg((g->nx + 31) / 32, (g->nx + 7) / 8, g->nz);

@@ -11,12 +11,11 @@ namespace mct {
 namespace {
 
 struct FpParams {
-    bool by_samples;  // the adjoint takes samples one by one
-    int nx, nz, nu, nv, views, K, cone, curved, pmat;
     float sid, sdd, cx, cy, cz;
     float stepvd, l_min, inv_px, inv_pz;
     float x0, y0, zoff;  // voxel (0,0) centre x, y; z0 = zoff + cz_view
     float zpv;
+    int nx, nz, nu, nv, views, K, cone, curved, pmat;
     // fp_kernel's ray tiles: a block of 2^ls rays is 16 detector columns x 2^vshift views x
     // 2^(ls - 4 - vshift) detector rows, a warp 2^wcs columns x 2^(5 - wcs) of the block's
     // (view, row) slots; blockIdx.y runs over 2^rs row tiles within each view group (the
