@@ -104,17 +104,17 @@ MCT_HD bool setup_ray(const FpParams& p, int iu, int iv, int j, const float* __r
     return r.ks <= r.ke;
 }
 
-// Steps [kis, kie] whose sample lies at least 1e-3 voxel inside the box on every
-// tested axis (and one more step in from both ends): for them the reference's inside
+// Steps [kis, kie] whose sample lies at least 1e-3 voxel (a float, if that is more) inside the
+// box on every tested axis (and one more step in from both ends): for them the reference's inside
 // test certainly passes, far beyond float rounding, so it can be skipped.  A ray with a term
 // that is no finite number (from an angle, a centre, a matrix) has no such steps, so no index
 // is taken from it; false is returned if the terms that are finite would leave it some.
 MCT_HD bool interior_range(const FpParams& p, const Ray& r, bool test_z, int& kis, int& kie) {
-    const float eps = 1e-3f;
     float lo = -3.0e38f, hi = 3.0e38f;
     bool empty = false, finite = true;
     auto axis = [&](float f0, float df, float n) {
         finite = finite && fabsf(f0) <= 3.4e38f && fabsf(df) <= 3.4e38f;
+        const float eps = fmaxf(1e-3f, n * 0x1p-23f);  // at least a float below n - 1
         const float a = eps, b = n - 1.0f - eps;
         if (!(a <= b)) empty = true;  // one plane: no cell (t1, t2 would span the plane's two sides)
         if (fabsf(df) < 1e-20f) {

@@ -124,3 +124,17 @@ def test_a_ray_without_a_position_has_no_range(table, bad, host_lib):
     rest[hit] = False
     assert not has[hit].any()
     assert (steps.reshape(8, 7, 16, 4)[rest] == good.reshape(8, 7, 16, 4)[rest]).all()
+
+
+@pytest.mark.parametrize("nx", [8191, 20001, 40001, 46339])
+def test_the_last_row_of_a_wide_image_is_no_cell(nx, host_lib):
+    """A ray along the last row of voxels: above 2^15 columns 1e-3 is less than half a float there."""
+    g, t = geom(nx, 1, 9, 1, 4, cone=False, wide=1e-4)
+    for axis, name in ((0, "cx"), (1, "cy")):
+        for sign in (-1, 1):
+            g.cx = g.cy = 0.0
+            setattr(g, name, sign * (nx - 1) / 2 * g.px)
+            steps, terms = ranges(host_lib, g, t)
+            middle = terms.reshape(4, 9, 6)[:, 4]
+            assert (np.abs(middle[:, [0, 2]] - (nx - 1)) < 0.01).any() or (np.abs(middle[:, [0, 2]]) < 0.01).any()
+            check_inside(g, steps, terms)
