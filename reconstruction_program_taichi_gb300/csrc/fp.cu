@@ -250,10 +250,6 @@ fp_kernel(FpParams p, const float* __restrict__ angles, const float* __restrict_
         };
         int kis, kie;
         if (!interior_range(p, r, CONE, kis, kie)) acc = __int_as_float(0x7fffffff);  // its values have no weights
-        if (p.K >= kMaxWalkSteps) {  // step indices would not be exact in float32
-            kis = r.ke + 1;
-            kie = r.ke;
-        }
         for (int k = r.ks; k < kis; ++k) sample(k);
         if (kis <= kie) {
             // Positions come from f = fma(k, df, f0) and floors from adding M = 1.5 * 2^23
@@ -624,10 +620,6 @@ __device__ __forceinline__ void adjoint_ray(const FpParams& p, const Ray& r, int
     };
     int kis, kie;
     interior_range(p, r, CONE, kis, kie);
-    if (p.K >= kMaxWalkSteps) {  // step indices would not be exact in float32
-        kis = r.ke + 1;
-        kie = r.ke;
-    }
     for (int k = r.ks; k < kis; ++k) sample(k);
     if (kis <= kie) {
         const float M = 12582912.0f;

@@ -104,6 +104,11 @@ MCT_HD bool setup_ray(const FpParams& p, int iu, int iv, int j, const float* __r
     return r.ks <= r.ke;
 }
 
+// Above this many steps a ray's indices are no longer exact in float32 (and would not advance one
+// by one), above this many planes its positions' floors: such rays are sampled one sample at a
+// time, each tested.
+constexpr int kMaxWalkSteps = 1 << 23, kMaxWalkPlanes = 1 << 22;
+
 // Steps [kis, kie] whose sample lies at least 1e-3 voxel (a float, if that is more) inside the
 // box on every tested axis (and one more step in from both ends): for them the reference's inside
 // test certainly passes, far beyond float rounding, so it can be skipped.  A ray with a term
@@ -137,16 +142,12 @@ MCT_HD bool interior_range(const FpParams& p, const Ray& r, bool test_z, int& ki
         kie = min(r.ke, (int)floorf(hi) - 1);
     }
     const bool lost = !finite && kis <= kie;
-    if (lost || kis > kie) {
+    if (lost || kis > kie || p.K >= kMaxWalkSteps || (test_z && p.nz > kMaxWalkPlanes)) {
         kis = r.ke + 1;
         kie = r.ke;
     }
     return !lost;
 }
-
-// Above this many steps a ray's indices are no longer exact in float32 (and would not
-// advance one by one): such rays are sampled one sample at a time.
-constexpr int kMaxWalkSteps = 1 << 23;
 
 // The launch parameters of a geometry, without a ray tile.
 inline FpParams ray_params(const mct_geom* g) {

@@ -135,3 +135,27 @@ def test_rays_along_planes(n, nz, nu, nv, step, cuda):
         assert rel_l2(ops.fp(dg, x, mask=m, **a).cpu().numpy(), ref) < TOL[storage]
     for ws in (True, None):
         assert rel_l2(_adjoint(dg, yt, m, ws), back) < 3 * TOL["f32"]
+
+
+def test_volume_of_more_planes_than_the_float_floor_holds(cuda):
+    """2^22 + 4096 planes without a workspace: the samples near the top, where adding 1.5 x 2^23 is
+    no floor, are taken from their own planes.  A ramp that is 0 at plane 2^22 gives each ray its
+    plane times its length; float32 places a plane there to within one, of about 1000."""
+    import torch
+    from reconstruction_program_taichi_gb300 import _lib, ops
+    nz, px, pz, plane, views, nu = (1 << 22) + 4096, 10.0, 0.01, (1 << 22) + 1000, 4, 5
+    steps = int(np.sqrt(2 * (2 * px) ** 2 + (nz * pz) ** 2) / (0.2 * np.sqrt(2 * px * px + pz * pz)))
+    g = _lib.Geom(nu=nu, nv=1, views=views, nv_total=1, nx=2, nz=nz, flags=_lib.MCT_CONE, view_mode=1, fp_steps=steps, du=1.0,
+                  dv=1.0, px=px, pz=pz, cz=(nz - 1) / 2 * pz - plane * pz, sid=300.0, sdd=550.0, total_scan_angle=2 * np.pi,
+                  fp_step=0.2)
+    dg = ops.DeviceGeometry(g, angles=0.3 + np.arange(views) * np.pi / 2, u=np.arange(nu) - 2.0, v=[0.0])
+    z = torch.arange(nz, device="cuda", dtype=torch.float32) - float(1 << 22)
+    ramp = z.clamp(min=0)[:, None, None].expand(nz, 2, 2).contiguous()
+    one = torch.ones_like(ramp)
+    length = ops.fp(dg, one, workspace=None)
+    assert (length > 5.0).all()
+    assert ((ops.fp(dg, ramp, workspace=None) / length - 1000).abs() < 2).all()
+    back = ops.fp_adjoint(dg, torch.ones(dg.sgm_shape, device="cuda"), workspace=None)
+    hit = back.sum((1, 2)).nonzero().flatten()
+    assert ((hit - plane).abs() <= 2).all()
+    assert abs(float(back.sum()) / float(length.sum()) - 1) < 1e-4

@@ -138,3 +138,23 @@ def test_the_last_row_of_a_wide_image_is_no_cell(nx, host_lib):
             middle = terms.reshape(4, 9, 6)[:, 4]
             assert (np.abs(middle[:, [0, 2]] - (nx - 1)) < 0.01).any() or (np.abs(middle[:, [0, 2]]) < 0.01).any()
             check_inside(g, steps, terms)
+
+
+@pytest.mark.parametrize("nz,walked", [((1 << 22) - 1, True), (1 << 22, True), ((1 << 22) + 1, False), ((1 << 22) + 4096, False)])
+def test_planes_that_the_float_floor_does_not_hold_are_not_walked(nz, walked, host_lib):
+    """Adding 1.5 x 2^23 is exactly the floor below 2^22; in taller volumes each sample is tested
+    and takes its index from a conversion."""
+    g, t = geom(2, nz, 5, 3, 4, px=10.0, pz=0.01, high=1e-6, cz=(nz - 1) / 2 * 0.01 - (nz - 100) * 0.01)
+    steps, terms = ranges(host_lib, g, t)
+    middle = (terms[:, 4] + steps[:, :2].mean(1) * terms[:, 5])[steps[:, 0] <= steps[:, 1]]
+    assert middle.size and (np.abs(middle - (nz - 100)) < 10).all()  # the rays lie just below the top
+    assert (steps[:, 2] <= steps[:, 3]).any() == walked
+
+
+def test_long_marches_are_not_walked(host_lib):
+    """Step indices are exact in float32 up to 2^23."""
+    for steps_, walked in (((1 << 23) - 1, True), (1 << 23, False)):
+        g, t = geom(32, 9, 9, 3, 4)
+        g.fp_steps = steps_
+        steps, _ = ranges(host_lib, g, t)
+        assert (steps[:, 2] <= steps[:, 3]).any() == walked
