@@ -89,13 +89,6 @@ __device__ __forceinline__ void fill_view_table(const BpParams& p, const float* 
 //         more than 2^22 rows
 // MODE 1: fan beam in the coronal or sagittal view mode (per-voxel u)
 // MODE 3: projection matrix geometry in any view mode (per-column matrix rows)
-__device__ __forceinline__ float2 reciprocal2(float2 x) {
-    float2 r;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r.x) : "f"(x.x));
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r.y) : "f"(x.y));
-    return __ffma2_rn(r, __ffma2_rn(make_float2(-x.x, -x.y), r, make_float2(1.0f, 1.0f)), r);
-}
-
 template <int MODE, bool CONE, typename QT, typename PT, bool CURVED = false, int ZC = BP_ZC>
 __global__ void __launch_bounds__(BP_TX* BP_TY, bp_min_blocks<MODE, QT, CURVED, ZC>())
 fdk_bp_kernel(BpParams p, const float* __restrict__ angles, const float* __restrict__ pmat,
@@ -149,7 +142,8 @@ fdk_bp_kernel(BpParams p, const float* __restrict__ angles, const float* __restr
             // the detector goes on with a clamped index to the end of its run of kViewRun
             // views.  512x512x256 / 1080 views, FDK: float32 53.7 -> 49.2 ms; 256^3 / 360
             // views coronal, bf16: 4.55 -> 4.08 ms; 333x333x101 / 500 views, curved 6.42 ->
-            // 5.30 ms (bit-identical).  L1 wavefronts bind now (82 % for float32).
+            // 5.30 ms (float32 bit-identical; the bf16 volume moved by 2e-7, single voxels by up to
+            // 8e-5 of the range).  L1 wavefronts bind now (82 % for float32).
             static_assert(CONE && ZC % 2 == 0, "cone-beam modes, slices in pairs");
             struct View {
                 const char* base;  // the view's cell (row 0, column floor(u))
