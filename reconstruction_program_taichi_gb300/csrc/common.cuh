@@ -185,6 +185,18 @@ struct Quad<h16x4> {
         hi = h16x2_to_float2(q.y);
     }
 };
+// Whether the backprojectors take columns of 8 slices instead of 16: where 16 leave the SMs short of
+// warps (blocks16 blocks of two warps) or too many of the last slices empty; otherwise their
+// geometry, which 8 slices pay as often as 16, costs 8 to 12 %, and more on curved detectors.
+// FDK with columns of 16 / 8: 96x96x64, 180 views 125 / 110 us (576 blocks of 16 slices),
+// bf16 157 / 122; 112x112x64 (784 blocks) 144 / 167, bf16 170 / 174; 64^3 113 / 92;
+// 256x256, 360 views: 24 slices 528 / 480, 40 823 / 776 (bf16 842 / 757, curved 850 / 860),
+// 56 1082 / 1056, 72 1323 / 1323; 512x512x8, 360 views 966 / 546.
+inline bool columns_of_8(int64_t blocks16, int slices, bool curved) {
+    const int64_t pad16 = (slices + 15LL) / 16 * 16, pad8 = (slices + 7LL) / 8 * 8;
+    const bool empty = curved ? pad16 * 4 > pad8 * 5 : pad16 * 8 > pad8 * 9;
+    return (blocks16 <= 152 * 4 || empty) && pad8 / 8 <= 65535;
+}
 // Views between checks whether a column has left the detector (8 and 256 within 0.5 %).
 constexpr int kViewRun = 32;
 

@@ -634,16 +634,8 @@ extern "C" int mct_fdk_bp(const mct_geom* g, const mct_tables* t, const void* pa
     p.ss = permuted ? g->nx : plane;
     dim3 block(BP_TX, BP_TY);
     dim3 grid((g->nx + BP_TX - 1) / BP_TX, (p.ncb + BP_TY - 1) / BP_TY, (p.nsl + BP_ZC - 1) / BP_ZC);
-    // Columns of 8 slices where 16 leave the SMs short of warps or too many of the last
-    // slices empty; otherwise their geometry, which 8 slices pay as often as 16, costs 8 to 12 %.
-    // FDK with columns of 16 / 8: 96x96x64, 180 views 125 / 110 us (576 blocks of 16 slices),
-    // bf16 157 / 122; 112x112x64 (784 blocks) 144 / 167, bf16 170 / 174; 64^3 113 / 92;
-    // 256x256, 360 views: 24 slices 528 / 480, 40 823 / 776 (bf16 842 / 757, curved 850 / 860),
-    // 56 1082 / 1056, 72 1323 / 1323; 512x512x8, 360 views 966 / 546.
-    const int64_t pad16 = (p.nsl + 15) / 16 * 16, pad8 = (p.nsl + 7) / 8 * 8;
-    const bool few = (int64_t)grid.x * grid.y * grid.z <= 152 * 4;
-    const bool slices8 = cone && !pm && g->nv <= (1 << 22) && (few || (p.curved ? pad16 * 4 > pad8 * 5 : pad16 * 8 > pad8 * 9)) &&
-                         (p.nsl + 7) / 8 <= 65535;
+    const bool slices8 = cone && !pm && g->nv <= (1 << 22) &&
+                         columns_of_8((int64_t)grid.x * grid.y * grid.z, p.nsl, p.curved);
     if (slices8) grid.z = (unsigned)((p.nsl + 7) / 8);
     MCT_REQUIRE(grid.y <= 65535 && grid.z <= 65535, "mct_fdk_bp: volume too large for the launch grid");
     cudaStream_t s = as_stream(stream);

@@ -640,7 +640,7 @@ void launch_axial_shape(const mct_geom* g, const UbParams& p, const mct_tables* 
                                                                                           packed, out, f16_max, e);
 }
 // Blocks of two warps, as in the FDK kernel, except with the epilogue, whose partial sums are
-// one per 32 x 8 columns; columns of 8 slices by the FDK kernel's rule.  CGLS of 3 iterations,
+// one per 32 x 8 columns; columns of 8 slices by the FDK kernel's rule (columns_of_8).  CGLS of 3 iterations,
 // ms, blocks of 8 warps / 2 warps / 2 warps with 8 slices: 128x128x48, 120 views 1.958 / 1.836
 // / 1.893; 64^3, 120 views 1.103 / 1.064 / 0.901; 96x96x64 1.547 / 1.551 / 1.484; 112x112x64
 // 2.029 / 1.914 / 1.969; 200x200, 180 views: 24 slices 3.622 / 3.342 / 2.963, 56 6.650 / 6.460
@@ -649,9 +649,8 @@ template <typename OT, bool EPI, bool PIPE, typename QT, typename PT>
 void launch_axial_q(const mct_geom* g, const UbParams& p, const mct_tables* t, const void* packed, OT* out,
                     const uint32_t* f16_max, const CgEpi& e, cudaStream_t s) {
     if constexpr (!EPI && PIPE) {
-        const int64_t pad16 = (g->nz + 15) / 16 * 16, pad8 = (g->nz + 7) / 8 * 8;
         const int64_t columns = (int64_t)((g->nx + 7) / 8) * ((g->nx + 7) / 8);
-        if ((columns * (pad16 / 16) <= 152 * 4 || pad16 * 8 > pad8 * 9) && pad8 / 8 <= 65535)
+        if (columns_of_8(columns * ((g->nz + 15) / 16), g->nz, false))
             launch_axial_shape<OT, EPI, PIPE, QT, PT, 8, 8>(g, p, t, packed, out, f16_max, e, s);
         else
             launch_axial_shape<OT, EPI, PIPE, QT, PT, 8, 16>(g, p, t, packed, out, f16_max, e, s);
