@@ -301,12 +301,15 @@ def run_gpu(args, w):
     cells = g_fdk.views * g_fdk.nv * (g_fdk.nu - 1)  # (nv - 1) cell rows + one NaN row per view
     bp_elem = 16 if pipe.dtype == ops.MCT_F32 else 8
     fp_rays = fpg.geom.nv * fpg.geom.views * fpg.geom.nu
+    # cells visited: a ray crosses 1.33 cells per voxel length on average over a scan
+    g_fp = fpg.geom
+    fp_cells = n_samples * min(1.0, 1.33 * g_fp.fp_step * (2.0 + (g_fp.pz / g_fp.px) ** 2) ** 0.5)
     kern = {
         "fp_kernel": dict(ms=float(st[3]), compulsory=nvox * 32 + fp_rays * 4,
-                          gather=n_samples * (32 if fp_dtype == ops.MCT_F32 else 16),
+                          gather=fp_cells * (32 if fp_dtype == ops.MCT_F32 else 16),
                           what="copies of the volume (32 B per voxel, both orientations) read once, the "
                                "projection written once; gathers: one 32-byte (16-bit: 16-byte) cell per "
-                               "in-volume sample (a ray loads a cell once for all its samples there)"),
+                               "cell visited, which a ray loads once for all its samples there"),
         "fdk_bp_kernel": dict(ms=float(st[2]), compulsory=cells * bp_elem + nvox * 4,
                               gather=nvox * w["views"] * bp_elem,
                               what="packed operand (16 B float32 / 8 B 16-bit per detector cell) read once, the "
