@@ -668,81 +668,12 @@ __device__ __forceinline__ void adjoint_ray_z(const FpParams& p, const Ray& r, i
         adjoint_ray<CONE, CELLS, fx, fy, false>(p, r, iv, yv, out);
 }
 
-// Exact transpose of fp_kernel: every in-volume sample scatters its trilinear weights
-// times the ray value into the volume.  As in the projector, the samples of one cell are
-// taken together: a corner's weights summed over n equally spaced samples with midpoint m
-// are n [u v w (m) + s^2 (du dv w + du dw v + dv dw u)(m)], s^2 = (n^2 - 1) / 12, for the
-// corner's linear weights u, v, w along the axes.
-//
-// A ray that crosses into the next cell along x or y is done with the face it leaves
-// behind: that face's corners are reduced, the ones it shares with the next cell stay in
-// registers.  A crossing along z (rare) does the same with the corners left behind, any
-// other change of cell reduces all.  Without CELLS the corners are added to the volume one
-// by one.  CELLS, cone beam: the faces' sums go to two buffers in the workspace, 16 bytes
-// per voxel each: XF(z, y, x) holds the face {y, y+1} x {z, z+1} at x, YF(z, y, x) the face
-// {x, x+1} x {z, z+1} at y, both ordered (lo, lo) (hi, lo) (lo, hi) (hi, hi) with z last:
-// one 16-byte reduction a face, two of 8 bytes in XF for a crossing along z;
-// adjoint_gather_kernel then sums each voxel's entries of the faces that contain it.
-// CELLS, fan beam: the 4 corner sums of a cell are one 16-byte reduction anyway (two edges
-// of 8 bytes cost more: a reduction of 8 bytes takes the L2 as long as one of 16).
-//
-// 250^2 x 45, 501 x 47 x 181 views: 2.5 ms, sample by sample with both 16-byte groups of a
-// cell reduced at every change of cell 4.6 ms.  The reductions bound it: the L2 is at 74 % of
-// its peak (16 bytes for each of some 6e8 crossings), and neither more warps nor fewer
-// instructions (16 selects less per cell: 2 %) nor an XF with y first, whose entries of
-// neighbouring rays share a sector (0 %), bring much more.  Without CELLS, ms before /
-// after: 123x123x51, 300 views 7.95 / 5.16, step 0.5 6.06 / 5.05; fan beam 300^2 x 4, 360
-// views 2.35 / 1.40.  Blocks of 8 rows of rays (4 cost the scalar additions 2 to 10 %); of 4
-// for cone beam with CELLS (grad above 2 %, 512^2 x 64 4 %), where the grid allows it.
-// Where a cell holds few samples, fp_adjoint_samples_kernel below (adjoint_by_samples).
+// One ray of the adjoint sample by sample: a cell's corner sums are kept in registers and all
+// added when the ray enters another, into the buffers of fp_adjoint_kernel with CELLS (cone beam:
+// the faces behind and ahead along x).
 template <bool CONE, bool CELLS>
-__global__ void __launch_bounds__(256)
-fp_adjoint_kernel(FpParams p, const float* __restrict__ angles, const float* __restrict__ u_arr,
-                  const float* __restrict__ v_arr, const float* __restrict__ czv, const float* __restrict__ pa,
-                  const float* __restrict__ pxs, const float* __restrict__ sgm, const float* __restrict__ mask,
-                  float* __restrict__ out) {
-    const int iu = blockIdx.x * blockDim.x + threadIdx.x;
-    const int iv = blockIdx.z * blockDim.y + threadIdx.y;
-    const int j = blockIdx.y;
-    if (iu >= p.nu || iv >= p.nv) return;
-    const int64_t oidx = ((int64_t)iv * p.views + j) * p.nu + iu;
-    if (mask && mask[oidx] != 1.0f) return;
-    const float yv = sgm[oidx] * p.stepvd;
-    if (yv == 0.0f) return;
-    Ray r;
-    if (!setup_ray(p, iu, iv, j, angles, u_arr, v_arr, czv, pa, pxs, true, r)) return;
-    if (r.dfx < 0.0f) {
-        if (r.dfy < 0.0f)
-            adjoint_ray_z<CONE, CELLS, true, true>(p, r, iv, yv, out);
-        else
-            adjoint_ray_z<CONE, CELLS, true, false>(p, r, iv, yv, out);
-    } else {
-        if (r.dfy < 0.0f)
-            adjoint_ray_z<CONE, CELLS, false, true>(p, r, iv, yv, out);
-        else
-            adjoint_ray_z<CONE, CELLS, false, false>(p, r, iv, yv, out);
-    }
-}
-
-// The adjoint sample by sample, for rays with few cells or about a sample per cell: a cell's corner
-// sums are kept in registers and all added when the ray enters another, into the buffers of
-// fp_adjoint_kernel with CELLS (cone beam: the faces behind and ahead along x).
-template <bool CONE, bool CELLS>
-__global__ void __launch_bounds__(256)
-fp_adjoint_samples_kernel(FpParams p, const float* __restrict__ angles, const float* __restrict__ u_arr,
-                          const float* __restrict__ v_arr, const float* __restrict__ czv, const float* __restrict__ pa,
-                          const float* __restrict__ pxs, const float* __restrict__ sgm, const float* __restrict__ mask,
-                          float* __restrict__ out) {
-    const int iu = blockIdx.x * blockDim.x + threadIdx.x;
-    const int iv = blockIdx.z * blockDim.y + threadIdx.y;
-    const int j = blockIdx.y;
-    if (iu >= p.nu || iv >= p.nv) return;
-    const int64_t oidx = ((int64_t)iv * p.views + j) * p.nu + iu;
-    if (mask && mask[oidx] != 1.0f) return;
-    const float yv = sgm[oidx] * p.stepvd;
-    if (yv == 0.0f) return;
-    Ray r;
-    if (!setup_ray(p, iu, iv, j, angles, u_arr, v_arr, czv, pa, pxs, true, r)) return;
+__device__ __forceinline__ void adjoint_ray_samples(const FpParams& p, const Ray& r, int iv, float yv,
+                                                    float* __restrict__ out) {
     const int nx = p.nx;
     const int plane = nx * nx;
     int cell = -1;
@@ -809,6 +740,86 @@ fp_adjoint_samples_kernel(FpParams p, const float* __restrict__ angles, const fl
         }
     }
     flush();
+}
+
+// Exact transpose of fp_kernel: every in-volume sample scatters its trilinear weights
+// times the ray value into the volume.  As in the projector, the samples of one cell are
+// taken together: a corner's weights summed over n equally spaced samples with midpoint m
+// are n [u v w (m) + s^2 (du dv w + du dw v + dv dw u)(m)], s^2 = (n^2 - 1) / 12, for the
+// corner's linear weights u, v, w along the axes.
+//
+// A ray that crosses into the next cell along x or y is done with the face it leaves
+// behind: that face's corners are reduced, the ones it shares with the next cell stay in
+// registers.  A crossing along z (rare) does the same with the corners left behind, any
+// other change of cell reduces all.  Without CELLS the corners are added to the volume one
+// by one.  CELLS, cone beam: the faces' sums go to two buffers in the workspace, 16 bytes
+// per voxel each: XF(z, y, x) holds the face {y, y+1} x {z, z+1} at x, YF(z, y, x) the face
+// {x, x+1} x {z, z+1} at y, both ordered (lo, lo) (hi, lo) (lo, hi) (hi, hi) with z last:
+// one 16-byte reduction a face, two of 8 bytes in XF for a crossing along z;
+// adjoint_gather_kernel then sums each voxel's entries of the faces that contain it.
+// CELLS, fan beam: the 4 corner sums of a cell are one 16-byte reduction anyway (two edges
+// of 8 bytes cost more: a reduction of 8 bytes takes the L2 as long as one of 16).
+//
+// 250^2 x 45, 501 x 47 x 181 views: 2.5 ms, sample by sample with both 16-byte groups of a
+// cell reduced at every change of cell 4.6 ms.  The reductions bound it: the L2 is at 74 % of
+// its peak (16 bytes for each of some 6e8 crossings), and neither more warps nor fewer
+// instructions (16 selects less per cell: 2 %) nor an XF with y first, whose entries of
+// neighbouring rays share a sector (0 %), bring much more.  Without CELLS, ms before /
+// after: 123x123x51, 300 views 7.95 / 5.16, step 0.5 6.06 / 5.05; fan beam 300^2 x 4, 360
+// views 2.35 / 1.40.  Blocks of 8 rows of rays (4 cost the scalar additions 2 to 10 %); of 4
+// for cone beam with CELLS (grad above 2 %, 512^2 x 64 4 %), where the grid allows it.
+// Where a cell holds few samples, fp_adjoint_samples_kernel below (adjoint_by_samples).
+template <bool CONE, bool CELLS>
+__global__ void __launch_bounds__(256)
+fp_adjoint_kernel(FpParams p, const float* __restrict__ angles, const float* __restrict__ u_arr,
+                  const float* __restrict__ v_arr, const float* __restrict__ czv, const float* __restrict__ pa,
+                  const float* __restrict__ pxs, const float* __restrict__ sgm, const float* __restrict__ mask,
+                  float* __restrict__ out) {
+    const int iu = blockIdx.x * blockDim.x + threadIdx.x;
+    const int iv = blockIdx.z * blockDim.y + threadIdx.y;
+    const int j = blockIdx.y;
+    if (iu >= p.nu || iv >= p.nv) return;
+    const int64_t oidx = ((int64_t)iv * p.views + j) * p.nu + iu;
+    if (mask && mask[oidx] != 1.0f) return;
+    const float yv = sgm[oidx] * p.stepvd;
+    if (yv == 0.0f) return;
+    Ray r;
+    if (!setup_ray(p, iu, iv, j, angles, u_arr, v_arr, czv, pa, pxs, true, r)) return;
+    if (!(fabsf(yv) <= 3.4e38f)) {  // an infinite value: corners are not what others leave of it
+        adjoint_ray_samples<CONE, CELLS>(p, r, iv, yv, out);
+        return;
+    }
+    if (r.dfx < 0.0f) {
+        if (r.dfy < 0.0f)
+            adjoint_ray_z<CONE, CELLS, true, true>(p, r, iv, yv, out);
+        else
+            adjoint_ray_z<CONE, CELLS, true, false>(p, r, iv, yv, out);
+    } else {
+        if (r.dfy < 0.0f)
+            adjoint_ray_z<CONE, CELLS, false, true>(p, r, iv, yv, out);
+        else
+            adjoint_ray_z<CONE, CELLS, false, false>(p, r, iv, yv, out);
+    }
+}
+
+// The adjoint sample by sample, for rays with few cells or about a sample per cell.
+template <bool CONE, bool CELLS>
+__global__ void __launch_bounds__(256)
+fp_adjoint_samples_kernel(FpParams p, const float* __restrict__ angles, const float* __restrict__ u_arr,
+                          const float* __restrict__ v_arr, const float* __restrict__ czv, const float* __restrict__ pa,
+                          const float* __restrict__ pxs, const float* __restrict__ sgm, const float* __restrict__ mask,
+                          float* __restrict__ out) {
+    const int iu = blockIdx.x * blockDim.x + threadIdx.x;
+    const int iv = blockIdx.z * blockDim.y + threadIdx.y;
+    const int j = blockIdx.y;
+    if (iu >= p.nu || iv >= p.nv) return;
+    const int64_t oidx = ((int64_t)iv * p.views + j) * p.nu + iu;
+    if (mask && mask[oidx] != 1.0f) return;
+    const float yv = sgm[oidx] * p.stepvd;
+    if (yv == 0.0f) return;
+    Ray r;
+    if (!setup_ray(p, iu, iv, j, angles, u_arr, v_arr, czv, pa, pxs, true, r)) return;
+    adjoint_ray_samples<CONE, CELLS>(p, r, iv, yv, out);
 }
 
 // vol[z][y][x] += its entries of the faces (cone beam, buffers XF and YF above) or cells
