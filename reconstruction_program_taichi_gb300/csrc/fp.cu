@@ -669,9 +669,10 @@ __device__ __forceinline__ void adjoint_ray_z(const FpParams& p, const Ray& r, i
 }
 
 // One ray of the adjoint sample by sample: a cell's corner sums are kept in registers and all
-// added when the ray enters another, into the buffers of fp_adjoint_kernel with CELLS (cone beam:
-// the faces behind and ahead along x).
-template <bool CONE, bool CELLS>
+// added when the ray enters another, to the volume or to the workspace: with FACES to XF of
+// fp_adjoint_kernel (the faces behind and ahead along x), else to the cell's own 8 (fan beam: 4)
+// sums, x first.
+template <bool CONE, bool CELLS, bool FACES>
 __device__ __forceinline__ void adjoint_ray_samples(const FpParams& p, const Ray& r, int iv, float yv,
                                                     float* __restrict__ out) {
     const int nx = p.nx;
@@ -681,12 +682,13 @@ __device__ __forceinline__ void adjoint_ray_samples(const FpParams& p, const Ray
     auto flush = [&]() {
         if (cell < 0) return;
         if constexpr (CELLS) {
-            float* c = out + (int64_t)cell * 4;
-            if (CONE) {
+            float* c = out + (int64_t)cell * (CONE && !FACES ? 8 : 4);
+            if (CONE && FACES) {
                 red_add_v4(c, s00, s10, t00, t10);
                 red_add_v4(c + 4, s01, s11, t01, t11);
             } else {
                 red_add_v4(c, s00, s01, s10, s11);
+                if (CONE) red_add_v4(c + 4, t00, t01, t10, t11);
             }
         } else {
             float* b = out + cell;
@@ -786,7 +788,7 @@ fp_adjoint_kernel(FpParams p, const float* __restrict__ angles, const float* __r
     Ray r;
     if (!setup_ray(p, iu, iv, j, angles, u_arr, v_arr, czv, pa, pxs, true, r)) return;
     if (!(fabsf(yv) <= 3.4e38f)) {  // an infinite value: corners are not what others leave of it
-        adjoint_ray_samples<CONE, CELLS>(p, r, iv, yv, out);
+        adjoint_ray_samples<CONE, CELLS, CONE>(p, r, iv, yv, out);
         return;
     }
     if (r.dfx < 0.0f) {
@@ -802,7 +804,9 @@ fp_adjoint_kernel(FpParams p, const float* __restrict__ angles, const float* __r
     }
 }
 
-// The adjoint sample by sample, for rays with few cells or about a sample per cell.
+// The adjoint sample by sample, for rays with few cells or about a sample per cell.  In the
+// workspace each cell has its own 32 bytes: in faces, which neighbouring cells share, many rays on a
+// small volume wait for each other's additions (42x42x2, 793 views, step 0.5 84 us, now 66).
 template <bool CONE, bool CELLS>
 __global__ void __launch_bounds__(256)
 fp_adjoint_samples_kernel(FpParams p, const float* __restrict__ angles, const float* __restrict__ u_arr,
@@ -819,12 +823,12 @@ fp_adjoint_samples_kernel(FpParams p, const float* __restrict__ angles, const fl
     if (yv == 0.0f) return;
     Ray r;
     if (!setup_ray(p, iu, iv, j, angles, u_arr, v_arr, czv, pa, pxs, true, r)) return;
-    adjoint_ray_samples<CONE, CELLS>(p, r, iv, yv, out);
+    adjoint_ray_samples<CONE, CELLS, false>(p, r, iv, yv, out);
 }
 
-// vol[z][y][x] += its entries of the faces (cone beam, buffers XF and YF above) or cells
-// (fan beam) that contain it, in a fixed order.
-template <bool CONE>
+// vol[z][y][x] += its entries of the cells that contain it (8 sums each in cone beam, 4 in fan
+// beam), or with FACES of the faces (buffers XF and YF above), in a fixed order.
+template <bool CONE, bool FACES>
 __global__ void __launch_bounds__(256)
 adjoint_gather_kernel(int nx, int nz, const float* __restrict__ cells, float* __restrict__ vol) {
     const int x = blockIdx.x * blockDim.x + threadIdx.x;
@@ -834,7 +838,7 @@ adjoint_gather_kernel(int nx, int nz, const float* __restrict__ cells, float* __
     const int64_t plane = (int64_t)nx * nx;
     const int64_t v = z * plane + (int64_t)y * nx + x;
     float acc = 0.0f;
-    if (CONE) {
+    if constexpr (FACES) {
         const float* yfaces = cells + (int64_t)nz * plane * 4;
 #pragma unroll
         for (int dz = 0; dz < 2; ++dz) {
@@ -847,13 +851,18 @@ adjoint_gather_kernel(int nx, int nz, const float* __restrict__ cells, float* __
             }
         }
     } else {
+        constexpr int C = CONE ? 8 : 4;
 #pragma unroll
-        for (int dy = 0; dy < 2; ++dy) {
-            if (y - dy < 0) continue;
+        for (int dz = 0; dz < C / 4; ++dz) {
+            if (z - dz < 0) continue;
 #pragma unroll
-            for (int dx = 0; dx < 2; ++dx) {
-                if (x - dx < 0) continue;
-                acc += __ldg(cells + (v - (int64_t)dy * nx - dx) * 4 + dy * 2 + dx);
+            for (int dy = 0; dy < 2; ++dy) {
+                if (y - dy < 0) continue;
+#pragma unroll
+                for (int dx = 0; dx < 2; ++dx) {
+                    if (x - dx < 0) continue;
+                    acc += __ldg(cells + (v - dz * plane - (int64_t)dy * nx - dx) * C + dz * 4 + dy * 2 + dx);
+                }
             }
         }
     }
@@ -1041,21 +1050,17 @@ inline bool walk_by_samples(const mct_geom* g, int32_t dtype, bool copies) {
 // without a workspace 7.8 / 13.6 us; 90x90x4, 73 views of 4 x 174, step 0.5, with one 36 / 42 us.
 // Fan beam with a workspace: the reductions are the same either way (445^2 x 2, 179 views, step
 // 0.5 417 / 425 us, 0.3 492 / 449).
-// Otherwise it is the faces that the walk by cells saves.  Without a workspace it pays until a
-// cell holds half a sample (123x123x51, 300 views, step 0.7 5.7 / 5.1 ms, 1.0 3.97 / 4.02, 1.5
-// 2.71 / 2.81; fan beam 300^2 x 4, 360 views, 1.0 1.49 / 1.33, 1.5 0.98 / 0.97).  With one, whose
-// reductions carry four values, the longer the wider the volume (51x51x19, 95 views, 0.8 31 / 46
-// us; 115x115x40, 674 views, 0.8 2.27 / 2.07 ms; 64^3, 180 views, 0.5 0.36 / 0.30 ms, 2.5 83 /
-// 103 us), and less where columns a voxel and more apart share few faces (67x67x100, 292 views
-// of 111 x 61, 1.2 259 / 316 us).
+// Otherwise it is the faces that the walk by cells saves, which pays until a cell holds half a
+// sample.  Without a workspace 123x123x51, 300 views, step 0.7 5.7 / 5.1 ms, 1.0 3.97 / 4.02, 1.5 2.71
+// / 2.81; fan beam 300^2 x 4, 360 views, 1.0 1.49 / 1.33, 1.5 0.98 / 0.97.  With one 51x51x19, 95 views,
+// 0.8 31 / 46 us; 55x55x10, 227 views, 0.5 143 / 88 us; 150x150x8, 265 views, 0.8 447 / 347 us;
+// 316x316x17, 69 views, 1.0 (0.43 samples) 964 / 796 us; 62x62x2, 561 views, 1.3 (0.33) 46 / 56 us.
 inline bool adjoint_by_samples(const mct_geom* g, bool cells) {
     const bool cone = (g->flags & MCT_CONE) != 0;
     const double n = samples_per_cell(g);
     const int64_t rays = sgm_elems(*g);
     if ((!cone && cells) || rays < 60000) return n < (rays < 4000 ? 1.6 : 1.2);
-    if (!cone) return false;
-    if (!cells) return n < (g->nx < 64 ? 0.6 : 0.45);
-    return n < (g->nx < 32 ? 1.5 : g->nx < 64 ? 1.2 : g->nx < 112 ? 0.6 : 4LL * g->nu <= 5LL * g->nx ? 0.4 : 0.0);
+    return cone && n < (g->nx < 64 ? 0.6 : cells ? 0.4 : 0.45);
 }
 inline size_t copy_elems(const mct_geom* g) { return (size_t)g->nz * g->nx * copy_pitch(g); }
 
@@ -1277,17 +1282,17 @@ int mct_fp_adjoint_cells(const mct_geom* g, const mct_tables* t, const float* sg
     MCT_REQUIRE(cudaMemsetAsync(cells, 0, mct_fp_adjoint_workspace_size(g), s) == cudaSuccess,
                 "mct_fp_adjoint_cells: clearing the workspace failed");
     const bool by_samples = adjoint_by_samples(g, true);
-    const int rows = p.cone && g->nv <= 4 * 65535 ? 4 : 8;
+    const int rows = p.cone && !by_samples && g->nv <= 4 * 65535 ? 4 : 8;
     dim3 block(32, rows), grid((g->nu + 31) / 32, g->views, (g->nv + rows - 1) / rows);
     auto go = p.cone ? (by_samples ? fp_adjoint_samples_kernel<true, true> : fp_adjoint_kernel<true, true>)
                      : (by_samples ? fp_adjoint_samples_kernel<false, true> : fp_adjoint_kernel<false, true>);
     go<<<grid, block, 0, s>>>(p, t->angles, t->u, t->v, t->cz, t->pmat_a, t->pmat_xs, sgm, mask, cells);
     MCT_TRY(launched("fp_adjoint_kernel"));
     dim3 gb(32, 8), gg((g->nx + 31) / 32, (g->nx + 7) / 8, g->nz);
-    if (p.cone)
-        adjoint_gather_kernel<true><<<gg, gb, 0, s>>>(g->nx, g->nz, cells, vol);
-    else
-        adjoint_gather_kernel<false><<<gg, gb, 0, s>>>(g->nx, g->nz, cells, vol);
+    auto gather = !p.cone ? adjoint_gather_kernel<false, false>
+                  : by_samples ? adjoint_gather_kernel<true, false>
+                               : adjoint_gather_kernel<true, true>;
+    gather<<<gg, gb, 0, s>>>(g->nx, g->nz, cells, vol);
     return launched("adjoint_gather_kernel");
 }
 
