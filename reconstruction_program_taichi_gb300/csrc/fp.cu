@@ -1034,14 +1034,16 @@ inline bool long_scan(const mct_geom* g) { return g->views >= 256 || g->views >=
 //     0.5 27.5 / 32.3 (26.8), 54x54x36, 23 views, 1.2 14.5 / 17.9 (16.4);
 //   fan beam 491 columns, 147 views, 0.5 (1.1) 194 / 223 (207), 253 columns, 52 views, 1.2
 //     43.7 / 49.1 (45.3); step 0.3 (1.8) costs samples 1.5 to 1.9 times as much.
-// With windows, from 256 columns on, float32 cells stay for short scans (512x512x64, 90 views, 0.5
-// 3567 / 3252); long ones go by samples where a cell holds about one (319x319x109, 617 views,
-// 0.5 13570 / 14380 (13964); 426 columns, 0.7 (0.6) 15725 / 15290 but 270 columns 1933 / 2094
-// (1990); 1.0 (0.4) 2 % more for samples).  Without copies they stay (even at 0.5).
+// With windows, from 256 columns on, float32 with copies: short scans stay by cells (512x512x64, 90
+// views, 0.5 3567 / 3252) until a cell holds few samples (509x509x185, 125 views, 1.3 (0.33) 7640 /
+// 8940 (8230)); long ones go by samples (319x319x109, 617 views, 0.5 13570 / 14380 (13964); 277x277x74,
+// 439 views, 1.0 (0.43) 4185 / 4780 (4189); 426 columns, 0.7 (0.6) 15725 / 15290).  Without copies
+// 362x362x161, 284 views, 0.5 49.1 / 56.6 (56.8) ms, 402x402x15, 346 views 4.25 / 4.54 (5.49), 0.8
+// 458x458x52, 306 views 6.57 / 6.57 (8.45).
 inline bool walk_by_samples(const mct_geom* g, int32_t dtype, bool copies) {
     const bool cone = (g->flags & MCT_CONE) != 0, wide = walk_in_windows(g);
     const double n = samples_per_cell(g);
-    if (dtype == MCT_F32 && cone && wide) return copies && long_scan(g) && n >= 0.6 && n < 1.2;
+    if (dtype == MCT_F32 && cone && wide) return n < (copies && !long_scan(g) ? 0.4 : 1.2);
     return n < (dtype == MCT_BF16 || (dtype == MCT_F16 && !wide) ? 1.5 : 1.2);
 }
 // Whether the adjoint goes by samples; figures by samples / by cells.
@@ -1155,10 +1157,16 @@ int fp_storage_impl(const mct_geom* g, const mct_tables* t, const TIN* vol_in, c
     // cross nearly the same cells, and the outer rows' slab (up to ~50 planes) does not fit
     // L2 across all views.  Otherwise row tiles are only grouped where the grid needs it.
     const bool copies = p.cone && workspace, by_samples = walk_by_samples(g, dtype, copies);
-    const bool small_tile = by_samples && !(dtype == MCT_F32 && p.cone && walk_in_windows(g)) && g->nv <= 65535;
+    // Wide float32 volumes without copies, or by samples with far apart views, take 4 views x 4 rows
+    // in warps of 16 columns.  By samples, with 16 views / so: without copies 362x362x161, 284 views,
+    // step 0.5 65.8 / 49.1 ms, 458x458x52, 306 views, 0.8 7.40 / 6.57; with copies 509x509x185, 125
+    // views, 1.3 8.12 / 7.64.  By cells without copies 298x298x35, 536 views, 0.1 6.97 / 6.98.
+    const bool wide32 = dtype == MCT_F32 && p.cone && walk_in_windows(g);
+    const bool small_tile = by_samples && !wide32 && g->nv <= 65535;
+    const bool row_tile = wide32 && (!copies || (by_samples && !long_scan(g)));
     p.ls = small_tile ? 7 : 8;
-    p.vshift = small_tile ? 3 : copies && dtype != MCT_F32 ? 2 : 4;
-    if (p.cone) p.wcs = long_scan(g) ? 2 : by_samples ? 3 : 4;
+    p.vshift = small_tile ? 3 : (copies && dtype != MCT_F32) || row_tile ? 2 : 4;
+    if (p.cone) p.wcs = row_tile ? 4 : long_scan(g) ? 2 : by_samples ? 3 : 4;
     else p.wcs = g->nv >= 4 && 2 * g->views < g->nx ? 4 : 3;
     if (!small_tile) {
         auto rays = [&](int vs) {  // of the tiles of 2^vs views, in and outside the scan
