@@ -1034,6 +1034,9 @@ inline bool long_scan(const mct_geom* g) { return g->views >= 256 || g->views >=
 //     0.5 27.5 / 32.3 (26.8), 54x54x36, 23 views, 1.2 14.5 / 17.9 (16.4);
 //   fan beam 491 columns, 147 views, 0.5 (1.1) 194 / 223 (207), 253 columns, 52 views, 1.2
 //     43.7 / 49.1 (45.3); step 0.3 (1.8) costs samples 1.5 to 1.9 times as much.
+//   16-bit between the two: bf16 81x81x3, 158 views (1.53) 25 / 38 (33), 459x459x10, 288 views
+//     (1.63) 2093 / 2170, 412x412x94, 376 views (1.63) 16920 / 16140; float16 187x187x10, 59 views
+//     (1.53) 109 / 123 (134), 96x96x53 (1.63) 932 / 858.
 // With windows, from 256 columns on, float32 with copies: short scans stay by cells (512x512x64, 90
 // views, 0.5 3567 / 3252) until a cell holds few samples (509x509x185, 125 views, 1.3 (0.33) 7640 /
 // 8940 (8230)); long ones go by samples (319x319x109, 617 views, 0.5 13570 / 14380 (13964); 277x277x74,
@@ -1044,7 +1047,7 @@ inline bool walk_by_samples(const mct_geom* g, int32_t dtype, bool copies) {
     const bool cone = (g->flags & MCT_CONE) != 0, wide = walk_in_windows(g);
     const double n = samples_per_cell(g);
     if (dtype == MCT_F32 && cone && wide) return n < (copies && !long_scan(g) ? 0.4 : 1.2);
-    return n < (dtype == MCT_BF16 || (dtype == MCT_F16 && !wide) ? 1.5 : 1.2);
+    return n < (dtype == MCT_BF16 ? 1.65 : dtype == MCT_F16 && !wide ? 1.55 : 1.2);
 }
 // Whether the adjoint goes by samples; figures by samples / by cells.
 // A thread pays for a walk by cells before its first sample, so grids that leave the GPU
