@@ -763,7 +763,7 @@ __device__ __forceinline__ void adjoint_ray_samples(const FpParams& p, const Ray
 // of 8 bytes cost more: a reduction of 8 bytes takes the L2 as long as one of 16).
 //
 // 250^2 x 45, 501 x 47 x 181 views: 2.5 ms, sample by sample with both 16-byte groups of a
-// cell reduced at every change of cell 4.6 ms.  The reductions bound it: the L2 is at 74 % of
+// cell reduced at every change of cell 4.6 ms.  The reductions bound it: the L2 is at 78 % of
 // its peak (16 bytes for each of some 6e8 crossings), and neither more warps nor fewer
 // instructions (16 selects less per cell: 2 %) nor an XF with y first, whose entries of
 // neighbouring rays share a sector (0 %), bring much more.  Without CELLS, ms before /
