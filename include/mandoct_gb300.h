@@ -254,15 +254,16 @@ int mct_fp_adjoint(const mct_geom* g, const mct_tables* t, const float* sgm, con
                    float* vol, void* stream);
 
 /* Bytes of the mct_fp_adjoint_cells workspace: 32 per voxel in cone beam (the 4
- * corner sums of two cell faces, one across x and one across y), 16 in fan beam (the 4 of
- * a slice's cell). */
+ * corner sums of two cell faces, one across x and one across y, or the 8 of a cell), 16 in
+ * fan beam (the 4 of a slice's cell). */
 size_t mct_fp_adjoint_workspace_size(const mct_geom* g);
 
 /* mct_fp_adjoint (vol += P^T sgm) with the scatter done in cell space: each ray
- * adds the corner sums of the cell face it leaves behind (fan: of the cell) with one 16-byte
- * vector reduction to workspace (mct_fp_adjoint_workspace_size bytes, 16-byte aligned,
- * cleared on the stream by this call), then one pass adds to each voxel the entries of
- * the faces (cells) that contain it.  Same operator as mct_fp_adjoint up to the order of the
+ * adds the corner sums of the cell face it leaves behind (fan, and where cells hold few
+ * samples: of the cell) with 16-byte vector reductions to workspace
+ * (mct_fp_adjoint_workspace_size bytes, 16-byte aligned, cleared on the stream by this
+ * call), then one pass adds to each voxel the entries of the faces (cells) that contain
+ * it.  Same operator as mct_fp_adjoint up to the order of the
  * float32 additions.  No counterpart in the reference. */
 int mct_fp_adjoint_cells(const mct_geom* g, const mct_tables* t, const float* sgm, const float* mask,
                          float* vol, void* workspace, void* stream);
